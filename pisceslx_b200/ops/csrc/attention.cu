@@ -24,6 +24,17 @@ int set_smem(K kern, int bytes) {
   return static_cast<int>(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
 }
 
+int sm_count() {
+  static PerDeviceInt count;
+  if (!count.cur()) {
+    int dev = 0, n = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    count.cur() = n > 0 ? n : 148;
+  }
+  return count.cur();
+}
+
 constexpr float kLog2eHost = 1.4426950408889634f;
 
 }  // namespace
@@ -43,13 +54,15 @@ int launch_attn_fwd(const AttnArgs& a, cudaStream_t stream) {
   p.lse = a.lse;
   p.cu_q = a.cu_q;
   p.cu_k = a.cu_k ? a.cu_k : a.cu_q;
-  p.hq = a.hq; p.hk = a.hk;
+  p.hq = a.hq; p.hk = a.hk; p.batch = a.batch;
   p.o_stride = a.o_stride;
   p.total_q = a.total_q;
   p.causal = a.causal;
   p.scale_log2 = a.scale * kLog2eHost;
   p.status = a.status;
-  dim3 grid((a.max_q + 127) / 128, a.hq, a.batch);
+  p.items = static_cast<int64_t>((a.max_q + 255) / 256) * a.hq * a.batch;
+  const int sms = sm_count();
+  const unsigned grid = static_cast<unsigned>(p.items < sms ? p.items : sms);
   if (a.d == 128) {
     static PerDeviceInt cfg;
     if (!cfg.cur()) { r = set_smem(attn_fwd_kernel<128>, AttnFwdSmem<128>::kTotal); if (r) return r; cfg.cur() = 1; }

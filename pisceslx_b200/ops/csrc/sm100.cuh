@@ -47,6 +47,17 @@ __device__ __forceinline__ bool elect_one() {
   return pred != 0;
 }
 
+// Registers per thread of the calling warpgroup (all four warps): give some up, or take more of what the block was
+// launched with (the warpgroups' shares must not add up to more than that).
+template <int N>
+__device__ __forceinline__ void regs_give() {
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
+}
+template <int N>
+__device__ __forceinline__ void regs_take() {
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N));
+}
+
 // ---------------------------------------------------------------------------------------------
 // mbarrier
 // ---------------------------------------------------------------------------------------------
@@ -394,6 +405,13 @@ __device__ __forceinline__ uint64_t make_smem_desc_rows16(uint32_t smem_addr) {
 //   [23] scale format (1 = e8m0)   [24,29) M >> 4   [29,31) byte of the scale-factor column used for A
 __host__ __device__ constexpr uint32_t make_idesc_mxf8(int m, int n) {
   return (static_cast<uint32_t>(n >> 3) << 17) | (1u << 23) | (static_cast<uint32_t>(m >> 4) << 24);
+}
+
+// 2^x on the special-function unit (denormal results are flushed to zero)
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
 }
 
 // pack two floats into one bf16x2 register (lo = a, hi = b)

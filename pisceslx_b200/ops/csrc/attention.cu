@@ -105,31 +105,36 @@ int launch_attn_bwd(const AttnBwdArgs& b, cudaStream_t stream) {
   p.scale_log2 = a.scale * kLog2eHost;
   p.status = a.status;
 
-  const int64_t warps = a.total_q * a.hq;
-  attn_delta_kernel<<<static_cast<unsigned>((warps + 7) / 8), 256, 0, stream>>>(
-      reinterpret_cast<const __nv_bfloat16*>(a.o), reinterpret_cast<const __nv_bfloat16*>(b.dout), b.delta,
-      a.total_q, a.hq, a.d, a.o_stride, b.do_stride);
+  // the tensor maps have seen to 16-byte alignment of dO
+  const int64_t lanes = a.total_q * a.hq * (a.d / 8);
+  const unsigned grid_d = static_cast<unsigned>((lanes + 255) / 256);
+  const bool vec = (reinterpret_cast<uintptr_t>(a.o) & 15u) == 0 && (a.o_stride & 7) == 0;
+  auto delta_kernel = a.d == 128 ? (vec ? attn_delta_kernel<128, true> : attn_delta_kernel<128, false>)
+                                 : (vec ? attn_delta_kernel<64, true> : attn_delta_kernel<64, false>);
+  delta_kernel<<<grid_d, 256, 0, stream>>>(reinterpret_cast<const __nv_bfloat16*>(a.o),
+                                           reinterpret_cast<const __nv_bfloat16*>(b.dout), b.delta, a.total_q, a.hq,
+                                           a.o_stride, b.do_stride);
 
   dim3 grid_q((a.max_q + 127) / 128, a.hq, a.batch);
   dim3 grid_k((a.max_k + 127) / 128, a.hk, a.batch);
   if (a.d == 128) {
     static PerDeviceInt cfg;
     if (!cfg.cur()) {
-      r = set_smem(attn_bwd_dq_kernel<128>, AttnBwdSmem<128>::kTotal); if (r) return r;
+      r = set_smem(attn_bwd_dq_kernel<128>, AttnBwdSmem<128>::kTotalDQ); if (r) return r;
       r = set_smem(attn_bwd_dkv_kernel<128>, AttnBwdSmem<128>::kTotal); if (r) return r;
       cfg.cur() = 1;
     }
     attn_bwd_dkv_kernel<128><<<grid_k, kAttnBwdThreads, AttnBwdSmem<128>::kTotal, stream>>>(p);
-    attn_bwd_dq_kernel<128><<<grid_q, kAttnBwdThreads, AttnBwdSmem<128>::kTotal, stream>>>(p);
+    attn_bwd_dq_kernel<128><<<grid_q, kAttnBwdThreads, AttnBwdSmem<128>::kTotalDQ, stream>>>(p);
   } else {
     static PerDeviceInt cfg;
     if (!cfg.cur()) {
-      r = set_smem(attn_bwd_dq_kernel<64>, AttnBwdSmem<64>::kTotal); if (r) return r;
+      r = set_smem(attn_bwd_dq_kernel<64>, AttnBwdSmem<64>::kTotalDQ); if (r) return r;
       r = set_smem(attn_bwd_dkv_kernel<64>, AttnBwdSmem<64>::kTotal); if (r) return r;
       cfg.cur() = 1;
     }
     attn_bwd_dkv_kernel<64><<<grid_k, kAttnBwdThreads, AttnBwdSmem<64>::kTotal, stream>>>(p);
-    attn_bwd_dq_kernel<64><<<grid_q, kAttnBwdThreads, AttnBwdSmem<64>::kTotal, stream>>>(p);
+    attn_bwd_dq_kernel<64><<<grid_q, kAttnBwdThreads, AttnBwdSmem<64>::kTotalDQ, stream>>>(p);
   }
   return static_cast<int>(cudaGetLastError());
 }

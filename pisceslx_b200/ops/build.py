@@ -19,12 +19,12 @@ CSRC = HERE / "csrc"
 OBJ = HERE / "build"
 SO = HERE / "_yv_ops.so"
 
-CUDA_SOURCES = ["gemm.cu", "elementwise.cu", "moe.cu", "loss_optim.cu", "attention.cu", "comm.cu", "noalloc.cu", "ssm.cu", "pq_film.cu",
+CUDA_SOURCES = ["gemm.cu", "skinny.cu", "elementwise.cu", "moe.cu", "loss_optim.cu", "attention.cu", "comm.cu", "noalloc.cu", "ssm.cu", "pq_film.cu",
                 "stream.cu", "latent.cu", "grouped.cu"]
 CPP_SOURCES = ["binding.cpp"]
 # Layered models can be served by a library of their own: the products and the stream, and the operators of their mixers.
 FAMILIES = {"latent_attention": ["latent.cu"], "grouped_attention": ["grouped.cu"]}
-LAYERED_CUDA_SOURCES = ["gemm.cu", "stream.cu"]
+LAYERED_CUDA_SOURCES = ["gemm.cu", "skinny.cu", "skinny.cu", "stream.cu"]
 LAYERED_CPP_SOURCES = ["binding_layered.cpp"]
 LAYERED_DEFINES = {"gemm.cu": ["-DYV_SERVING_PRODUCTS"]}
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",

@@ -61,6 +61,35 @@ void gemm_grouped_k(const Tensor& a, const Tensor& b, Tensor c, const Tensor& se
   g.status = statusp(status);
   check_rc(yv::launch_gemm(g, cur_stream()), "gemm_grouped_k");
 }
+// Grouped along M with few tokens per expert, of which live rows alone are read and written: x [rows, K] in the layout of
+// the dispatch plan, w [E, N, K] (swiglu: [E, 2 N, K], gate rows then up rows, N a multiple of 64), out [rows, N].
+// `slots` is the number of tokens per expert to prepare for; experts with more take several passes.
+void gemm_skinny_grouped(const Tensor& x, const Tensor& w, Tensor out, const Tensor& tile_expert, const Tensor& num_m_tiles,
+                         const Tensor& seg_offsets, const Tensor& counts, int64_t slots, bool swiglu,
+                         const c10::optional<Tensor>& status) {
+  check_bf16(x, "x"); check_bf16(w, "w"); check_bf16(out, "out");
+  check_i32(tile_expert, "tile_expert"); check_i32(num_m_tiles, "num_m_tiles");
+  check_i32(seg_offsets, "seg_offsets"); check_i32(counts, "counts");
+  TORCH_CHECK(x.dim() == 2 && w.dim() == 3 && out.dim() == 2 && x.is_contiguous() && w.is_contiguous() &&
+              out.is_contiguous() && x.size(1) == w.size(2) && x.size(0) == out.size(0),
+              "gemm_skinny_grouped: contiguous x[rows,K], w[E,*,K], out[rows,N] expected");
+  TORCH_CHECK(w.size(1) == out.size(1) * (swiglu ? 2 : 1), "gemm_skinny_grouped: output width");
+  TORCH_CHECK(x.size(0) % 128 == 0 && tile_expert.numel() * 128 >= x.size(0) && seg_offsets.numel() == w.size(0) + 1 &&
+              counts.numel() == w.size(0), "gemm_skinny_grouped: dispatch plan");
+  TORCH_CHECK((reinterpret_cast<uintptr_t>(out.data_ptr()) & 15u) == 0, "gemm_skinny_grouped: out not aligned");
+  const c10::cuda::CUDAGuard guard(x.device());
+  yv::SkinnyArgs a;
+  a.x = x.data_ptr(); a.w = w.data_ptr(); a.out = out.data_ptr();
+  a.x_rows = x.size(0); a.ldx = x.size(1); a.ldw = w.size(2); a.ldo = out.size(1);
+  a.N = static_cast<int>(out.size(1)); a.K = static_cast<int>(x.size(1));
+  a.experts = static_cast<int>(w.size(0)); a.max_tiles = static_cast<int>(x.size(0) / 128);
+  a.slots = static_cast<int>(slots); a.swiglu = swiglu ? 1 : 0;
+  a.tile_expert = tile_expert.data_ptr<int>(); a.num_m_tiles = num_m_tiles.data_ptr<int>();
+  a.seg_offsets = seg_offsets.data_ptr<int>(); a.counts = counts.data_ptr<int>();
+  a.status = statusp(status);
+  check_rc(yv::launch_skinny(a, cur_stream()), "gemm_skinny_grouped");
+}
+
 // c[g] = ec * (a[g] @ b[g]^T) + eb * cin[g] + ea * I   (square [n, n] outputs, n a multiple of 128): the
 // Newton-Schulz polynomial b A + c A^2 + a I formed in the epilogue of the A A product
 void gemm_batched_affine(const Tensor& a, const Tensor& b, const Tensor& cin, Tensor c, double ea, double eb, double ec,

@@ -1,0 +1,94 @@
+// Host side of the few-token products: tensor maps, number of K slices, choice of the token slots.
+#include "per_device.h"
+#include "skinny.cuh"
+#include "tensormap.h"
+#include "yv_ops.h"
+
+namespace yv {
+
+namespace {
+
+int sm_count() {
+  static PerDeviceInt n;
+  int& v = n.cur();
+  if (v == 0) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+    if (v <= 0) v = 148;
+  }
+  return v;
+}
+
+template <int NT, int MODE>
+int launch(const SkinnyParams& p, int grid, int cluster, cudaStream_t stream) {
+  auto kern = skinny_kernel<NT, MODE>;
+  static PerDeviceInt configured;
+  if (!configured.cur()) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SkinnySmem<NT>::kTotal);
+    if (e != cudaSuccess) return static_cast<int>(e);
+    configured.cur() = 1;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(grid));
+  cfg.blockDim = dim3(kSkThreads);
+  cfg.dynamicSmemBytes = SkinnySmem<NT>::kTotal;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = static_cast<unsigned>(cluster);
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return static_cast<int>(cudaLaunchKernelEx(&cfg, kern, p));
+}
+
+template <int MODE>
+int dispatch(int tokens, const SkinnyParams& p, int grid, int cluster, cudaStream_t stream) {
+  if (tokens <= 16) return launch<16, MODE>(p, grid, cluster, stream);
+  if (tokens <= 32) return launch<32, MODE>(p, grid, cluster, stream);
+  if (tokens <= 64) return launch<64, MODE>(p, grid, cluster, stream);
+  return launch<128, MODE>(p, grid, cluster, stream);
+}
+
+}  // namespace
+
+int launch_skinny(const SkinnyArgs& a, cudaStream_t stream) {
+  if (a.N <= 0 || a.K <= 0) return -1;
+  SkinnyParams p = {};
+  p.N = a.N; p.K = a.K;
+  p.out = a.out; p.out_fp32 = a.out_fp32; p.ldo = a.ldo;
+  p.bias = static_cast<const __nv_bfloat16*>(a.bias);
+  p.status = a.status;
+  const bool grouped = a.experts > 0;
+  const int rows = a.swiglu ? 64 : kSkRows;
+  p.tiles_w = (a.N + rows - 1) / rows;
+  p.w_rows = a.swiglu ? 2 * a.N : a.N;
+  const uint64_t w_rows = static_cast<uint64_t>(p.w_rows) * static_cast<uint64_t>(grouped ? a.experts : 1);
+  int r = make_tmap_2d(&p.tma_w, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, a.w, a.K, w_rows, a.ldw, 64, rows);
+  if (r != 0) return -20 + r;
+  r = make_tmap_2d(&p.tma_x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, a.x, a.K, a.x_rows, a.ldx, 64, 16);
+  if (r != 0) return -30 + r;
+  if (!grouped) {
+    if (a.M < 1 || a.M > 128 || a.swiglu) return -2;
+    p.M = a.M;
+    // as many slices of K as keep all CTAs resident (two per SM) and leave four 64-wide steps to each
+    const int kc = (a.K + 63) / 64, room = 2 * sm_count() / p.tiles_w;
+    int slices = 1;
+    for (int s : {2, 3, 4, 6, 8})
+      if (s <= room && s * 4 <= kc) slices = s;
+    return dispatch<0>(a.M, p, p.tiles_w * slices, slices, stream);
+  }
+  // a tile that reached into the next expert's rows would compute with them; its outputs past N are dropped, the gate and up
+  // halves of a fused tile must be whole
+  if (a.out_fp32 || a.bias != nullptr || (a.swiglu && a.N % 64 != 0)) return -3;
+  p.tile_expert = a.tile_expert; p.num_m_tiles = a.num_m_tiles;
+  p.seg_offsets = a.seg_offsets; p.counts = a.counts;
+  const int64_t units = static_cast<int64_t>(a.max_tiles) * p.tiles_w, room = 2 * sm_count();
+  const int grid = static_cast<int>(units < room ? units : room);
+  if (grid <= 0) return 0;
+  return a.swiglu ? dispatch<2>(a.slots, p, grid, 1, stream) : dispatch<1>(a.slots, p, grid, 1, stream);
+}
+
+}  // namespace yv

@@ -1,0 +1,352 @@
+// Products of a few token rows with large weights (decoding, short prompts): out[t, n] = sum_k x[t, k] * w[n, k].
+//
+// Every weight is used by at most 128 tokens, so the time is that of streaming the weights from HBM.  The operands are
+// swapped against the general kernel: 128 weight rows fill the M side of tcgen05.mma and the tokens, padded to 16, the N
+// side, so that shared memory and the L2 carry weights and not the rows of an empty 128-row token tile, and nothing but
+// live outputs is written.  Two CTAs per SM, about 100 KB of loads in flight each.
+//
+//   dense    One CTA per (128 weight rows, slice of K); the slices of a tile form a cluster and add their fp32 sums, in
+//            the order of the slices, through distributed shared memory: no workspace, no second kernel.  The number of
+//            slices depends on N and K alone, so a row's result does not depend on the rows it is batched with.
+//   grouped  Persistent CTAs over (tile of <= 128 tokens of one expert, 128 weight rows).  With SWIGLU the 128 rows are 64
+//            gate rows and their 64 up rows, and silu(gate) * up leaves the kernel; the products stay in fp32 until then.
+//
+// Bound by HBM and, for the smaller matrices, by about 5 us of start and end.  Measured in a graph, weights not in L2, one
+// token (before: the split of K by the general kernel and a second kernel that added the parts): 11264 x 4096 18.7 us,
+// 32000 x 4096 44.7 us (5.9 TB/s; before 57), 6144 x 4096 16.4, 4096 x 4096 10.8, 4096 x 5632 12.5, 64 x 4096 5.5 (before 18);
+// 64 experts of 4096 x 1408 with 64 tokens, top-6, both products and the activation 350 us (6.3 TB/s; before 435).
+#pragma once
+#include "sm100.cuh"
+
+namespace yv {
+
+struct SkinnyParams {
+  CUtensorMap tma_w;            // [weight rows, K], box 64 x 128 (SWIGLU: 64 x 64)
+  CUtensorMap tma_x;            // [token rows, K], box 64 x 16
+  int M, N, K;                  // dense: tokens; outputs per token (SWIGLU: F); depth
+  int out_fp32;                 // dense only
+  int tiles_w;                  // tiles of weight rows (of one expert)
+  int w_rows;                   // grouped: weight rows per expert
+  void* out;
+  long long ldo;                // elements between output rows
+  const __nv_bfloat16* bias;    // dense, optional
+  const int* tile_expert;       // grouped: the dispatch plan
+  const int* num_m_tiles;
+  const int* seg_offsets;
+  const int* counts;
+  uint32_t* status;
+};
+
+constexpr int kSkThreads = 192;              // TMA producer, MMA issuer, four epilogue warps
+constexpr int kSkRows = 128;                 // weight rows per tile
+constexpr int kSkWBytes = kSkRows * 128;     // one stage of weights: 128 rows x 64 bf16
+constexpr int kSkXBox = 16 * 128;            // 16 tokens x 64 bf16
+constexpr int kSkEpiBytes = 16 * kSkRows * 4;
+
+// NT: token slots (16, 32, 64 or 128).  A tile with more live tokens than slots is worked off in passes.
+template <int NT>
+struct SkinnySmem {
+  static constexpr int kStageBytes = kSkWBytes + (NT / 16) * kSkXBox;
+  static constexpr int kStages = NT == 128 ? 3 : (NT == 64 ? 4 : 5);
+  static constexpr int kRing = kStages * kStageBytes;
+  static constexpr int kTotal = kRing + kSkEpiBytes + 256;       // two CTAs per SM: at most 113 KB each
+  static_assert(kTotal <= 115712 && NT * kSkRows * 4 <= kRing, "two CTAs per SM; the dense sums reuse the ring");
+};
+
+struct SkinnyTile {
+  int w_row, w_row2;            // first weight row (SWIGLU: of the gate rows and of the up rows)
+  int x_row;                    // first token row
+  int cnt;                      // live tokens
+  int col;                      // first output column
+};
+
+template <int MODE>             // 0 dense, 1 grouped, 2 grouped with SWIGLU
+__device__ __forceinline__ bool skinny_tile(const SkinnyParams& p, int unit, int units, SkinnyTile& t) {
+  if (unit >= units) return false;
+  if (MODE == 0) {
+    t.w_row = t.col = unit * kSkRows;
+    t.w_row2 = 0;
+    t.x_row = 0;
+    t.cnt = p.M;
+    return true;
+  }
+  const int j = unit / p.tiles_w, i = unit - j * p.tiles_w;
+  const int e = p.tile_expert[j];
+  t.x_row = j * 128;
+  t.cnt = max(1, min(128, p.seg_offsets[e] + p.counts[e] - t.x_row));
+  if (MODE == 2) {
+    t.col = i * 64;
+    t.w_row = e * p.w_rows + t.col;
+    t.w_row2 = t.w_row + p.N;
+  } else {
+    t.col = i * kSkRows;
+    t.w_row = e * p.w_rows + t.col;
+    t.w_row2 = 0;
+  }
+  return true;
+}
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr, uint32_t rank) {
+  float4 v;
+  asm volatile(
+      "{\n"
+      ".reg .b32 ra;\n"
+      "mapa.shared::cluster.u32 ra, %4, %5;\n"
+      "ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [ra];\n"
+      "}\n"
+      : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+      : "r"(addr), "r"(rank)
+      : "memory");
+  return v;
+}
+
+// Four consecutive outputs of one token; columns at or past `n` are dropped.
+__device__ __forceinline__ void skinny_store4(void* out, int fp32, long long at, int col, int n, float4 v) {
+  float f[4] = {v.x, v.y, v.z, v.w};
+  const bool whole = col + 4 <= n && (at & 3) == 0;
+  if (fp32) {
+    float* o = static_cast<float*>(out) + at;
+    if (whole) {
+      *reinterpret_cast<float4*>(o) = v;
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (col + i < n) o[i] = f[i];
+    }
+  } else {
+    __nv_bfloat16* o = static_cast<__nv_bfloat16*>(out) + at;
+    if (whole) {
+      *reinterpret_cast<uint2*>(o) = make_uint2(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]));
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (col + i < n) o[i] = __float2bfloat16(f[i]);
+    }
+  }
+}
+
+template <int NT, int MODE>
+__global__ void __launch_bounds__(kSkThreads, 2) skinny_kernel(const __grid_constant__ SkinnyParams p) {
+  using S = SkinnySmem<NT>;
+  constexpr int kStages = S::kStages;
+  constexpr int kAccBufs = MODE == 0 ? 1 : 2;
+  constexpr uint32_t kTmemCols = kAccBufs * NT < 32 ? 32 : kAccBufs * NT;
+
+  extern __shared__ __align__(1024) uint8_t skinny_smem[];
+  uint8_t* smem = skinny_smem;
+  float* epi = reinterpret_cast<float*>(smem + S::kRing);
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + S::kRing + kSkEpiBytes);
+  uint64_t* empty_bar = full_bar + kStages;
+  uint64_t* acc_full = empty_bar + kStages;
+  uint64_t* acc_empty = acc_full + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // the swizzled tiles need shared memory that starts on 1024 bytes
+  if ((smem_u32(smem) & 1023u) != 0u) {
+    if (threadIdx.x == 0 && p.status != nullptr) atomicOr(p.status, kStatusBadArgument);
+    return;
+  }
+  const int kc = (p.K + 63) / 64;
+  int slices = 1, slice = 0, units, first, step;
+  if (MODE == 0) {
+    uint32_t n;
+    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(n));
+    slices = static_cast<int>(n);
+    slice = static_cast<int>(cluster_rank());
+    first = static_cast<int>(blockIdx.x) / slices;
+    units = p.tiles_w;
+    step = units;                                  // one tile per cluster
+  } else {
+    units = *p.num_m_tiles * p.tiles_w;
+    first = blockIdx.x;
+    step = gridDim.x;
+  }
+  const int k0 = kc * slice / slices, k1 = kc * (slice + 1) / slices;
+
+  if (threadIdx.x == 0) {
+    tma_prefetch_desc(&p.tma_w);
+    tma_prefetch_desc(&p.tma_x);
+    for (int s = 0; s < kStages; ++s) {
+      mbar_init(&full_bar[s], 1);
+      mbar_init(&empty_bar[s], 1);
+    }
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&acc_full[s], 1);
+      mbar_init(&acc_empty[s], 1);
+    }
+    fence_barrier_init();
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, kTmemCols);
+    tmem_relinquish();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;
+
+  if (warp == 0) {
+    if (elect_one()) {
+      uint32_t it = 0;
+      bool ok = true;
+      SkinnyTile t;
+      for (int u = first; ok && skinny_tile<MODE>(p, u, units, t); u += step) {
+        for (int at = 0; ok && at < t.cnt; at += NT) {
+          const int boxes = (min(NT, t.cnt - at) + 15) / 16;
+          const uint32_t bytes = kSkWBytes + static_cast<uint32_t>(boxes) * kSkXBox;
+          for (int k = k0; k < k1; ++k, ++it) {
+            const int s = it % kStages;
+            ok = mbar_wait(&empty_bar[s], ((it / kStages) & 1u) ^ 1u, p.status);
+            if (!ok) break;
+            uint8_t* sw = smem + s * S::kStageBytes;
+            uint8_t* sx = sw + kSkWBytes;
+            mbar_expect_tx(&full_bar[s], bytes);
+            tma_load_2d(sw, &p.tma_w, &full_bar[s], k * 64, t.w_row);
+            if (MODE == 2) tma_load_2d(sw + kSkWBytes / 2, &p.tma_w, &full_bar[s], k * 64, t.w_row2);
+            for (int b = 0; b < boxes; ++b)
+              tma_load_2d(sx + b * kSkXBox, &p.tma_x, &full_bar[s], k * 64, t.x_row + at + 16 * b);
+          }
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (elect_one()) {
+      uint32_t it = 0, tile_it = 0;
+      bool ok = true;
+      SkinnyTile t;
+      for (int u = first; ok && skinny_tile<MODE>(p, u, units, t); u += step) {
+        for (int at = 0; ok && at < t.cnt; at += NT, ++tile_it) {
+          const int acc = tile_it % kAccBufs;
+          ok = mbar_wait(&acc_empty[acc], ((tile_it / kAccBufs) & 1u) ^ 1u, p.status);
+          if (!ok) break;
+          tc_fence_after_sync();
+          const uint32_t tmem_d = tmem_base + static_cast<uint32_t>(acc * NT);
+          const uint32_t idesc = make_idesc_bf16(kSkRows, ((min(NT, t.cnt - at) + 15) / 16) * 16, false, false);
+          for (int k = k0; k < k1; ++k, ++it) {
+            const int s = it % kStages;
+            ok = mbar_wait(&full_bar[s], (it / kStages) & 1u, p.status);
+            if (!ok) break;
+            tc_fence_after_sync();
+            const uint32_t sw = smem_u32(smem + s * S::kStageBytes), sx = sw + kSkWBytes;
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk)
+              tc_mma_f16_ss(tmem_d, make_smem_desc(sw + kk * 32, 16, 1024), make_smem_desc(sx + kk * 32, 16, 1024), idesc,
+                            (k > k0 || kk > 0) ? 1u : 0u);
+            tc_commit(&empty_bar[s]);
+          }
+          if (ok) tc_commit(&acc_full[acc]);
+        }
+      }
+    }
+  } else {
+    const int quarter = warp & 3;                  // TMEM lane quarter of this warp
+    const int row = quarter * 32 + lane;           // weight row of the tile
+    const int tid = static_cast<int>(threadIdx.x) - 64;
+    uint32_t tile_it = 0;
+    SkinnyTile t;
+    bool live = true;
+    for (int u = first; live && skinny_tile<MODE>(p, u, units, t); u += step) {
+      for (int at = 0; at < t.cnt; at += NT, ++tile_it) {
+        const int acc = tile_it % kAccBufs, cnt = min(NT, t.cnt - at);
+        uint32_t ok = mbar_wait(&acc_full[acc], (tile_it / kAccBufs) & 1u, p.status) ? 1u : 0u;
+        asm volatile(
+            "{\n"
+            ".reg .pred pin, pout;\n"
+            "setp.ne.u32 pin, %0, 0;\n"
+            "bar.red.and.pred pout, 1, 128, pin;\n"
+            "selp.u32 %0, 1, 0, pout;\n"
+            "}\n"
+            : "+r"(ok)::"memory");
+        live = ok != 0u;
+        if (!live) break;
+        tc_fence_after_sync();
+        const uint32_t taddr = tmem_base + static_cast<uint32_t>(acc * NT) + (static_cast<uint32_t>(quarter * 32) << 16);
+        const int boxes = (cnt + 15) / 16;
+        for (int b = 0; b < boxes; ++b) {
+          uint32_t v[16];
+          tmem_ld16(taddr + 16 * b, v);
+          tc_wait_ld();
+          // staged as [token][weight row], so that consecutive threads write consecutive outputs of one token
+          float* st = MODE == 0 ? reinterpret_cast<float*>(smem) + 16 * b * kSkRows : epi;
+          if (MODE != 0 && b > 0) asm volatile("bar.sync 1, 128;" ::: "memory");
+#pragma unroll
+          for (int i = 0; i < 16; ++i) st[i * kSkRows + row] = __uint_as_float(v[i]);
+          if (MODE == 0) continue;
+          asm volatile("bar.sync 1, 128;" ::: "memory");
+          constexpr int kQuads = MODE == 2 ? 16 : 32;          // groups of four outputs per token
+#pragma unroll
+          for (int i = 0; i < 16 * kQuads / 128; ++i) {
+            const int w = i * 128 + tid, tok = w / kQuads, c = (w % kQuads) * 4;
+            float4 o = *reinterpret_cast<const float4*>(st + tok * kSkRows + c);
+            if (MODE == 2) {
+              const float4 up = *reinterpret_cast<const float4*>(st + tok * kSkRows + 64 + c);
+              o.x = o.x / (1.f + __expf(-o.x)) * up.x;
+              o.y = o.y / (1.f + __expf(-o.y)) * up.y;
+              o.z = o.z / (1.f + __expf(-o.z)) * up.z;
+              o.w = o.w / (1.f + __expf(-o.w)) * up.w;
+            }
+            if (16 * b + tok < cnt)
+              skinny_store4(p.out, 0, (t.x_row + at + 16 * b + tok) * p.ldo + t.col + c, t.col + c, p.N, o);
+          }
+        }
+        tc_fence_before_sync();
+        asm volatile("bar.sync 1, 128;" ::: "memory");         // all of the accumulator and the staging have been read
+        if (tid == 0) mbar_arrive(&acc_empty[acc]);
+      }
+    }
+  }
+
+  __syncwarp();                                    // the aligned barriers below need whole warps
+  tc_fence_before_sync();
+  if (MODE == 0) {
+    cluster_sync_all();                            // every slice's sums are in its shared memory
+    const bool bad = p.status != nullptr && *reinterpret_cast<volatile uint32_t*>(p.status) != 0u;
+    const uint32_t base = smem_u32(smem);
+    const int col0 = first * kSkRows;
+    for (int w = slice * kSkThreads + static_cast<int>(threadIdx.x); !bad && w < p.M * 32; w += slices * kSkThreads) {
+      const int tok = w >> 5, c = (w & 31) * 4;
+      const uint32_t at = base + static_cast<uint32_t>(tok * kSkRows + c) * 4u;
+      float4 v[8];
+#pragma unroll
+      for (int s = 0; s < 8; ++s)
+        if (s < slices) v[s] = ld_cluster_f4(at, static_cast<uint32_t>(s));
+      float4 o = v[0];
+#pragma unroll
+      for (int s = 1; s < 8; ++s)
+        if (s < slices) { o.x += v[s].x; o.y += v[s].y; o.z += v[s].z; o.w += v[s].w; }
+      const int col = col0 + c;
+      if (col >= p.N) continue;
+      if (p.bias != nullptr) {
+        o.x += __bfloat162float(p.bias[col]);
+        if (col + 1 < p.N) o.y += __bfloat162float(p.bias[col + 1]);
+        if (col + 2 < p.N) o.z += __bfloat162float(p.bias[col + 2]);
+        if (col + 3 < p.N) o.w += __bfloat162float(p.bias[col + 3]);
+      }
+      skinny_store4(p.out, p.out_fp32, tok * p.ldo + col, col, p.N, o);
+    }
+    cluster_sync_all();                            // nobody reads this CTA's shared memory any more
+  } else {
+    __syncthreads();
+  }
+  if (p.status != nullptr && *reinterpret_cast<volatile uint32_t*>(p.status) != 0u) {
+    // a wait ran out somewhere: let loads in flight land before shared memory and TMEM are released
+    const uint64_t t0 = globaltimer_ns();
+    while (globaltimer_ns() - t0 < 200000ull) { __nanosleep(1000); }
+    __syncthreads();
+  }
+  if (warp == 1) {
+    tc_fence_after_sync();
+    tmem_dealloc(tmem_base, kTmemCols);
+  }
+}
+
+}  // namespace yv

@@ -129,9 +129,23 @@ int launch_ssm_scan_fwd(const float* u, const float* delta, const float* A, cons
 int launch_ssm_scan_bwd(const float* u, const float* delta, const float* A, const float* Bm, const float* Cm,
                         const float* Dp, const float* hs, const float* dy, float* du, float* ddelta, float* dA,
                         float* dB, float* dC, float* dD, int batch, int L, int D, int N, cudaStream_t stream);
-// out[M,N] (bf16) = sum over slices of ws[slice][m_pad, N] (fp32) (+ bias[N]): second half of a split-K product
-int launch_splitk_reduce(const float* ws, const void* bias, void* out, int slices, int M, int m_pad, int N,
-                         cudaStream_t stream);
+// Products of few token rows with large weights (skinny.cu): out[t, n] = sum_k x[t, k] * w[n, k].
+struct SkinnyArgs {
+  const void* x = nullptr;             // [x_rows, K] bf16, pitch ldx
+  const void* w = nullptr;             // [N, K] bf16, pitch ldw; grouped: [experts, N (swiglu: 2 N), K]
+  void* out = nullptr;                 // [x_rows, N], pitch ldo
+  const void* bias = nullptr;          // dense: bf16 [N]
+  int64_t x_rows = 0, ldx = 0, ldw = 0, ldo = 0;
+  int M = 0, N = 0, K = 0;             // M: dense, 1..128 tokens
+  int out_fp32 = 0;
+  // grouped over experts: the dispatch plan of a 128-row-padded token layout
+  int experts = 0, max_tiles = 0;
+  int slots = 0;                       // tokens per pass (rounded up to 16, 32, 64 or 128); any count per tile is right
+  int swiglu = 0;
+  const int *tile_expert = nullptr, *num_m_tiles = nullptr, *seg_offsets = nullptr, *counts = nullptr;
+  uint32_t* status = nullptr;
+};
+int launch_skinny(const SkinnyArgs& a, cudaStream_t stream);
 
 // ------------------------------------------------------------------------------------------------
 // MoE routing (moe.cu)

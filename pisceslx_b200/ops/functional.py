@@ -88,14 +88,17 @@ def _splitk_setup(x2: torch.Tensor, w: torch.Tensor) -> Optional[Tuple[int, torc
     return slices, ws, offs
 
 
-def gemm_skinny(x2: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None) -> Optional[torch.Tensor]:
-    """y = x2 @ w.T through the split-K path, or None when the shape does not call for it."""
-    plan = _splitk_setup(x2, w)
-    if plan is None:
+def gemm_skinny(x2: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None,
+                out_dtype: torch.dtype = _BF16) -> Optional[torch.Tensor]:
+    """y = x2 @ w.T (+ bias) of up to 128 rows by the kernel that streams the weights once, or None when the operands are
+    not what it reads.  A row's result does not depend on the rows beside it.
+
+    The line lies at 128 rows, one tile of tokens: up to there the time is that of reading the weights."""
+    M, K = x2.shape
+    if not 1 <= M <= 128 or K == 0 or w.shape[0] == 0 or w.stride(1) != 1 or x2.stride(1) != 1:
         return None
-    _, ws, offs = plan
-    out = torch.empty(x2.shape[0], w.shape[0], dtype=_BF16, device=x2.device)
-    _k().gemm_splitk(x2, w, ws, offs, bias, out, _st(x2))
+    out = torch.empty(M, w.shape[0], dtype=out_dtype, device=x2.device)
+    _k().gemm_skinny(x2, w, bias, out, _st(x2))
     return out
 
 
@@ -106,7 +109,7 @@ def skinny_parts(x2: torch.Tensor, w: torch.Tensor) -> Optional[torch.Tensor]:
     if plan is None:
         return None
     slices, ws, offs = plan
-    _k().gemm_splitk(x2, w, ws, offs, None, None, _st(x2))
+    _k().gemm_splitk(x2, w, ws, offs, _st(x2))
     return ws[:slices * 128 * w.shape[0]].view(slices, 128, w.shape[0])
 
 
@@ -118,11 +121,10 @@ class _LinearFn(torch.autograd.Function):
             x2 = x2.contiguous()
         ctx.save_for_backward(x2, w)
         ctx.x_shape = x.shape
-        if not out_fp32 and x2.shape[0] <= 128:
-            ys = gemm_skinny(x2, w)
-            if ys is not None:
-                return ys.view(*x.shape[:-1], w.shape[0])
-        y = gemm(x2, w, out_dtype=torch.float32 if out_fp32 else _BF16)
+        out_dtype = torch.float32 if out_fp32 else _BF16
+        y = gemm_skinny(x2, w, None, out_dtype)
+        if y is None:
+            y = gemm(x2, w, out_dtype=out_dtype)
         return y.view(*x.shape[:-1], w.shape[0])
 
     @staticmethod

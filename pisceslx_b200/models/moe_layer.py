@@ -81,29 +81,31 @@ class YvDeepSeekMoELayer(nn.Module):
     # ------------------------------------------------------------------------------------------------
     def _shared(self, x: torch.Tensor) -> torch.Tensor:
         S, Fs = self.num_shared, self.shared_ffn
-        T = x.shape[0]
+        sw = self.shared_expert_weight
+        if torch.is_grad_enabled():
+            mix = torch.softmax(sw.float(), 0)
+        else:
+            # serving: the mixing weights change only when the parameter does; keep them instead of running a softmax and
+            # two casts per layer per decode step
+            key = (sw.data_ptr(), sw._version, x.dtype)
+            cached = getattr(self, "_mix_cache", None)
+            if cached is None or cached[0] != key:
+                mix = torch.softmax(sw.detach().float(), 0)
+                cached = (key, mix, mix.to(x.dtype))
+                self._mix_cache = cached
+            mix = cached[1]
+        act = None
         if self.tp_size > 1:
             from ..parallel import tp
             y1 = tp.allgather_linear(x, self.shared_w13, self.tp_group)
         else:
-            y1 = F_.linear(x, self.shared_w13)
-        T = y1.shape[0]
-        act = F_.swiglu(y1.view(T * S, 2 * Fs)).view(T, S, Fs)
-        if S > 1 or self.shared_expert_weight.requires_grad:
-            sw = self.shared_expert_weight
-            if torch.is_grad_enabled():
-                mix = torch.softmax(sw.float(), 0).to(act.dtype)
-            else:
-                # serving: the mixing weights change only when the parameter does; keep them instead of running a
-                # softmax and two casts per layer per decode step
-                key = (sw.data_ptr(), sw._version, act.dtype)
-                cached = getattr(self, "_mix_cache", None)
-                if cached is None or cached[0] != key:
-                    cached = (key, torch.softmax(sw.detach().float(), 0).to(act.dtype))
-                    self._mix_cache = cached
-                mix = cached[1]
-            act = act * mix.view(1, S, 1)
-        act = act.reshape(T, S * Fs)
+            if x.is_cuda and not torch.is_grad_enabled():
+                act = F_.skinny_swiglu(x, self.shared_w13, Fs, cached[2])
+            y1 = F_.linear(x, self.shared_w13) if act is None else None
+        if act is None:
+            T = y1.shape[0]
+            act = F_.swiglu_mix(y1.view(T * S, 2 * Fs), mix)
+        act = act.reshape(-1, S * Fs)
         if self.tp_size > 1:
             from ..parallel import tp
             return tp.linear_reduce_scatter(act, self.shared_w2, self.tp_group)
@@ -115,22 +117,21 @@ class YvDeepSeekMoELayer(nn.Module):
         x = x.reshape(-1, shape[-1])
         weights, idx, aux = self.router(x)
         counts = self.router.last_counts
+        sh = self._shared(x) if self.num_shared else None
         if self.ep_size > 1:
             from ..parallel import ep
-            routed = ep.moe_experts_ep(x, self.experts_w13, self.experts_w2, weights, idx, self.num_experts,
-                                       self.ep_group, fused=self.cfg.fused_comm, deterministic=self.deterministic,
-                                       counts=counts)
+            out = ep.moe_experts_ep(x, self.experts_w13, self.experts_w2, weights, idx, self.num_experts,
+                                    self.ep_group, fused=self.cfg.fused_comm, deterministic=self.deterministic,
+                                    counts=counts)
+            if sh is not None:
+                out = out + sh
         else:
-            routed = moe_ops.moe_experts(x, self.experts_w13, self.experts_w2, weights, idx, counts,
-                                         self.deterministic, fp8=getattr(self.cfg, "expert_fp8", None))
-        out = routed
-        if self.num_shared:
-            sh = self._shared(x)
-            out = out + sh
-            if self.skip_prev:
-                if self._prev_shared is not None and self._prev_shared.shape == sh.shape:
-                    out = out + 0.1 * self._prev_shared
-                self._prev_shared = sh.detach()
+            out = moe_ops.moe_experts(x, self.experts_w13, self.experts_w2, weights, idx, counts,
+                                      self.deterministic, fp8=getattr(self.cfg, "expert_fp8", None), add=sh)
+        if sh is not None and self.skip_prev:
+            if self._prev_shared is not None and self._prev_shared.shape == sh.shape:
+                out = out + 0.1 * self._prev_shared
+            self._prev_shared = sh.detach()
         return out.view(shape), aux
 
     # ------------------------------------------------------------------------------------------------

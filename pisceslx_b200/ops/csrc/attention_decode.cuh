@@ -180,20 +180,41 @@ __global__ void __launch_bounds__(128) paged_decode_kernel(const PagedDecodePara
 template <int D>
 __global__ void paged_decode_merge_kernel(const float* __restrict__ partial_o, const float* __restrict__ partial_ml,
                                           __nv_bfloat16* __restrict__ o, int64_t heads_total, int splits) {
+  // D / 32 columns a lane; lane s weighs ranges s, s + 32, ...: one read of (m, l) each instead of a chain of them, and eight
+  // rows of partials in flight.
+  constexpr int V = D / 32;
   const int lane = threadIdx.x & 31;
   const int64_t w = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (w >= heads_total) return;
+  const float2* ml = reinterpret_cast<const float2*>(partial_ml) + w * splits;
   float mm = -1.0e29f;
-  for (int s = 0; s < splits; ++s) mm = fmaxf(mm, partial_ml[(w * splits + s) * 2]);
-  float lt = 0.f;
-  for (int s = 0; s < splits; ++s) lt += partial_ml[(w * splits + s) * 2 + 1] * exp2f(partial_ml[(w * splits + s) * 2] - mm);
-  const float inv = lt > 0.f ? 1.f / lt : 0.f;
-  for (int d = lane; d < D; d += 32) {
-    float t = 0.f;
-    for (int s = 0; s < splits; ++s)
-      t += partial_o[(w * splits + s) * D + d] * exp2f(partial_ml[(w * splits + s) * 2] - mm);
-    o[w * D + d] = __float2bfloat16(t * inv);
+  for (int s = lane; s < splits; s += 32) mm = fmaxf(mm, ml[s].x);
+#pragma unroll
+  for (int i = 16; i > 0; i >>= 1) mm = fmaxf(mm, __shfl_xor_sync(0xFFFFFFFFu, mm, i));
+  float lt = 0.f, acc[V];
+#pragma unroll
+  for (int i = 0; i < V; ++i) acc[i] = 0.f;
+  const float* rows = partial_o + w * splits * D + lane * V;
+  for (int s0 = 0; s0 < splits; s0 += 32) {
+    const int n = min(32, splits - s0);
+    const float2 mine = lane < n ? ml[s0 + lane] : make_float2(-1.0e29f, 0.f);
+    const float f = lane < n ? exp2f(mine.x - mm) : 0.f;
+    lt += f * mine.y;
+#pragma unroll 8
+    for (int s = 0; s < n; ++s) {
+      const float fs = __shfl_sync(0xFFFFFFFFu, f, s);
+      float v[V];
+      if (V == 4) *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(rows + static_cast<int64_t>(s0 + s) * D);
+      else *reinterpret_cast<float2*>(v) = *reinterpret_cast<const float2*>(rows + static_cast<int64_t>(s0 + s) * D);
+#pragma unroll
+      for (int i = 0; i < V; ++i) acc[i] += v[i] * fs;
+    }
   }
+#pragma unroll
+  for (int i = 16; i > 0; i >>= 1) lt += __shfl_xor_sync(0xFFFFFFFFu, lt, i);
+  const float inv = lt > 0.f ? 1.f / lt : 0.f;
+#pragma unroll
+  for (int i = 0; i < V; ++i) o[w * D + lane * V + i] = __float2bfloat16(acc[i] * inv);
 }
 
 // Append new K/V rows into the paged cache: slot = block_id * block + offset.

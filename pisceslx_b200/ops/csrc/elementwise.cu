@@ -303,8 +303,9 @@ __global__ void rope3d_kernel(__nv_bfloat16* __restrict__ q, __nv_bfloat16* __re
 // ---------------------------------------------------------------------------------------------
 // SwiGLU
 // ---------------------------------------------------------------------------------------------
+// `scale` (optional, `period` floats): row r is multiplied by scale[r % period]
 __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat16* __restrict__ out,
-                                  int64_t rows, int F) {
+                                  int64_t rows, int F, const float* __restrict__ scale, int period) {
   const int fv = F >> 3;
   const int64_t total = rows * fv;
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total;
@@ -314,8 +315,9 @@ __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfl
     float g[8], u[8], o[8];
     load8(in + r * 2 * F + c, g);
     load8(in + r * 2 * F + F + c, u);
+    const float f = scale != nullptr ? scale[r % period] : 1.f;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) o[j] = g[j] / (1.f + __expf(-g[j])) * u[j];
+    for (int j = 0; j < 8; ++j) o[j] = f * (g[j] / (1.f + __expf(-g[j])) * u[j]);
     store8(out + r * F + c, o);
   }
 }
@@ -348,17 +350,19 @@ __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ in, const __
 //   in [rows, 2F] (gate | up pre-activations), dact [rows, F] = UNWEIGHTED gradient of the activation,
 //   row_w [rows] = combine weight of the row (0 on pad rows and dropped assignments)
 //   din  [rows, 2F] = row_w * dSwiGLU(in, dact)          (gradient of the up projection's output)
-//   actw [rows, F]  = row_w * SwiGLU(in)                 (B operand of the down projection's weight gradient)
+//   actw [rows, F]  = row_w * SwiGLU(in)                 (B operand of the down projection's weight gradient; optional)
+// `period` > 0: row r has the weight row_w[r % period]
 //   rowdot [rows]   = sum_f SwiGLU(in)[f] * dact[f]      (gradient of the row's combine weight)
 __global__ void swiglu_bwd_rows_kernel(const __nv_bfloat16* __restrict__ in, const __nv_bfloat16* __restrict__ dact,
                                        const float* __restrict__ row_w, __nv_bfloat16* __restrict__ din,
-                                       __nv_bfloat16* __restrict__ actw, float* __restrict__ rowdot, int64_t rows, int F) {
+                                       __nv_bfloat16* __restrict__ actw, float* __restrict__ rowdot, int64_t rows, int F,
+                                       int period) {
   const int lane = threadIdx.x & 31;
   const int fv = F >> 3;
   const int64_t warp0 = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5;
   const int64_t nwarps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
   for (int64_t r = warp0; r < rows; r += nwarps) {
-    const float w = row_w[r];
+    const float w = row_w[period > 0 ? r % period : r];
     float dot = 0.f;
     for (int cv = lane; cv < fv; cv += 32) {
       const int c = cv * 8;
@@ -378,7 +382,7 @@ __global__ void swiglu_bwd_rows_kernel(const __nv_bfloat16* __restrict__ in, con
       }
       store8(din + r * 2 * F + c, dg);
       store8(din + r * 2 * F + F + c, du);
-      store8(actw + r * F + c, a);
+      if (actw != nullptr) store8(actw + r * F + c, a);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
@@ -526,19 +530,19 @@ int launch_rope3d(void* q, void* k, const int* pos_thw, int64_t tokens, int hq, 
   return static_cast<int>(cudaGetLastError());
 }
 
-int launch_swiglu_fwd(const void* in, void* out, int64_t rows, int F, cudaStream_t stream) {
+int launch_swiglu_fwd(const void* in, void* out, int64_t rows, int F, const float* scale, int period, cudaStream_t stream) {
   if (rows <= 0) return 0;
   if ((F & 7) != 0) return -1;
-  swiglu_fwd_kernel<<<grid_for(rows * (F >> 3), 256), 256, 0, stream>>>(YV_BF(in), YV_BFM(out), rows, F);
+  swiglu_fwd_kernel<<<grid_for(rows * (F >> 3), 256), 256, 0, stream>>>(YV_BF(in), YV_BFM(out), rows, F, scale, period);
   return static_cast<int>(cudaGetLastError());
 }
 
 int launch_swiglu_bwd_rows(const void* in, const void* dact, const float* row_w, void* din, void* actw, float* rowdot,
-                           int64_t rows, int F, cudaStream_t stream) {
+                           int64_t rows, int F, int period, cudaStream_t stream) {
   if (rows <= 0) return 0;
   if ((F & 7) != 0) return -1;
   swiglu_bwd_rows_kernel<<<grid_for(rows * 32, 256), 256, 0, stream>>>(YV_BF(in), YV_BF(dact), row_w, YV_BFM(din),
-                                                                      YV_BFM(actw), rowdot, rows, F);
+                                                                      YV_BFM(actw), rowdot, rows, F, period);
   return static_cast<int>(cudaGetLastError());
 }
 

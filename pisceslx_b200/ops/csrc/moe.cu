@@ -272,12 +272,22 @@ __global__ void moe_zero_pad_kernel(__nv_bfloat16* __restrict__ xp, const int* _
   }
 }
 
+// grid (tokens, column parts).  The rows and weights of the token are read once, so that the k row loads go out together;
+// with few tokens the columns are spread over blocks.
 __global__ void moe_combine_kernel(const __nv_bfloat16* __restrict__ y, const int* __restrict__ row_map,
                                    const float* __restrict__ weights, const __nv_bfloat16* __restrict__ add,
                                    __nv_bfloat16* __restrict__ out, int k, int cols) {
+  __shared__ int s_row[kMaxTopK];
+  __shared__ float s_w[kMaxTopK];
   const int64_t t = blockIdx.x;
+  if (threadIdx.x < k) {
+    const float w = weights[t * k + threadIdx.x];
+    s_w[threadIdx.x] = w;
+    s_row[threadIdx.x] = w != 0.f ? row_map[t * k + threadIdx.x] : 0;
+  }
+  __syncthreads();
   const int nvec = cols >> 3;
-  for (int v = threadIdx.x; v < nvec; v += blockDim.x) {
+  for (int v = blockIdx.y * blockDim.x + threadIdx.x; v < nvec; v += gridDim.y * blockDim.x) {
     float acc[8];
     if (add != nullptr) {
       load8(add + t * cols + v * 8, acc);
@@ -285,14 +295,13 @@ __global__ void moe_combine_kernel(const __nv_bfloat16* __restrict__ y, const in
 #pragma unroll
       for (int i = 0; i < 8; ++i) acc[i] = 0.f;
     }
+#pragma unroll 4
     for (int j = 0; j < k; ++j) {
-      const float w = weights[t * k + j];
-      if (w != 0.f) {
-        float r[8];
-        load8(y + static_cast<int64_t>(row_map[t * k + j]) * cols + v * 8, r);
+      const float w = s_w[j];
+      float r[8];
+      load8(y + static_cast<int64_t>(s_row[j]) * cols + v * 8, r);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) acc[i] += w * r[i];
-      }
+      for (int i = 0; i < 8; ++i) acc[i] += w != 0.f ? w * r[i] : 0.f;
     }
     store8(out + t * cols + v * 8, acc);
   }
@@ -549,9 +558,12 @@ int launch_moe_combine(const void* y, const int* row_map, const float* weights, 
                        int64_t tokens, int k, int cols, cudaStream_t stream) {
   if (tokens <= 0) return 0;
   if ((cols & 7) != 0) return -1;
-  const int block = (cols >> 3) >= 256 ? 256 : 128;
-  moe_combine_kernel<<<static_cast<unsigned>(tokens), block, 0, stream>>>(YV_BF(y), row_map, weights, YV_BF(add),
-                                                                          YV_BFM(out), k, cols);
+  if (k > kMaxTopK) return -2;
+  // enough blocks for every SM when the tokens alone are too few
+  const int block = (cols >> 3) >= 256 && tokens >= 148 ? 256 : 128;
+  const unsigned parts = tokens >= 148 ? 1u : static_cast<unsigned>(((cols >> 3) + block - 1) / block);
+  moe_combine_kernel<<<dim3(static_cast<unsigned>(tokens), parts), block, 0, stream>>>(YV_BF(y), row_map, weights, YV_BF(add),
+                                                                                       YV_BFM(out), k, cols);
   return static_cast<int>(cudaGetLastError());
 }
 

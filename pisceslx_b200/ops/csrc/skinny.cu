@@ -71,14 +71,18 @@ int launch_skinny(const SkinnyArgs& a, cudaStream_t stream) {
   r = make_tmap_2d(&p.tma_x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, a.x, a.K, a.x_rows, a.ldx, 64, 16);
   if (r != 0) return -30 + r;
   if (!grouped) {
-    if (a.M < 1 || a.M > 128 || a.swiglu) return -2;
+    if (a.M < 1 || a.M > 128) return -2;
+    if (a.swiglu && (a.seg <= 0 || a.seg % 64 != 0 || a.N % a.seg != 0 || a.bias != nullptr)) return -4;
     p.M = a.M;
+    p.seg = a.seg;
+    p.scale = static_cast<const __nv_bfloat16*>(a.scale);
     // as many slices of K as keep all CTAs resident (two per SM) and leave four 64-wide steps to each
     const int kc = (a.K + 63) / 64, room = 2 * sm_count() / p.tiles_w;
     int slices = 1;
     for (int s : {2, 3, 4, 6, 8})
       if (s <= room && s * 4 <= kc) slices = s;
-    return dispatch<0>(a.M, p, p.tiles_w * slices, slices, stream);
+    const int grid = p.tiles_w * slices;
+    return a.swiglu ? dispatch<3>(a.M, p, grid, slices, stream) : dispatch<0>(a.M, p, grid, slices, stream);
   }
   // a tile that reached into the next expert's rows would compute with them; its outputs past N are dropped, the gate and up
   // halves of a fused tile must be whole

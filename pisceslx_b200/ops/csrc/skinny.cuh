@@ -8,6 +8,7 @@
 //   dense    One CTA per (128 weight rows, slice of K); the slices of a tile form a cluster and add their fp32 sums, in
 //            the order of the slices, through distributed shared memory: no workspace, no second kernel.  The number of
 //            slices depends on N and K alone, so a row's result does not depend on the rows it is batched with.
+//            With SWIGLU as below; a factor per segment of the outputs (a shared expert's weight) may go with it.
 //   grouped  Persistent CTAs over (tile of <= 128 tokens of one expert, 128 weight rows).  With SWIGLU the 128 rows are 64
 //            gate rows and their 64 up rows, and silu(gate) * up leaves the kernel; the products stay in fp32 until then.
 //
@@ -27,6 +28,8 @@ struct SkinnyParams {
   int out_fp32;                 // dense only
   int tiles_w;                  // tiles of weight rows (of one expert)
   int w_rows;                   // grouped: weight rows per expert
+  int seg;                      // dense SWIGLU: outputs per segment (its gate rows are followed by its up rows)
+  const __nv_bfloat16* scale;   // dense SWIGLU, optional: one factor per segment
   void* out;
   long long ldo;                // elements between output rows
   const __nv_bfloat16* bias;    // dense, optional
@@ -60,12 +63,19 @@ struct SkinnyTile {
   int col;                      // first output column
 };
 
-template <int MODE>             // 0 dense, 1 grouped, 2 grouped with SWIGLU
+// MODE: 0 dense, 1 grouped, 2 grouped with SWIGLU, 3 dense with SWIGLU
+__host__ __device__ constexpr bool skinny_dense(int mode) { return mode == 0 || mode == 3; }
+__host__ __device__ constexpr bool skinny_swiglu(int mode) { return mode >= 2; }
+
+__device__ __forceinline__ float swiglu1(float gate, float up) { return gate / (1.f + __expf(-gate)) * up; }
+
+template <int MODE>
 __device__ __forceinline__ bool skinny_tile(const SkinnyParams& p, int unit, int units, SkinnyTile& t) {
   if (unit >= units) return false;
-  if (MODE == 0) {
-    t.w_row = t.col = unit * kSkRows;
-    t.w_row2 = 0;
+  if (skinny_dense(MODE)) {
+    t.col = unit * (MODE == 3 ? 64 : kSkRows);
+    t.w_row = MODE == 3 ? t.col + t.col / p.seg * p.seg : t.col;
+    t.w_row2 = t.w_row + p.seg;
     t.x_row = 0;
     t.cnt = p.M;
     return true;
@@ -137,7 +147,7 @@ template <int NT, int MODE>
 __global__ void __launch_bounds__(kSkThreads, 2) skinny_kernel(const __grid_constant__ SkinnyParams p) {
   using S = SkinnySmem<NT>;
   constexpr int kStages = S::kStages;
-  constexpr int kAccBufs = MODE == 0 ? 1 : 2;
+  constexpr int kAccBufs = skinny_dense(MODE) ? 1 : 2;
   constexpr uint32_t kTmemCols = kAccBufs * NT < 32 ? 32 : kAccBufs * NT;
 
   extern __shared__ __align__(1024) uint8_t skinny_smem[];
@@ -157,7 +167,7 @@ __global__ void __launch_bounds__(kSkThreads, 2) skinny_kernel(const __grid_cons
   }
   const int kc = (p.K + 63) / 64;
   int slices = 1, slice = 0, units, first, step;
-  if (MODE == 0) {
+  if (skinny_dense(MODE)) {
     uint32_t n;
     asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(n));
     slices = static_cast<int>(n);
@@ -211,7 +221,7 @@ __global__ void __launch_bounds__(kSkThreads, 2) skinny_kernel(const __grid_cons
             uint8_t* sx = sw + kSkWBytes;
             mbar_expect_tx(&full_bar[s], bytes);
             tma_load_2d(sw, &p.tma_w, &full_bar[s], k * 64, t.w_row);
-            if (MODE == 2) tma_load_2d(sw + kSkWBytes / 2, &p.tma_w, &full_bar[s], k * 64, t.w_row2);
+            if (skinny_swiglu(MODE)) tma_load_2d(sw + kSkWBytes / 2, &p.tma_w, &full_bar[s], k * 64, t.w_row2);
             for (int b = 0; b < boxes; ++b)
               tma_load_2d(sx + b * kSkXBox, &p.tma_x, &full_bar[s], k * 64, t.x_row + at + 16 * b);
           }
@@ -276,11 +286,11 @@ __global__ void __launch_bounds__(kSkThreads, 2) skinny_kernel(const __grid_cons
           tmem_ld16(taddr + 16 * b, v);
           tc_wait_ld();
           // staged as [token][weight row], so that consecutive threads write consecutive outputs of one token
-          float* st = MODE == 0 ? reinterpret_cast<float*>(smem) + 16 * b * kSkRows : epi;
-          if (MODE != 0 && b > 0) asm volatile("bar.sync 1, 128;" ::: "memory");
+          float* st = skinny_dense(MODE) ? reinterpret_cast<float*>(smem) + 16 * b * kSkRows : epi;
+          if (!skinny_dense(MODE) && b > 0) asm volatile("bar.sync 1, 128;" ::: "memory");
 #pragma unroll
           for (int i = 0; i < 16; ++i) st[i * kSkRows + row] = __uint_as_float(v[i]);
-          if (MODE == 0) continue;
+          if (skinny_dense(MODE)) continue;
           asm volatile("bar.sync 1, 128;" ::: "memory");
           constexpr int kQuads = MODE == 2 ? 16 : 32;          // groups of four outputs per token
 #pragma unroll
@@ -289,10 +299,7 @@ __global__ void __launch_bounds__(kSkThreads, 2) skinny_kernel(const __grid_cons
             float4 o = *reinterpret_cast<const float4*>(st + tok * kSkRows + c);
             if (MODE == 2) {
               const float4 up = *reinterpret_cast<const float4*>(st + tok * kSkRows + 64 + c);
-              o.x = o.x / (1.f + __expf(-o.x)) * up.x;
-              o.y = o.y / (1.f + __expf(-o.y)) * up.y;
-              o.z = o.z / (1.f + __expf(-o.z)) * up.z;
-              o.w = o.w / (1.f + __expf(-o.w)) * up.w;
+              o = make_float4(swiglu1(o.x, up.x), swiglu1(o.y, up.y), swiglu1(o.z, up.z), swiglu1(o.w, up.w));
             }
             if (16 * b + tok < cnt)
               skinny_store4(p.out, 0, (t.x_row + at + 16 * b + tok) * p.ldo + t.col + c, t.col + c, p.N, o);
@@ -307,24 +314,34 @@ __global__ void __launch_bounds__(kSkThreads, 2) skinny_kernel(const __grid_cons
 
   __syncwarp();                                    // the aligned barriers below need whole warps
   tc_fence_before_sync();
-  if (MODE == 0) {
+  if (skinny_dense(MODE)) {
     cluster_sync_all();                            // every slice's sums are in its shared memory
     const bool bad = p.status != nullptr && *reinterpret_cast<volatile uint32_t*>(p.status) != 0u;
     const uint32_t base = smem_u32(smem);
-    const int col0 = first * kSkRows;
-    for (int w = slice * kSkThreads + static_cast<int>(threadIdx.x); !bad && w < p.M * 32; w += slices * kSkThreads) {
-      const int tok = w >> 5, c = (w & 31) * 4;
+    constexpr int kQuads = MODE == 3 ? 16 : 32;              // groups of four outputs per token
+    const int col0 = first * 4 * kQuads;
+    for (int w = slice * kSkThreads + static_cast<int>(threadIdx.x); !bad && w < p.M * kQuads; w += slices * kSkThreads) {
+      const int tok = w / kQuads, c = (w % kQuads) * 4, col = col0 + c;
+      if (col >= p.N) continue;
       const uint32_t at = base + static_cast<uint32_t>(tok * kSkRows + c) * 4u;
-      float4 v[8];
+      float4 v[8], up[8];
 #pragma unroll
       for (int s = 0; s < 8; ++s)
-        if (s < slices) v[s] = ld_cluster_f4(at, static_cast<uint32_t>(s));
-      float4 o = v[0];
+        if (s < slices) {
+          v[s] = ld_cluster_f4(at, static_cast<uint32_t>(s));
+          if (MODE == 3) up[s] = ld_cluster_f4(at + 256u, static_cast<uint32_t>(s));
+        }
+      float4 o = v[0], u = up[0];
 #pragma unroll
       for (int s = 1; s < 8; ++s)
-        if (s < slices) { o.x += v[s].x; o.y += v[s].y; o.z += v[s].z; o.w += v[s].w; }
-      const int col = col0 + c;
-      if (col >= p.N) continue;
+        if (s < slices) {
+          o.x += v[s].x; o.y += v[s].y; o.z += v[s].z; o.w += v[s].w;
+          if (MODE == 3) { u.x += up[s].x; u.y += up[s].y; u.z += up[s].z; u.w += up[s].w; }
+        }
+      if (MODE == 3) {
+        const float f = p.scale != nullptr ? __bfloat162float(p.scale[col / p.seg]) : 1.f;
+        o = make_float4(f * swiglu1(o.x, u.x), f * swiglu1(o.y, u.y), f * swiglu1(o.z, u.z), f * swiglu1(o.w, u.w));
+      }
       if (p.bias != nullptr) {
         o.x += __bfloat162float(p.bias[col]);
         if (col + 1 < p.N) o.y += __bfloat162float(p.bias[col + 1]);

@@ -85,11 +85,12 @@ int launch_rope_tables(void* q, void* k, const float* cos_t, const float* sin_t,
 int launch_rope3d(void* q, void* k, const int* pos_thw, int64_t tokens, int hq, int hk, int head_dim, int d_t,
                   int d_h, int d_w, float theta, int inverse, cudaStream_t stream);
 // SwiGLU: out[r, j] = silu(in[r, j]) * in[r, F + j]   (in is [rows, 2F])
-int launch_swiglu_fwd(const void* in, void* out, int64_t rows, int F, cudaStream_t stream);
+// scale (optional): `period` floats, row r is multiplied by scale[r % period]
+int launch_swiglu_fwd(const void* in, void* out, int64_t rows, int F, const float* scale, int period, cudaStream_t stream);
 int launch_swiglu_bwd(const void* in, const void* dout, void* din, int64_t rows, int F, cudaStream_t stream);
 // expert rows: din = row_w * dSwiGLU(in, dact), actw = row_w * SwiGLU(in), rowdot = <SwiGLU(in), dact> per row
 int launch_swiglu_bwd_rows(const void* in, const void* dact, const float* row_w, void* din, void* actw, float* rowdot,
-                           int64_t rows, int F, cudaStream_t stream);
+                           int64_t rows, int F, int period, cudaStream_t stream);
 // FiLM: y = x * (1 + scale[g]) + shift[g], g = row / rows_per_group
 int launch_film(const void* x, const void* scale, const void* shift, void* y, int64_t rows, int cols,
                 int64_t rows_per_group, cudaStream_t stream);
@@ -132,7 +133,7 @@ int launch_ssm_scan_bwd(const float* u, const float* delta, const float* A, cons
 // Products of few token rows with large weights (skinny.cu): out[t, n] = sum_k x[t, k] * w[n, k].
 struct SkinnyArgs {
   const void* x = nullptr;             // [x_rows, K] bf16, pitch ldx
-  const void* w = nullptr;             // [N, K] bf16, pitch ldw; grouped: [experts, N (swiglu: 2 N), K]
+  const void* w = nullptr;             // [N (swiglu: 2 N), K] bf16, pitch ldw; grouped: [experts, N (swiglu: 2 N), K]
   void* out = nullptr;                 // [x_rows, N], pitch ldo
   const void* bias = nullptr;          // dense: bf16 [N]
   int64_t x_rows = 0, ldx = 0, ldw = 0, ldo = 0;
@@ -141,7 +142,9 @@ struct SkinnyArgs {
   // grouped over experts: the dispatch plan of a 128-row-padded token layout
   int experts = 0, max_tiles = 0;
   int slots = 0;                       // tokens per pass (rounded up to 16, 32, 64 or 128); any count per tile is right
-  int swiglu = 0;
+  int swiglu = 0;                      // gate rows and up rows -> silu(gate) * up
+  int seg = 0;                         // dense with swiglu: w = [seg gate rows, seg up rows] for every segment of N
+  const void* scale = nullptr;         // dense with swiglu: bf16 factor per segment
   const int *tile_expert = nullptr, *num_m_tiles = nullptr, *seg_offsets = nullptr, *counts = nullptr;
   uint32_t* status = nullptr;
 };

@@ -98,7 +98,20 @@ def gemm_skinny(x2: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] 
     if not 1 <= M <= 128 or K == 0 or w.shape[0] == 0 or w.stride(1) != 1 or x2.stride(1) != 1:
         return None
     out = torch.empty(M, w.shape[0], dtype=out_dtype, device=x2.device)
-    _k().gemm_skinny(x2, w, bias, out, _st(x2))
+    _k().gemm_skinny(x2, w, bias, out, 0, None, _st(x2))
+    return out
+
+
+def skinny_swiglu(x2: torch.Tensor, w: torch.Tensor, seg: int, scale: Optional[torch.Tensor] = None) -> Optional[torch.Tensor]:
+    """silu(gate) * up of up to 128 rows in the kernel that streams the weights, without a gradient: ``w`` holds ``seg`` gate
+    rows and their ``seg`` up rows for every segment of the outputs, ``scale`` a factor per segment.  None when the operands
+    are not what it reads."""
+    M, K = x2.shape
+    if not 1 <= M <= 128 or K == 0 or seg <= 0 or seg % 64 != 0 or w.stride(1) != 1 or x2.stride(1) != 1 or \
+            x2.dtype != _BF16 or w.dtype != _BF16:
+        return None
+    out = torch.empty(M, w.shape[0] // 2, dtype=_BF16, device=x2.device)
+    _k().gemm_skinny(x2, w, None, out, seg, scale, _st(x2))
     return out
 
 
@@ -288,6 +301,37 @@ def swiglu(gate_up: torch.Tensor) -> torch.Tensor:
     if gate_up.is_cuda and gate_up.dtype == _BF16:
         return _SwiGLUFn.apply(gate_up)
     return ref.swiglu(gate_up)
+
+
+class _SwiGLUMixFn(torch.autograd.Function):
+    """SwiGLU whose rows are multiplied by weights that repeat with their number: out[r] = mix[r % S] * swiglu(in[r])."""
+
+    @staticmethod
+    def forward(ctx, gate_up, mix):
+        g2 = _as2d(gate_up).contiguous()
+        out = torch.empty(g2.shape[0], g2.shape[1] // 2, dtype=_BF16, device=g2.device)
+        mix = mix.float().contiguous()
+        _k().swiglu_fwd(g2, out, mix)
+        ctx.save_for_backward(g2, mix)
+        ctx.shape = gate_up.shape
+        return out.view(*gate_up.shape[:-1], out.shape[1])
+
+    @staticmethod
+    def backward(ctx, dout):
+        g2, mix = ctx.saved_tensors
+        d2 = _as2d(dout).contiguous()
+        din = torch.empty_like(g2)
+        dots = torch.empty(g2.shape[0], dtype=torch.float32, device=g2.device)
+        _k().swiglu_bwd_rows(g2, d2, mix, din, None, dots)
+        return din.view(ctx.shape), dots.view(-1, mix.numel()).sum(0) if ctx.needs_input_grad[1] else None
+
+
+def swiglu_mix(gate_up: torch.Tensor, mix: torch.Tensor) -> torch.Tensor:
+    """mix[r % S] * silu(x[r, :F]) * x[r, F:] for rows r of ``gate_up`` [.., 2 F] and fp32 weights ``mix`` [S]."""
+    if gate_up.is_cuda and gate_up.dtype == _BF16:
+        return _SwiGLUMixFn.apply(gate_up, mix)
+    act = ref.swiglu(gate_up)
+    return (act.reshape(-1, mix.numel(), act.shape[-1]) * mix.to(act.dtype).view(1, -1, 1)).reshape(act.shape)
 
 
 # --------------------------------------------------------------------------------------------------

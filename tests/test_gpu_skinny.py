@@ -54,3 +54,48 @@ def test_experts_without_gradient_match_fp64(T, E, H, F, same):
             want[t] += float(weights[t, j]) * (w2[e].double() @ (torch.nn.functional.silu(gate) * up))
     # the activation, the experts' outputs and their sum are rounded to bf16
     assert _distance(got, want) < 3 * 2.0 ** -8
+
+
+@pytest.mark.parametrize("M,H,seg,parts", [(1, 64, 64, 1), (17, 520, 64, 3), (128, 256, 192, 2), (130, 256, 64, 2)])
+def test_shared_experts_activation_matches_fp64(M, H, seg, parts):
+    """silu(gate) * up times a weight per expert: inside the product (up to 128 rows) and by itself, with its gradients."""
+    g = torch.Generator("cuda").manual_seed(M)
+    x = torch.randn(M, H, device="cuda", generator=g).bfloat16()
+    w = (torch.randn(parts * 2 * seg, H, device="cuda", generator=g) * H ** -0.5).bfloat16()
+    mix = torch.softmax(torch.randn(parts, device="cuda", generator=g), 0).bfloat16()
+    y = (x.double() @ w.double().t()).view(M, parts, 2, seg)
+    want = torch.nn.functional.silu(y[:, :, 0]) * y[:, :, 1] * mix.double()[:, None]
+    inside = F_.skinny_swiglu(x, w, seg, mix)
+    assert (inside is None) == (M > 128)
+    if inside is not None:
+        assert _distance(inside.view_as(want), want) < 2.0 ** -8
+    y16 = F_.linear(x, w).view(M * parts, 2 * seg).detach().requires_grad_(True)
+    mix32 = mix.float().requires_grad_(True)
+    out = F_.swiglu_mix(y16, mix32)
+    grad = torch.randn(out.shape, device="cuda", generator=g).bfloat16()
+    got = torch.autograd.grad(out, (y16, mix32), grad)
+    y64, mix64 = y16.detach().double().requires_grad_(True), mix32.detach().double().requires_grad_(True)
+    a, b = y64.chunk(2, -1)
+    out64 = torch.nn.functional.silu(a) * b * mix64.repeat(M)[:, None]
+    ref = torch.autograd.grad(out64, (y64, mix64), grad.double())
+    assert _distance(out.detach(), out64.detach()) < 2.0 ** -8 and _distance(got[0], ref[0]) < 2.0 ** -8
+    # __expf and sums of M x seg products in fp32, of which some cancel
+    assert got[1].dtype == torch.float32 and _distance(got[1], ref[1]) < 1e-4
+
+
+@pytest.mark.parametrize("T", [1, 147, 148])
+def test_combine_adds_the_shared_experts(T):
+    g = torch.Generator("cuda").manual_seed(T)
+    E, H, F, k = 8, 1152, 64, 3
+    x = torch.randn(T, H, device="cuda", generator=g).bfloat16()
+    w13 = (torch.randn(E, 2 * F, H, device="cuda", generator=g) * H ** -0.5).bfloat16()
+    w2 = (torch.randn(E, H, F, device="cuda", generator=g) * F ** -0.5).bfloat16()
+    idx = torch.rand(T, E, device="cuda", generator=g).topk(k, -1).indices.int()
+    weights = torch.rand(T, k, device="cuda", generator=g)
+    add = torch.randn(T, H, device="cuda", generator=g).bfloat16().requires_grad_(True)
+    alone = moe_ops.moe_experts(x, w13, w2, weights, idx)
+    both = moe_ops.moe_experts(x, w13, w2, weights, idx, add=add)
+    # both results are rounded
+    assert _distance(both.detach(), alone.double() + add.detach().double()) < 2 * 2.0 ** -8
+    grad = torch.randn(T, H, device="cuda", generator=g).bfloat16()
+    assert torch.equal(torch.autograd.grad(both, add, grad)[0], grad)

@@ -249,11 +249,11 @@ int launch_paged_decode(const PagedDecodeArgs& a, cudaStream_t stream) {
   const int64_t heads_total = static_cast<int64_t>(a.batch) * a.hq;
   const unsigned mgrid = static_cast<unsigned>((heads_total + 3) / 4);
   if (a.d == 128) {
-    paged_decode_merge_kernel<128><<<mgrid, 128, 0, stream>>>(a.partial_o, a.partial_ml, p.o, heads_total, a.splits);
-  } else {
-    paged_decode_merge_kernel<64><<<mgrid, 128, 0, stream>>>(a.partial_o, a.partial_ml, p.o, heads_total, a.splits);
+    return launch_chained(paged_decode_merge_kernel<128>, dim3(mgrid), dim3(128), 0, stream, 0, a.partial_o, a.partial_ml, p.o,
+                          heads_total, a.splits);
   }
-  return static_cast<int>(cudaGetLastError());
+  return launch_chained(paged_decode_merge_kernel<64>, dim3(mgrid), dim3(128), 0, stream, 0, a.partial_o, a.partial_ml, p.o,
+                        heads_total, a.splits);
 }
 
 int launch_kv_cache_write(const void* k, const void* v, void* k_cache, void* v_cache, const int* slot_map,
@@ -261,11 +261,10 @@ int launch_kv_cache_write(const void* k, const void* v, void* k_cache, void* v_c
                           uint32_t* status, cudaStream_t stream) {
   if (tokens <= 0) return 0;
   if ((row_elems & 7) != 0) return -1;
-  kv_cache_write_kernel<<<static_cast<unsigned>(tokens), 128, 0, stream>>>(
-      reinterpret_cast<const __nv_bfloat16*>(k), reinterpret_cast<const __nv_bfloat16*>(v),
-      reinterpret_cast<__nv_bfloat16*>(k_cache), reinterpret_cast<__nv_bfloat16*>(v_cache), slot_map, row_elems,
-      k_stride, v_stride, num_slots, status);
-  return static_cast<int>(cudaGetLastError());
+  return launch_chained(kv_cache_write_kernel, dim3(static_cast<unsigned>(tokens)), dim3(128), 0, stream, 0,
+                        reinterpret_cast<const __nv_bfloat16*>(k), reinterpret_cast<const __nv_bfloat16*>(v),
+                        reinterpret_cast<__nv_bfloat16*>(k_cache), reinterpret_cast<__nv_bfloat16*>(v_cache), slot_map, row_elems,
+                        k_stride, v_stride, num_slots, status);
 }
 
 }  // namespace yv

@@ -9,6 +9,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "chain.cuh"
 #include "sm100.cuh"
 
 namespace yv {
@@ -183,6 +184,8 @@ __global__ void paged_decode_merge_kernel(const float* __restrict__ partial_o, c
   // D / 32 columns a lane; lane s weighs ranges s, s + 32, ...: one read of (m, l) each instead of a chain of them, and eight
   // rows of partials in flight.
   constexpr int V = D / 32;
+  chain_next();
+  chain_wait();
   const int lane = threadIdx.x & 31;
   const int64_t w = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (w >= heads_total) return;
@@ -222,6 +225,8 @@ __global__ void kv_cache_write_kernel(const __nv_bfloat16* __restrict__ k, const
                                       __nv_bfloat16* __restrict__ k_cache, __nv_bfloat16* __restrict__ v_cache,
                                       const int* __restrict__ slot_map, int row_elems, int64_t k_stride,
                                       int64_t v_stride, int64_t num_slots, uint32_t* status) {
+  chain_next();
+  chain_wait();
   const int64_t t = blockIdx.x;
   const int64_t slot = slot_map[t];
   if (slot < 0) return;                       // padding token

@@ -27,6 +27,7 @@
 // otherwise an unnormalised partial (max, sum, out) per query head and split, merged by another kernel.
 #pragma once
 #include "per_device.h"
+#include "chain.cuh"
 #include "sm100.cuh"
 #include "tensormap.h"
 
@@ -119,6 +120,21 @@ __global__ void __launch_bounds__(kDmThreads, NB == 1 && G < 16 ? 2 : 1) paged_d
   const int heads = min(G, p.group - chunk * G);
   const int tid = threadIdx.x, lane = tid & 31;
   const int warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0);                 // known to be uniform
+  if (tid == 0) {
+    tma_prefetch_desc(&p.tma_k);
+    tma_prefetch_desc(&p.tma_v);
+    for (int s = 0; s < kDmStages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&s_bar[i], 1); mbar_init(&pv_bar[i], 1); mbar_init(&p_bar[i], 128); }
+    fence_barrier_init();
+  }
+  if (warp == 0) {
+    tmem_alloc(&tmem_slot, 64);
+    tmem_relinquish();
+  }
+  // the tensor memory is this kernel's before the next one may begin
+  __syncthreads();
+  chain_next();
+  chain_wait();
   int seq_len = p.seq_lens[b];
   if (seq_len < 0 || seq_len > static_cast<int64_t>(p.max_blocks_per_seq) * kDmBlock) {   // reported and cut to the row
     if (tid == 0 && p.status != nullptr) atomicOr(p.status, kStatusIndexOutOfRange);
@@ -137,17 +153,6 @@ __global__ void __launch_bounds__(kDmThreads, NB == 1 && G < 16 ? 2 : 1) paged_d
     for (int i = tid; i < blk1 - blk0; i += kDmThreads) s_table[i] = gtable[blk0 + i];
   const int* table = staged ? (s_table - blk0) : gtable;          // indexed by absolute block number either way
 
-  if (tid == 0) {
-    tma_prefetch_desc(&p.tma_k);
-    tma_prefetch_desc(&p.tma_v);
-    for (int s = 0; s < kDmStages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
-    for (int i = 0; i < 2; ++i) { mbar_init(&s_bar[i], 1); mbar_init(&pv_bar[i], 1); mbar_init(&p_bar[i], 128); }
-    fence_barrier_init();
-  }
-  if (warp == 0) {
-    tmem_alloc(&tmem_slot, 64);
-    tmem_relinquish();
-  }
   // Qpad: heads and columns that do not exist are zero.  P: rows >= G stay zero for the whole kernel.
   for (int i = tid; i < NB * 16 * 8; i += kDmThreads) {
     const int v = i & 7, g = (i >> 3) & 15, c = i >> 7, col = c * 64 + v * 8;
@@ -427,8 +432,7 @@ int paged_decode_mma_run(const PagedDecodeMmaParams& p, dim3 grid, cudaStream_t 
     if (e != cudaSuccess) return static_cast<int>(e);
     configured.cur() = 1;
   }
-  paged_decode_mma_kernel<G, NB><<<grid, kDmThreads, DecodeMmaSmem<NB>::kTotal, stream>>>(p);
-  return static_cast<int>(cudaGetLastError());
+  return launch_chained(paged_decode_mma_kernel<G, NB>, grid, dim3(kDmThreads), DecodeMmaSmem<NB>::kTotal, stream, 0, p);
 }
 
 // (size, kv head, slot) map of cache pages [slots, kv_heads, size]; copies of 64 columns of one block

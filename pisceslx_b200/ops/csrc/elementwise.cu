@@ -6,6 +6,7 @@
 #include <math.h>
 #include <stdint.h>
 
+#include "chain.cuh"
 #include "yv_ops.h"
 
 namespace yv {
@@ -70,6 +71,8 @@ __global__ void rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __
   const int nvec = cols >> 3;
   float v[VPT][8];
   float ss = 0.f;
+  chain_next();
+  chain_wait();
 #pragma unroll
   for (int i = 0; i < VPT; ++i) {
     const int vec = threadIdx.x + i * blockDim.x;
@@ -234,6 +237,8 @@ __global__ void __launch_bounds__(256) rope_vec_kernel(__nv_bfloat16* __restrict
                                                        const int* __restrict__ positions, int64_t tokens, int hq, int hk,
                                                        int head_dim, int chunks, int inverse, int64_t q_stride,
                                                        int64_t k_stride) {
+  chain_next();
+  chain_wait();
   const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
   const int64_t t = i / (chunks * 8);
   if (t >= tokens) return;
@@ -461,17 +466,15 @@ int launch_rmsnorm_fwd(const void* x, const void* residual, const void* w, const
   const int block = norm_block(cols, &vpt);
   const unsigned grid = static_cast<unsigned>(rows);
 #define YV_LAUNCH(V)                                                                                          \
-  rmsnorm_fwd_kernel<V><<<grid, block, 0, stream>>>(YV_BF(x), YV_BF(residual), YV_BF(w), YV_BF(film_scale),   \
-                                                     YV_BF(film_shift), film_rows_per_group, YV_BFM(y),       \
-                                                     YV_BFM(res_out), rstd, cols, eps)
+  return launch_chained(rmsnorm_fwd_kernel<V>, dim3(grid), dim3(block), 0, stream, 0, YV_BF(x), YV_BF(residual), YV_BF(w),      \
+                        YV_BF(film_scale), YV_BF(film_shift), film_rows_per_group, YV_BFM(y), YV_BFM(res_out), rstd, cols, eps)
   switch (vpt) {
-    case 1: YV_LAUNCH(1); break;
-    case 2: YV_LAUNCH(2); break;
-    case 4: YV_LAUNCH(4); break;
-    default: YV_LAUNCH(8); break;
+    case 1: YV_LAUNCH(1);
+    case 2: YV_LAUNCH(2);
+    case 4: YV_LAUNCH(4);
+    default: YV_LAUNCH(8);
   }
 #undef YV_LAUNCH
-  return static_cast<int>(cudaGetLastError());
 }
 
 int launch_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd, const void* dres_in,
@@ -509,9 +512,9 @@ int launch_rope_tables(void* q, void* k, const float* cos_t, const float* sin_t,
                          reinterpret_cast<uintptr_t>(sin_t)) & 15u) == 0;
   if (rot_dim > 0 && rot_dim % 16 == 0 && head_dim % 8 == 0 && q_stride % 8 == 0 && k_stride % 8 == 0 && aligned) {
     const int chunks = rot_dim / 16;
-    rope_vec_kernel<<<static_cast<unsigned>((tokens * chunks * 8 + 255) / 256), 256, 0, stream>>>(
-        YV_BFM(q), YV_BFM(k), cos_t, sin_t, positions, tokens, hq, hk, head_dim, chunks, inverse, q_stride, k_stride);
-    return static_cast<int>(cudaGetLastError());
+    return launch_chained(rope_vec_kernel, dim3(static_cast<unsigned>((tokens * chunks * 8 + 255) / 256)), dim3(256), 0, stream, 0,
+                          YV_BFM(q), YV_BFM(k), cos_t, sin_t, positions, tokens, hq, hk, head_dim, chunks, inverse, q_stride,
+                          k_stride);
   }
   const int total = (hq + hk) * (rot_dim >> 1);
   const int block = total >= 256 ? 256 : ((total + 31) / 32) * 32;

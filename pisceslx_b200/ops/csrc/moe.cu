@@ -7,6 +7,7 @@
 #include <float.h>
 #include <stdint.h>
 
+#include "chain.cuh"
 #include "yv_ops.h"
 
 namespace yv {
@@ -61,6 +62,8 @@ __global__ void gate_topk_kernel(const float* __restrict__ logits, const float* 
                                  int* __restrict__ counts, int64_t tokens, int E, int k, int bias_in_combine,
                                  int renorm_mode) {
   extern __shared__ int hist[];
+  chain_next();
+  chain_wait();
   for (int e = threadIdx.x; e < E; e += blockDim.x) hist[e] = 0;
   __syncthreads();
   const int lane = threadIdx.x & 31;
@@ -199,6 +202,8 @@ __global__ void moe_plan_kernel(const int* __restrict__ counts, int* __restrict_
   __shared__ int s_off[257];
   __shared__ int s_scan[256];
   const int tid = threadIdx.x;
+  chain_next();
+  chain_wait();
   s_scan[tid] = tid < E ? ((counts[tid] + 127) / 128) * 128 : 0;
   __syncthreads();
   for (int d = 1; d < 256; d <<= 1) {
@@ -230,6 +235,8 @@ __global__ void moe_permute_kernel(const __nv_bfloat16* __restrict__ x, const in
                                    __nv_bfloat16* __restrict__ xp, int k, int cols) {
   __shared__ int dest[kMaxTopK];
   const int64_t t = blockIdx.x;
+  chain_next();
+  chain_wait();
   if (threadIdx.x < k) {
     const int e = idx[t * k + threadIdx.x];
     const int r = atomicAdd(&cursor[e], 1);
@@ -280,6 +287,8 @@ __global__ void moe_combine_kernel(const __nv_bfloat16* __restrict__ y, const in
   __shared__ int s_row[kMaxTopK];
   __shared__ float s_w[kMaxTopK];
   const int64_t t = blockIdx.x;
+  chain_next();
+  chain_wait();
   if (threadIdx.x < k) {
     const float w = weights[t * k + threadIdx.x];
     s_w[threadIdx.x] = w;
@@ -497,9 +506,8 @@ int launch_gate_topk(const float* logits, const float* bias, float* weights, int
   const int block = 256;
   int64_t grid = (tokens + 7) / 8;
   if (grid > 148 * 8) grid = 148 * 8;
-  gate_topk_kernel<<<static_cast<unsigned>(grid), block, E * sizeof(int), stream>>>(
-      logits, bias, weights, idx, probs, counts, tokens, E, k, bias_in_combine, renorm_mode);
-  return static_cast<int>(cudaGetLastError());
+  return launch_chained(gate_topk_kernel, dim3(static_cast<unsigned>(grid)), dim3(block), E * sizeof(int), stream, 0, logits, bias,
+                        weights, idx, probs, counts, tokens, E, k, bias_in_combine, renorm_mode);
 }
 
 int launch_gate_topk_bwd(const float* dweights, const float* probs, const int* idx, const float* weights,
@@ -515,8 +523,8 @@ int launch_gate_topk_bwd(const float* dweights, const float* probs, const int* i
 int launch_moe_plan(const int* counts, int* seg_offsets, int* tile_expert, int* num_m_tiles, int* cursor, int E,
                     int max_tiles, cudaStream_t stream) {
   if (E > 256) return -1;
-  moe_plan_kernel<<<1, 256, 0, stream>>>(counts, seg_offsets, tile_expert, num_m_tiles, cursor, E, max_tiles);
-  return static_cast<int>(cudaGetLastError());
+  return launch_chained(moe_plan_kernel, dim3(1), dim3(256), 0, stream, 0, counts, seg_offsets, tile_expert, num_m_tiles, cursor, E,
+                        max_tiles);
 }
 
 int launch_moe_rank(const int* idx, const int* seg_offsets, int* row_map, int64_t n, int E, cudaStream_t stream) {
@@ -539,8 +547,8 @@ int launch_moe_permute(const void* x, const int* idx, int* cursor, int* row_map,
   if ((cols & 7) != 0 || k > kMaxTopK) return -1;
   const int block = (cols >> 3) >= 256 ? 256 : 128;
   if (cursor != nullptr) {
-    moe_permute_kernel<<<static_cast<unsigned>(tokens), block, 0, stream>>>(YV_BF(x), idx, cursor, row_map,
-                                                                            YV_BFM(xp), k, cols);
+    return launch_chained(moe_permute_kernel, dim3(static_cast<unsigned>(tokens)), dim3(block), 0, stream, 0, YV_BF(x), idx, cursor,
+                          row_map, YV_BFM(xp), k, cols);
   } else {
     moe_permute_mapped_kernel<<<static_cast<unsigned>(tokens), block, 0, stream>>>(YV_BF(x), row_map, YV_BFM(xp), k,
                                                                                    cols);
@@ -562,9 +570,8 @@ int launch_moe_combine(const void* y, const int* row_map, const float* weights, 
   // enough blocks for every SM when the tokens alone are too few
   const int block = (cols >> 3) >= 256 && tokens >= 148 ? 256 : 128;
   const unsigned parts = tokens >= 148 ? 1u : static_cast<unsigned>(((cols >> 3) + block - 1) / block);
-  moe_combine_kernel<<<dim3(static_cast<unsigned>(tokens), parts), block, 0, stream>>>(YV_BF(y), row_map, weights, YV_BF(add),
-                                                                                       YV_BFM(out), k, cols);
-  return static_cast<int>(cudaGetLastError());
+  return launch_chained(moe_combine_kernel, dim3(static_cast<unsigned>(tokens), parts), dim3(block), 0, stream, 0, YV_BF(y), row_map,
+                        weights, YV_BF(add), YV_BFM(out), k, cols);
 }
 
 int launch_moe_combine_bwd(const void* dout, const void* y, const int* row_map, const float* weights, void* dy,

@@ -29,19 +29,7 @@ int launch(const SkinnyParams& p, int grid, int cluster, cudaStream_t stream) {
     if (e != cudaSuccess) return static_cast<int>(e);
     configured.cur() = 1;
   }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(grid));
-  cfg.blockDim = dim3(kSkThreads);
-  cfg.dynamicSmemBytes = SkinnySmem<NT>::kTotal;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = static_cast<unsigned>(cluster);
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return static_cast<int>(cudaLaunchKernelEx(&cfg, kern, p));
+  return launch_chained(kern, dim3(static_cast<unsigned>(grid)), dim3(kSkThreads), SkinnySmem<NT>::kTotal, stream, cluster, p);
 }
 
 template <int MODE>

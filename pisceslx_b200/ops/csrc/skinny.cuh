@@ -17,6 +17,7 @@
 // 32000 x 4096 44.7 us (5.9 TB/s; before 57), 6144 x 4096 16.4, 4096 x 4096 10.8, 4096 x 5632 12.5, 64 x 4096 5.5 (before 18);
 // 64 experts of 4096 x 1408 with 64 tokens, top-6, both products and the activation 350 us (6.3 TB/s; before 435).
 #pragma once
+#include "chain.cuh"
 #include "sm100.cuh"
 
 namespace yv {
@@ -44,6 +45,7 @@ constexpr int kSkThreads = 192;              // TMA producer, MMA issuer, four e
 constexpr int kSkRows = 128;                 // weight rows per tile
 constexpr int kSkWBytes = kSkRows * 128;     // one stage of weights: 128 rows x 64 bf16
 constexpr int kSkXBox = 16 * 128;            // 16 tokens x 64 bf16
+constexpr int kSkAhead = 16;                  // 64-wide steps of K that a dense CTA fetches ahead of the kernel before it
 constexpr int kSkEpiBytes = 16 * kSkRows * 4;
 
 // NT: token slots (16, 32, 64 or 128).  A tile with more live tokens than slots is worked off in passes.
@@ -162,11 +164,12 @@ __global__ void __launch_bounds__(kSkThreads, 2) skinny_kernel(const __grid_cons
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // the swizzled tiles need shared memory that starts on 1024 bytes
   if ((smem_u32(smem) & 1023u) != 0u) {
+    chain_wait();
     if (threadIdx.x == 0 && p.status != nullptr) atomicOr(p.status, kStatusBadArgument);
     return;
   }
   const int kc = (p.K + 63) / 64;
-  int slices = 1, slice = 0, units, first, step;
+  int slices = 1, slice = 0, units = 0, first, step;
   if (skinny_dense(MODE)) {
     uint32_t n;
     asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(n));
@@ -176,7 +179,6 @@ __global__ void __launch_bounds__(kSkThreads, 2) skinny_kernel(const __grid_cons
     units = p.tiles_w;
     step = units;                                  // one tile per cluster
   } else {
-    units = *p.num_m_tiles * p.tiles_w;
     first = blockIdx.x;
     step = gridDim.x;
   }
@@ -203,7 +205,21 @@ __global__ void __launch_bounds__(kSkThreads, 2) skinny_kernel(const __grid_cons
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  chain_next();
+  if (skinny_dense(MODE) && warp == 0 && elect_one()) {
+    // the weights do not depend on the kernel before this one: start them on their way to the L2 (not into shared memory, where
+    // weights that the kernel before wrote would be stale)
+    SkinnyTile t;
+    if (skinny_tile<MODE>(p, first, units, t))
+      for (int k = k0; k < k1 && k < k0 + kSkAhead; ++k) {
+        tma_prefetch_l2_2d(&p.tma_w, k * 64, t.w_row);
+        if (skinny_swiglu(MODE)) tma_prefetch_l2_2d(&p.tma_w, k * 64, t.w_row2);
+      }
+  }
+  chain_wait();
+  if (!skinny_dense(MODE)) units = *p.num_m_tiles * p.tiles_w;
 
+  __syncwarp();
   if (warp == 0) {
     if (elect_one()) {
       uint32_t it = 0;

@@ -61,6 +61,35 @@ void gemm_grouped_k(const Tensor& a, const Tensor& b, Tensor c, const Tensor& se
   g.status = statusp(status);
   check_rc(yv::launch_gemm(g, cur_stream()), "gemm_grouped_k");
 }
+// out[M,N] = a[M,K] @ b[K,N] with the K range cut into seg_offsets.numel()-1 slices (offsets are multiples of 64 but for the last),
+// each summed by its own CTAs into the fp32 workspace ws [slices, ceil128(M), N] and then in the order of the slices.
+void gemm_split(const Tensor& a, const Tensor& b, Tensor ws, const Tensor& seg_offsets, Tensor out,
+                const c10::optional<Tensor>& status) {
+  check_bf16(a, "a"); check_bf16(b, "b"); check_f32(ws, "ws"); check_i32(seg_offsets, "seg_offsets"); check_bf16(out, "out");
+  TORCH_CHECK(a.dim() == 2 && b.dim() == 2 && a.stride(1) == 1 && b.stride(1) == 1 && ws.is_contiguous(),
+              "gemm_split: a [M,K], b [K,N] with unit inner stride, contiguous ws");
+  const int slices = static_cast<int>(seg_offsets.numel()) - 1;
+  const int M = static_cast<int>(a.size(0)), K = static_cast<int>(a.size(1)), N = static_cast<int>(b.size(1));
+  const int m_pad = (M + 127) / 128 * 128;
+  TORCH_CHECK(slices >= 1 && b.size(0) == K && N % 4 == 0, "gemm_split: shape mismatch");
+  TORCH_CHECK(out.is_contiguous() && out.dim() == 2 && out.size(0) == M && out.size(1) == N, "gemm_split: out [M,N] contiguous");
+  TORCH_CHECK(ws.numel() >= static_cast<int64_t>(slices) * m_pad * N, "gemm_split: workspace too small");
+  const c10::cuda::CUDAGuard guard(a.device());
+  yv::GemmArgs g;
+  g.a = a.data_ptr(); g.b = b.data_ptr(); g.c = ws.data_ptr();
+  g.b_mn = true;
+  g.M = M; g.N = N; g.K = K;
+  g.lda = a.stride(0); g.ldb = b.stride(0); g.ldc = N;
+  g.out_fp32 = 1;
+  g.mode = 4;
+  g.num_groups = slices;
+  g.seg_offsets = seg_offsets.data_ptr<int>();
+  g.bn = N > 128 ? 256 : 128;
+  g.status = statusp(status);
+  check_rc(yv::launch_gemm(g, cur_stream()), "gemm_split");
+  check_rc(yv::launch_sum_slices(ws.data_ptr<float>(), out.data_ptr(), slices, M, m_pad, N, cur_stream()), "sum_slices");
+}
+
 // Grouped along M with few tokens per expert, of which live rows alone are read and written: x [rows, K] in the layout of
 // the dispatch plan, w [E, N, K] (swiglu: [E, 2 N, K], gate rows then up rows, N a multiple of 64), out [rows, N].
 // `slots` is the number of tokens per expert to prepare for; experts with more take several passes.

@@ -118,15 +118,14 @@ int launch_gemm(const GemmArgs& a, cudaStream_t stream) {
     p.c_group_stride = a.M;
     c_outer = groups * static_cast<uint64_t>(a.M);
   } else if (a.mode == 4) {
-    // split-K of a dense product with both operands stored K-inner (activations [M,K], weights [N,K]): slice g
-    // reduces over K range seg_offsets[g] .. seg_offsets[g+1] and writes its partial to rows g*Mpad.. of C, where
-    // Mpad = M rounded up to 128.  Runs the grouped-K tile loop; used for skinny M (decode), where the N tiles alone
-    // would occupy a fraction of the SMs.
-    if (a.a_mn || a.b_mn || a.seg_offsets == nullptr || a.accumulate) return -60;
+    // split-K of a dense product with A stored K-inner: slice g reduces over K range seg_offsets[g] .. seg_offsets[g+1]
+    // (multiples of 64 but for the end) and writes its partial to rows g*Mpad.. of C, where Mpad = M rounded up to 128.
+    // Runs the grouped-K tile loop; used where the output tiles alone would occupy a fraction of the SMs.
+    if (a.a_mn || a.seg_offsets == nullptr || a.accumulate) return -60;
     const int m_pad = ((a.M + kBM - 1) / kBM) * kBM;
     p.mode = kGroupedK;
     a_inner = a.K;  a_outer = a.M;
-    b_inner = a.K;  b_outer = a.N;
+    b_inner = a.b_mn ? a.N : a.K;  b_outer = a.b_mn ? a.K : a.N;
     p.c_group_stride = m_pad;
     c_outer = groups * static_cast<uint64_t>(m_pad);
   } else if (a.mode == kBatched) {
@@ -250,5 +249,32 @@ int launch_gemm(const GemmArgs& a, cudaStream_t stream) {
   return a.out_fp32 ? dispatch_layout<128, float>(a, p, grid, stream)
                     : dispatch_layout<128, __nv_bfloat16>(a, p, grid, stream);
 }
+
+#ifndef YV_SERVING_PRODUCTS
+namespace {
+// out[m, n] = sum_s parts[s][m, n] in the order of s; four columns per thread, the slices' loads in flight together
+__global__ void __launch_bounds__(256) sum_slices_kernel(const float* __restrict__ parts, __nv_bfloat16* __restrict__ out, int slices,
+                                                         int64_t quads, int64_t stride) {
+  const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+  if (i >= quads) return;
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+  for (int s = 0; s < slices; ++s) {
+    const float4 v = *reinterpret_cast<const float4*>(parts + s * stride + i * 4);
+    acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+  }
+  *reinterpret_cast<uint2*>(out + i * 4) = make_uint2(pack_bf16(acc.x, acc.y), pack_bf16(acc.z, acc.w));
+}
+}  // namespace
+
+int launch_sum_slices(const float* parts, void* out, int slices, int M, int m_pad, int N, cudaStream_t stream) {
+  if (M <= 0 || N <= 0) return 0;
+  if ((N & 3) != 0 || slices <= 0 || m_pad < M || (reinterpret_cast<uintptr_t>(out) & 7u) != 0) return -1;
+  const int64_t quads = static_cast<int64_t>(M) * N / 4;
+  sum_slices_kernel<<<static_cast<unsigned>((quads + 255) / 256), 256, 0, stream>>>(
+      parts, reinterpret_cast<__nv_bfloat16*>(out), slices, quads, static_cast<int64_t>(m_pad) * N);
+  return static_cast<int>(cudaGetLastError());
+}
+#endif
 
 }  // namespace yv

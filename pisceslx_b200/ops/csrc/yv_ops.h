@@ -130,6 +130,9 @@ int launch_ssm_scan_fwd(const float* u, const float* delta, const float* A, cons
 int launch_ssm_scan_bwd(const float* u, const float* delta, const float* A, const float* Bm, const float* Cm,
                         const float* Dp, const float* hs, const float* dy, float* du, float* ddelta, float* dA,
                         float* dB, float* dC, float* dD, int batch, int L, int D, int N, cudaStream_t stream);
+// out[M,N] (bf16) = sum over slices of parts[slice][m_pad, N] (fp32): second half of a product split along K
+int launch_sum_slices(const float* parts, void* out, int slices, int M, int m_pad, int N, cudaStream_t stream);
+
 // Products of few token rows with large weights (skinny.cu): out[t, n] = sum_k x[t, k] * w[n, k].
 struct SkinnyArgs {
   const void* x = nullptr;             // [x_rows, K] bf16, pitch ldx

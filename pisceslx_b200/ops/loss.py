@@ -13,6 +13,36 @@ from . import kernels, reference as ref, status_word
 _BF16 = torch.bfloat16
 
 
+def _slices(M: int, N: int, K: int) -> int:
+    """Slices of K for the gradient of the hidden states, [M, V] x [V, N]: a long sum over few output tiles.
+
+    Counted in steps of 64 by all SMs (0.45 us each for a 128 x 256 tile) and in bytes of the fp32 parts, which are written and
+    read (5 TB/s); one slice unless that saves a fifth.  At 154856 x 1024: 2048 rows 670 us in one slice, 517 in nine; 283 rows
+    679 and 108 (twelve)."""
+    tiles, steps = -(-M // 128) * -(-N // 256), -(-K // 64)
+    if tiles > 148 or steps < 64 or N % 4:
+        return 1
+
+    def cost(s: int) -> float:
+        return 0.45 * -(-tiles * s // 148) * -(-steps // s) + (M * N * 8e-6 * s / 5 + 5 if s > 1 else 0)
+
+    best = min(range(1, 17), key=cost)
+    return best if cost(best) < 0.8 * cost(1) else 1
+
+
+def _times_weights(dl: torch.Tensor, w: torch.Tensor, out: torch.Tensor, st: torch.Tensor) -> None:
+    """out [n, H] = dl [n, V] @ w [V, H]."""
+    (M, K), N = dl.shape, w.shape[1]
+    s = _slices(M, N, K)
+    if s == 1:
+        kernels().gemm(dl, w, out, False, True, False, 0, st)
+        return
+    per = -(-(-(-K // 64)) // s) * 64
+    cuts = torch.arange(0, (s + 1) * per, per, dtype=torch.int32, device=dl.device).clamp_(max=K)
+    parts = torch.empty(s, -(-M // 128) * 128, N, dtype=torch.float32, device=dl.device)
+    kernels().gemm_split(dl, w, parts, cuts, out, st)
+
+
 class _LinearCEFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, h, w, labels, ignore_index, scale, chunk):
@@ -44,7 +74,7 @@ class _LinearCEFn(torch.autograd.Function):
             dl = dlogits[:n] if dlogits is not None else None
             K.ce_fwd_bwd(lg, labels[r0:r1], loss_rows[r0:r1], dl, ignore_index, scale)
             if need_dh:
-                K.gemm(dl, w, dh[r0:r1], False, True, False, 0, st)                 # [n,V] x [V,H]
+                _times_weights(dl, w, dh[r0:r1], st)
             if need_dw:
                 if dw32 is not None:
                     K.gemm(dl, h[r0:r1], dw32, True, True, True, 0, st)             # [V,n] x [n,H], accumulate

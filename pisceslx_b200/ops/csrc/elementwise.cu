@@ -234,7 +234,7 @@ __global__ void rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const _
 }
 
 // Sum of the rows: 32 columns a block, sixteen rows at a time.  One thread per column walked 592 rows behind one another on
-// cols / 256 blocks: 17 to 25 us a norm.
+// cols / 256 blocks: 592 rows of 4096 columns 25 us, now 8; of 1024 columns 17, now 5.
 constexpr int kColsumRows = 16;
 __global__ void __launch_bounds__(32 * kColsumRows) colsum_kernel(const float* __restrict__ partial, int blocks, int cols, void* out,
                                                                   int out_fp32, int accumulate) {

@@ -24,7 +24,7 @@ CUDA_SOURCES = ["gemm.cu", "skinny.cu", "elementwise.cu", "moe.cu", "loss_optim.
 CPP_SOURCES = ["binding.cpp"]
 # Layered models can be served by a library of their own: the products and the stream, and the operators of their mixers.
 FAMILIES = {"latent_attention": ["latent.cu"], "grouped_attention": ["grouped.cu"]}
-LAYERED_CUDA_SOURCES = ["gemm.cu", "skinny.cu", "skinny.cu", "stream.cu"]
+LAYERED_CUDA_SOURCES = ["gemm.cu", "skinny.cu", "stream.cu"]
 LAYERED_CPP_SOURCES = ["binding_layered.cpp"]
 LAYERED_DEFINES = {"gemm.cu": ["-DYV_SERVING_PRODUCTS"]}
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",

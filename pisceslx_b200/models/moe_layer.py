@@ -82,29 +82,18 @@ class YvDeepSeekMoELayer(nn.Module):
     def _shared(self, x: torch.Tensor) -> torch.Tensor:
         S, Fs = self.num_shared, self.shared_ffn
         sw = self.shared_expert_weight
-        if torch.is_grad_enabled():
-            mix = torch.softmax(sw.float(), 0)
-        else:
-            # serving: the mixing weights change only when the parameter does; keep them instead of running a softmax and
-            # two casts per layer per decode step
-            key = (sw.data_ptr(), sw._version, x.dtype)
-            cached = getattr(self, "_mix_cache", None)
-            if cached is None or cached[0] != key:
-                mix = torch.softmax(sw.detach().float(), 0)
-                cached = (key, mix, mix.to(x.dtype))
-                self._mix_cache = cached
-            mix = cached[1]
         act = None
         if self.tp_size > 1:
             from ..parallel import tp
             y1 = tp.allgather_linear(x, self.shared_w13, self.tp_group)
         else:
             if x.is_cuda and not torch.is_grad_enabled():
-                act = F_.skinny_swiglu(x, self.shared_w13, Fs, cached[2])
+                # the kernel takes the softmax of the mixing weights itself: nothing derived from the parameter is kept
+                act = F_.skinny_swiglu(x, self.shared_w13, Fs, sw if sw.dtype == torch.bfloat16 else sw.float(), True)
             y1 = F_.linear(x, self.shared_w13) if act is None else None
         if act is None:
             T = y1.shape[0]
-            act = F_.swiglu_mix(y1.view(T * S, 2 * Fs), mix)
+            act = F_.swiglu_mix(y1.view(T * S, 2 * Fs), torch.softmax(sw.float(), 0))
         act = act.reshape(-1, S * Fs)
         if self.tp_size > 1:
             from ..parallel import tp

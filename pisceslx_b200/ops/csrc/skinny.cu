@@ -63,7 +63,9 @@ int launch_skinny(const SkinnyArgs& a, cudaStream_t stream) {
     if (a.swiglu && (a.seg <= 0 || a.seg % 64 != 0 || a.N % a.seg != 0 || a.bias != nullptr)) return -4;
     p.M = a.M;
     p.seg = a.seg;
-    p.scale = static_cast<const __nv_bfloat16*>(a.scale);
+    p.scale = a.scale;
+    p.scale_fp32 = a.scale_fp32;
+    p.scale_softmax = a.scale_softmax;
     // as many slices of K as keep all CTAs resident (two per SM) and leave four 64-wide steps to each
     const int kc = (a.K + 63) / 64, room = 2 * sm_count() / p.tiles_w;
     int slices = 1;

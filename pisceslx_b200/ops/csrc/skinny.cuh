@@ -30,7 +30,9 @@ struct SkinnyParams {
   int tiles_w;                  // tiles of weight rows (of one expert)
   int w_rows;                   // grouped: weight rows per expert
   int seg;                      // dense SWIGLU: outputs per segment (its gate rows are followed by its up rows)
-  const __nv_bfloat16* scale;   // dense SWIGLU, optional: one factor per segment
+  const void* scale;            // dense SWIGLU, optional: one factor per segment (bf16, or fp32 with scale_fp32)
+  int scale_fp32;
+  int scale_softmax;            // the factors are the softmax of `scale` over the segments
   void* out;
   long long ldo;                // elements between output rows
   const __nv_bfloat16* bias;    // dense, optional
@@ -68,6 +70,23 @@ struct SkinnyTile {
 // MODE: 0 dense, 1 grouped, 2 grouped with SWIGLU, 3 dense with SWIGLU
 __host__ __device__ constexpr bool skinny_dense(int mode) { return mode == 0 || mode == 3; }
 __host__ __device__ constexpr bool skinny_swiglu(int mode) { return mode >= 2; }
+
+// Factor of a segment of the outputs.  The softmax of the few values is taken here, from the parameter itself, so that nothing
+// derived from it has to be kept between launches.
+__device__ __forceinline__ float skinny_factor(const SkinnyParams& p, int segment) {
+  if (p.scale == nullptr) return 1.f;
+  auto at = [&](int i) {
+    return p.scale_fp32 ? static_cast<const float*>(p.scale)[i]
+                        : __bfloat162float(static_cast<const __nv_bfloat16*>(p.scale)[i]);
+  };
+  const float mine = at(segment);
+  if (!p.scale_softmax) return mine;
+  const int n = p.N / p.seg;
+  float top = mine, sum = 0.f;
+  for (int i = 0; i < n; ++i) top = fmaxf(top, at(i));
+  for (int i = 0; i < n; ++i) sum += expf(at(i) - top);
+  return expf(mine - top) / sum;
+}
 
 __device__ __forceinline__ float swiglu1(float gate, float up) { return gate / (1.f + __expf(-gate)) * up; }
 
@@ -336,6 +355,7 @@ __global__ void __launch_bounds__(kSkThreads, 2) skinny_kernel(const __grid_cons
     const uint32_t base = smem_u32(smem);
     constexpr int kQuads = MODE == 3 ? 16 : 32;              // groups of four outputs per token
     const int col0 = first * 4 * kQuads;
+    const float f = MODE == 3 ? skinny_factor(p, col0 / p.seg) : 1.f;      // a tile lies in one segment
     for (int w = slice * kSkThreads + static_cast<int>(threadIdx.x); !bad && w < p.M * kQuads; w += slices * kSkThreads) {
       const int tok = w / kQuads, c = (w % kQuads) * 4, col = col0 + c;
       if (col >= p.N) continue;
@@ -355,7 +375,6 @@ __global__ void __launch_bounds__(kSkThreads, 2) skinny_kernel(const __grid_cons
           if (MODE == 3) { u.x += up[s].x; u.y += up[s].y; u.z += up[s].z; u.w += up[s].w; }
         }
       if (MODE == 3) {
-        const float f = p.scale != nullptr ? __bfloat162float(p.scale[col / p.seg]) : 1.f;
         o = make_float4(f * swiglu1(o.x, u.x), f * swiglu1(o.y, u.y), f * swiglu1(o.z, u.z), f * swiglu1(o.w, u.w));
       }
       if (p.bias != nullptr) {

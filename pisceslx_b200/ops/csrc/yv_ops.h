@@ -147,7 +147,8 @@ struct SkinnyArgs {
   int slots = 0;                       // tokens per pass (rounded up to 16, 32, 64 or 128); any count per tile is right
   int swiglu = 0;                      // gate rows and up rows -> silu(gate) * up
   int seg = 0;                         // dense with swiglu: w = [seg gate rows, seg up rows] for every segment of N
-  const void* scale = nullptr;         // dense with swiglu: bf16 factor per segment
+  const void* scale = nullptr;         // dense with swiglu: factor per segment (bf16 or fp32), or its softmax's argument
+  int scale_fp32 = 0, scale_softmax = 0;
   const int *tile_expert = nullptr, *num_m_tiles = nullptr, *seg_offsets = nullptr, *counts = nullptr;
   uint32_t* status = nullptr;
 };

@@ -98,20 +98,21 @@ def gemm_skinny(x2: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] 
     if not 1 <= M <= 128 or K == 0 or w.shape[0] == 0 or w.stride(1) != 1 or x2.stride(1) != 1:
         return None
     out = torch.empty(M, w.shape[0], dtype=out_dtype, device=x2.device)
-    _k().gemm_skinny(x2, w, bias, out, 0, None, _st(x2))
+    _k().gemm_skinny(x2, w, bias, out, 0, None, False, _st(x2))
     return out
 
 
-def skinny_swiglu(x2: torch.Tensor, w: torch.Tensor, seg: int, scale: Optional[torch.Tensor] = None) -> Optional[torch.Tensor]:
+def skinny_swiglu(x2: torch.Tensor, w: torch.Tensor, seg: int, scale: Optional[torch.Tensor] = None,
+                  softmax: bool = False) -> Optional[torch.Tensor]:
     """silu(gate) * up of up to 128 rows in the kernel that streams the weights, without a gradient: ``w`` holds ``seg`` gate
-    rows and their ``seg`` up rows for every segment of the outputs, ``scale`` a factor per segment.  None when the operands
-    are not what it reads."""
+    rows and their ``seg`` up rows for every segment of the outputs, ``scale`` (bf16 or fp32) a factor per segment; with
+    ``softmax`` the factors are its softmax.  None when the operands are not what it reads."""
     M, K = x2.shape
     if not 1 <= M <= 128 or K == 0 or seg <= 0 or seg % 64 != 0 or w.stride(1) != 1 or x2.stride(1) != 1 or \
             x2.dtype != _BF16 or w.dtype != _BF16:
         return None
     out = torch.empty(M, w.shape[0] // 2, dtype=_BF16, device=x2.device)
-    _k().gemm_skinny(x2, w, None, out, seg, scale, _st(x2))
+    _k().gemm_skinny(x2, w, None, out, seg, scale, softmax, _st(x2))
     return out
 
 

@@ -83,11 +83,13 @@ class YvDeepSeekMoELayer(nn.Module):
         S, Fs = self.num_shared, self.shared_ffn
         sw = self.shared_expert_weight
         act = None
+        # serving, not a pass that recomputation repeats with a gradient: that one runs the same kernels as its repetition
+        serving = not (torch.is_grad_enabled() or self.training)
         if self.tp_size > 1:
             from ..parallel import tp
             y1 = tp.allgather_linear(x, self.shared_w13, self.tp_group)
         else:
-            if x.is_cuda and not torch.is_grad_enabled():
+            if x.is_cuda and serving:
                 # the kernel takes the softmax of the mixing weights itself: nothing derived from the parameter is kept
                 act = F_.skinny_swiglu(x, self.shared_w13, Fs, sw if sw.dtype == torch.bfloat16 else sw.float(), True)
             y1 = F_.linear(x, self.shared_w13) if act is None else None
@@ -116,7 +118,8 @@ class YvDeepSeekMoELayer(nn.Module):
                 out = out + sh
         else:
             out = moe_ops.moe_experts(x, self.experts_w13, self.experts_w2, weights, idx, counts,
-                                      self.deterministic, fp8=getattr(self.cfg, "expert_fp8", None), add=sh)
+                                      self.deterministic, fp8=getattr(self.cfg, "expert_fp8", None), add=sh,
+                                      few=not self.training)
         if sh is not None and self.skip_prev:
             if self._prev_shared is not None and self._prev_shared.shape == sh.shape:
                 out = out + 0.1 * self._prev_shared

@@ -145,7 +145,7 @@ class _MoEExpertsFn(torch.autograd.Function):
         is zero (dropped by the capacity rule)."""
 
     @staticmethod
-    def forward(ctx, x, w13, w2, weights, idx, counts, deterministic, training=True, fp8=None, add=None):
+    def forward(ctx, x, w13, w2, weights, idx, counts, deterministic, training=True, fp8=None, add=None, few=True):
         K = _k()
         st = status_word(x.device)
         T, H = x.shape
@@ -156,7 +156,7 @@ class _MoEExpertsFn(torch.autograd.Function):
         mx = fp8 == "mx" and H % 128 == 0 and twoF % 128 == 0 and F % 128 == 0
         xp, plan = permute_tokens(x, idx, counts, E, deterministic, zero_pad=training or mx)
         wts = weights.float().contiguous()
-        if not training and not mx and _few_tokens(T * idx.shape[1], w13, w2):
+        if few and not training and not mx and _few_tokens(T * idx.shape[1], w13, w2):
             y2 = _experts_few(xp, plan, w13, w2, st)
             out = torch.empty(T, H, dtype=_BF16, device=x.device)
             K.moe_combine(y2, plan.row_map, wts, add, out)
@@ -231,7 +231,7 @@ class _MoEExpertsFn(torch.autograd.Function):
         del xp, dy1
         dx = torch.empty(T, H, dtype=_BF16, device=dev)
         K.moe_unpermute_sum(dxp, row_map, dx, k)
-        return dx, dw13, dw2, dwts.to(ctx.w_dtype), None, None, None, None, None, (dout if ctx.has_add else None)
+        return dx, dw13, dw2, dwts.to(ctx.w_dtype), None, None, None, None, None, (dout if ctx.has_add else None), None
 
 
 _MX_WEIGHTS: dict = {}
@@ -252,13 +252,14 @@ def _mx_weight(w: torch.Tensor):
 
 def moe_experts(x: torch.Tensor, w13: torch.Tensor, w2: torch.Tensor, weights: torch.Tensor, idx: torch.Tensor,
                 counts: Optional[torch.Tensor] = None, deterministic: bool = False,
-                fp8: Optional[str] = None, add: Optional[torch.Tensor] = None) -> torch.Tensor:
+                fp8: Optional[str] = None, add: Optional[torch.Tensor] = None, few: bool = True) -> torch.Tensor:
     """Routed experts: out[t] = sum_j weights[t,j] * SwiGLU_FFN_{idx[t,j]}(x[t]).
 
     x [T,H]; w13 [E, 2F, H] (gate rows then up rows); w2 [E, H, F]; weights/idx [T,k]; counts [E] int32
     (the histogram the gate kernel produced; recomputed when omitted).  ``fp8="mx"`` runs the two forward products
     with e4m3 operands and one power-of-two scale per 32 elements (CUDA; H, F multiples of 128).  ``add`` [T,H], the shared
-    experts' output, is added before the result is rounded."""
+    experts' output, is added before the result is rounded.  ``few`` lets a pass without a gradient take the kernel for few
+    tokens, which rounds in other places; off, it equals a pass with a gradient bit for bit."""
     if not x.is_cuda:
         out = ref.moe_experts(x, w13, w2, weights, idx)
         return out if add is None else out + add
@@ -267,7 +268,7 @@ def moe_experts(x: torch.Tensor, w13: torch.Tensor, w2: torch.Tensor, weights: t
         counts = torch.bincount(idx.flatten().long(), minlength=E).int()
     # without autograd (inference) nothing reads what the pad rows of the expert segments produce: skip zeroing them
     return _MoEExpertsFn.apply(x.to(_BF16), w13, w2, weights, idx.int(), counts.int(), deterministic,
-                               torch.is_grad_enabled(), fp8, None if add is None else add.to(_BF16))
+                               torch.is_grad_enabled(), fp8, None if add is None else add.to(_BF16), few)
 
 
 def capacity_mask(weights: torch.Tensor, idx: torch.Tensor, probs: torch.Tensor, counts: torch.Tensor,

@@ -62,3 +62,31 @@ def test_softmax_inside_the_product(parts):
     # the factors differ by a few roundings in fp32, which move a bf16 result to its neighbour at most
     assert (inside.float() - factors.float()).abs().max() <= 2.0 ** -7 * factors.float().abs().max()
     assert (inside.double() - factors.double()).norm() < 2.0 ** -12 * factors.double().norm()
+
+
+@pytest.mark.parametrize("rows", [1, 64, 128, 512, 768, 1000])
+def test_first_pass_of_a_recomputed_layer_equals_its_repetition(rows):
+    """Recomputation runs the layer without a gradient first and with one later: the same function, bit for bit."""
+    layer = _layer(2).train()
+    layer.router.recomputing = True                 # leaves the routing statistics alone
+    x = torch.randn(rows, layer.cfg.hidden_size, device=DEV).bfloat16()
+    with torch.no_grad():
+        first = layer(x)[0]
+    again = layer(x)[0]
+    assert again.requires_grad and torch.equal(first, again.detach())
+
+
+@pytest.mark.parametrize("tokens", [40, 300])
+def test_loss_and_gradients_do_not_depend_on_recomputation(tokens):
+    from pisceslx_b200.models import build_model
+    seen = []
+    for recompute in (True, False):
+        cfg = YvConfig.tiny_text_moe(vocab_size=512)
+        cfg.n_layer, cfg.use_gradient_checkpointing = 2, recompute
+        cfg.extra["moe_deterministic"] = True
+        model = build_model(cfg, DEV, torch.bfloat16, seed=3).train()
+        ids = torch.randint(0, 512, (2, tokens), device=DEV, generator=torch.Generator(DEV).manual_seed(1))
+        loss = model(input_ids=ids, labels=ids, num_valid=2 * (tokens - 1))["loss"]
+        loss.backward()
+        seen.append([loss.detach()] + [layer.mlp.experts_w13.grad for layer in model.model.layers])
+    assert all(torch.equal(a, b) for a, b in zip(*seen))

@@ -164,7 +164,6 @@ def grow_hidden(model: nn.Module, new_hidden: int, init_noise_scale: float = 0.0
             ng = nn.Linear(new_hidden, g.out_features, bias=False).to(g.weight.device, g.weight.dtype)
             ng.weight.copy_(_pad_last(g.weight, new_hidden, 0.0))
             mlp.router.gate = ng
-            mlp.router.__dict__.pop("_gate_bf16", None)
         else:
             mlp.w13 = P(_pad_last(mlp.w13, new_hidden, s))
             mlp.w2 = P(_pad_dim(mlp.w2, 0, new_hidden))

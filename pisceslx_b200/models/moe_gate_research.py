@@ -311,7 +311,7 @@ class YvResearchMoEGate(YvStableMoEGate):
                 w, idx, counts = self._path_cache
                 self.last_counts = counts
                 return w, idx, x2.new_zeros((), dtype=torch.float32)
-        logits = F_.linear(x2, self._gate_weight(), out_fp32=True)
+        logits = F_.linear(x2, self.gate.weight, out_fp32=True)
         extra, soft = self._auxiliary_logits(x2)
         logits = logits + extra
         if modal_id is not None:

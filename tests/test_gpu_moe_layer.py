@@ -90,3 +90,19 @@ def test_loss_and_gradients_do_not_depend_on_recomputation(tokens):
         loss.backward()
         seen.append([loss.detach()] + [layer.mlp.experts_w13.grad for layer in model.model.layers])
     assert all(torch.equal(a, b) for a, b in zip(*seen))
+
+
+def test_gate_in_fp32_is_read_as_it_is():
+    layer = _layer(1)
+    layer.router.gate.float()
+    x = torch.randn(9, layer.cfg.hidden_size, device=DEV).bfloat16()
+    with torch.no_grad():
+        layer.router(x)
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            captured = layer.router(x)[0]
+        layer.router.gate.weight.data.neg_()
+        got, fresh = layer.router(x)[0], copy.deepcopy(layer.router)(x)[0]
+        graph.replay()
+    assert torch.equal(got, fresh) and torch.equal(captured, fresh)

@@ -56,6 +56,7 @@ class YvFusedAdamW(torch.optim.Optimizer):
                 else:
                     ref.adamw_step(p.data, p.grad.to(p.dtype) * self.grad_scale, st["exp_avg"], st["exp_avg_sq"],
                                    group["lr"], b1, b2, group["eps"], group["weight_decay"], st["step"])
+                torch.autograd.graph.increment_version(p)          # written through .data: copies made of it are out of date
         return loss
 
 

@@ -135,6 +135,7 @@ class YvInkOptimizer(torch.optim.Optimizer):
                 if proj is not None:
                     upd = proj.project_back(upd)
                 p.data.add_((-group["lr"] * (upd + group["weight_decay"] * p.data.float())).to(p.dtype))
+                torch.autograd.graph.increment_version(p)          # written through .data: copies made of it are out of date
         return loss
 
 

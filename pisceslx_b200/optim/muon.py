@@ -257,6 +257,7 @@ class YvMuon(torch.optim.Optimizer):
             kernels().muon_apply(p.data, O.to(torch.bfloat16).contiguous(), lr, wd, scale)
         else:
             p.data.mul_(1 - lr * wd).add_(O.to(p.dtype), alpha=-lr * scale)
+        torch.autograd.graph.increment_version(p)                  # written through .data: copies made of it are out of date
 
     # ---- AdamW piece ----------------------------------------------------------------------------------
     def _apply_adamw(self, p: torch.Tensor, grad: torch.Tensor, group: Dict[str, Any]) -> None:
@@ -269,6 +270,7 @@ class YvMuon(torch.optim.Optimizer):
         else:
             ref.adamw_step(p.data, grad.to(p.dtype) * self._grad_scale, st["adam_exp_avg"], st["adam_exp_avg_sq"],
                            group["lr"], b1, b2, group["eps"], group["weight_decay"], st["adam_step"])
+        torch.autograd.graph.increment_version(p)
 
     # ---- plain mode ------------------------------------------------------------------------------------
     @torch.no_grad()

@@ -260,5 +260,6 @@ class YvGradientSynchronizer:
                 dist.all_gather(parts, g.my_param_shard().clone(), group=g.group)
                 g.flat_param.copy_(torch.cat(parts))
             for n, p in g.named:
+                torch.autograd.graph.increment_version(p)          # the gather writes the flat buffer behind the parameters
                 if p.grad is not None and g.owner[n] == g.rank:
                     p.grad = None

@@ -11,6 +11,7 @@ from __future__ import annotations
 from typing import Optional, Tuple
 
 import torch
+from torch.utils.weak import WeakIdKeyDictionary
 
 from . import kernels, reference as ref, status_word
 
@@ -234,19 +235,19 @@ class _MoEExpertsFn(torch.autograd.Function):
         return dx, dw13, dw2, dwts.to(ctx.w_dtype), None, None, None, None, None, (dout if ctx.has_add else None), None
 
 
-_MX_WEIGHTS: dict = {}
+_MX_WEIGHTS = WeakIdKeyDictionary()      # the copies of a weight live as long as the tensor that they were made of
 
 
 def _mx_weight(w: torch.Tensor):
     """Block-scaled copy of a stacked expert weight [E, N, K] (quantised again only after the tensor changed)."""
     from ..quant import fp8 as q8
     key = (w.data_ptr(), w._version, tuple(w.shape))
-    hit = _MX_WEIGHTS.get(w.data_ptr())
+    hit = _MX_WEIGHTS.get(w)
     if hit is None or hit[0] != key:
         E, N, Kd = w.shape
         q, sf = q8.quantize_mx(w.detach().reshape(E * N, Kd))
         hit = (key, q.view(E, N, Kd), sf)
-        _MX_WEIGHTS[w.data_ptr()] = hit
+        _MX_WEIGHTS[w] = hit
     return hit[1], hit[2]
 
 

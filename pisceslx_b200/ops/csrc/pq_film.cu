@@ -63,7 +63,7 @@ __device__ __forceinline__ bool pq_wait(uint64_t* bar, uint32_t parity, uint32_t
   while (true) {
     if (mbar_try_wait(bar, parity)) return true;
     if ((++spins & 0xFFu) == 0u) {
-      if (status != nullptr && *reinterpret_cast<volatile uint32_t*>(status) != 0u) return false;
+      if (gave_up(status)) return false;
       if (globaltimer_ns() - t0 > YV_WAIT_LIMIT_NS) {
         if (status != nullptr) atomicOr(status, kStatusWaitTimeout | (0x100u << where));
         return false;

@@ -139,6 +139,20 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr, uint32_t rank) {
   return v;
 }
 
+__device__ __forceinline__ uint32_t ld_cluster_u32(uint32_t addr, uint32_t rank) {
+  uint32_t v;
+  asm volatile(
+      "{\n"
+      ".reg .b32 ra;\n"
+      "mapa.shared::cluster.u32 ra, %1, %2;\n"
+      "ld.shared::cluster.u32 %0, [ra];\n"
+      "}\n"
+      : "=r"(v)
+      : "r"(addr), "r"(rank)
+      : "memory");
+  return v;
+}
+
 // Four consecutive outputs of one token; columns at or past `n` are dropped.
 __device__ __forceinline__ void skinny_store4(void* out, int fp32, long long at, int col, int n, float4 v) {
   float f[4] = {v.x, v.y, v.z, v.w};
@@ -179,6 +193,7 @@ __global__ void __launch_bounds__(kSkThreads, 2) skinny_kernel(const __grid_cons
   uint64_t* acc_full = empty_bar + kStages;
   uint64_t* acc_empty = acc_full + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+  uint32_t* failed = tmem_slot + 1;                // dense: a wait of this CTA ran out
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // the swizzled tiles need shared memory that starts on 1024 bytes
@@ -214,6 +229,7 @@ __global__ void __launch_bounds__(kSkThreads, 2) skinny_kernel(const __grid_cons
       mbar_init(&acc_full[s], 1);
       mbar_init(&acc_empty[s], 1);
     }
+    *failed = 0u;
     fence_barrier_init();
   }
   if (warp == 1) {
@@ -312,7 +328,10 @@ __global__ void __launch_bounds__(kSkThreads, 2) skinny_kernel(const __grid_cons
             "}\n"
             : "+r"(ok)::"memory");
         live = ok != 0u;
-        if (!live) break;
+        if (!live) {
+          if (tid == 0) *failed = 1u;
+          break;
+        }
         tc_fence_after_sync();
         const uint32_t taddr = tmem_base + static_cast<uint32_t>(acc * NT) + (static_cast<uint32_t>(quarter * 32) << 16);
         const int boxes = (cnt + 15) / 16;
@@ -351,12 +370,15 @@ __global__ void __launch_bounds__(kSkThreads, 2) skinny_kernel(const __grid_cons
   tc_fence_before_sync();
   if (skinny_dense(MODE)) {
     cluster_sync_all();                            // every slice's sums are in its shared memory
-    const bool bad = p.status != nullptr && *reinterpret_cast<volatile uint32_t*>(p.status) != 0u;
+    // a slice whose sums did not arrive: zeros, so that no stale memory is read further on.  What other kernels reported is
+    // no reason to leave the product out.
+    bool bad = false;
+    for (int s = 0; s < slices; ++s) bad |= ld_cluster_u32(smem_u32(failed), static_cast<uint32_t>(s)) != 0u;
     const uint32_t base = smem_u32(smem);
     constexpr int kQuads = MODE == 3 ? 16 : 32;              // groups of four outputs per token
     const int col0 = first * 4 * kQuads;
     const float f = MODE == 3 ? skinny_factor(p, col0 / p.seg) : 1.f;      // a tile lies in one segment
-    for (int w = slice * kSkThreads + static_cast<int>(threadIdx.x); !bad && w < p.M * kQuads; w += slices * kSkThreads) {
+    for (int w = slice * kSkThreads + static_cast<int>(threadIdx.x); w < p.M * kQuads; w += slices * kSkThreads) {
       const int tok = w / kQuads, c = (w % kQuads) * 4, col = col0 + c;
       if (col >= p.N) continue;
       const uint32_t at = base + static_cast<uint32_t>(tok * kSkRows + c) * 4u;
@@ -383,6 +405,7 @@ __global__ void __launch_bounds__(kSkThreads, 2) skinny_kernel(const __grid_cons
         if (col + 2 < p.N) o.z += __bfloat162float(p.bias[col + 2]);
         if (col + 3 < p.N) o.w += __bfloat162float(p.bias[col + 3]);
       }
+      if (bad) o = make_float4(0.f, 0.f, 0.f, 0.f);
       skinny_store4(p.out, p.out_fp32, tok * p.ldo + col, col, p.N, o);
     }
     cluster_sync_all();                            // nobody reads this CTA's shared memory any more

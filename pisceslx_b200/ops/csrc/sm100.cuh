@@ -137,8 +137,15 @@ __device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
 #define YV_WAIT_LIMIT_NS 2000000000ull
 #endif
 
+// A wait somewhere has run out.  An index that was reported does not count: the kernels that report one skip the access and
+// carry on, and so does whatever runs behind them.
+constexpr uint32_t kStatusGaveUp = kStatusWaitTimeout | kStatusPeerTimeout;
+__device__ __forceinline__ bool gave_up(const uint32_t* status) {
+  return status != nullptr && (*reinterpret_cast<const volatile uint32_t*>(status) & kStatusGaveUp) != 0u;
+}
+
 // Bounded wait.  Returns false (and records kStatusWaitTimeout) when the limit ran out or when
-// another thread of the grid already reported a failure.
+// another thread of the grid already reported that one did.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32_t* status) {
   if (mbar_try_wait(bar, parity)) return true;
   const uint64_t t0 = globaltimer_ns();
@@ -146,7 +153,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32
   while (true) {
     if (mbar_try_wait(bar, parity)) return true;
     if ((++spins & 0xFFu) == 0u) {
-      if (status != nullptr && *reinterpret_cast<volatile uint32_t*>(status) != 0u) return false;
+      if (gave_up(status)) return false;
       if (globaltimer_ns() - t0 > YV_WAIT_LIMIT_NS) {
         if (status != nullptr) atomicOr(status, kStatusWaitTimeout);
         return false;

@@ -301,12 +301,7 @@ __global__ void __launch_bounds__(kAttnBwdThreads, 1) attn_bwd_dq_kernel(const _
   }
 
   tc_fence_before_sync();
-  __syncthreads();
-  if (p.status != nullptr && *reinterpret_cast<volatile uint32_t*>(p.status) != 0u) {
-    const uint64_t t0 = globaltimer_ns();
-    while (globaltimer_ns() - t0 < 200000ull) { __nanosleep(1000); }
-    __syncthreads();
-  }
+  block_settle(p.status);
   if (warp == 1) { tc_fence_after_sync(); tmem_dealloc(tmem_base, kTmemCols); }
 }
 

@@ -410,13 +410,7 @@ portion_attn_kernel(const __grid_constant__ PortionAttnParams p) {
   }
 
   tc_fence_before_sync();
-  __syncthreads();
-  if (p.status != nullptr && *reinterpret_cast<volatile uint32_t*>(p.status) != 0u) {
-    // a wait may have run out with copies still in flight: let them land before the memory is released
-    const uint64_t t0 = globaltimer_ns();
-    while (globaltimer_ns() - t0 < 200000ull) { __nanosleep(1000); }
-    __syncthreads();
-  }
+  block_settle(p.status);
   if (warp == 1) {
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, kTmemCols);

@@ -329,18 +329,12 @@ __global__ void __launch_bounds__(kPqThreads, 1) pq_film_kernel(const __grid_con
       }
     }
     it += static_cast<uint32_t>(tiles_n);
-    __syncthreads();
-    if (p.status != nullptr && *reinterpret_cast<volatile uint32_t*>(p.status) != 0u) break;
+    if (block_gave_up(p.status)) break;
   }
   if (threadIdx.x == 64) tma_store_wait_all<0>();
 
   tc_fence_before_sync();
-  __syncthreads();
-  if (p.status != nullptr && *reinterpret_cast<volatile uint32_t*>(p.status) != 0u) {
-    const uint64_t t0 = globaltimer_ns();
-    while (globaltimer_ns() - t0 < 200000ull) { __nanosleep(1000); }
-    __syncthreads();
-  }
+  block_settle(p.status);
   if (warp == 1) {
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, 256);

@@ -409,15 +409,8 @@ __global__ void __launch_bounds__(kSkThreads, 2) skinny_kernel(const __grid_cons
       skinny_store4(p.out, p.out_fp32, tok * p.ldo + col, col, p.N, o);
     }
     cluster_sync_all();                            // nobody reads this CTA's shared memory any more
-  } else {
-    __syncthreads();
   }
-  if (p.status != nullptr && *reinterpret_cast<volatile uint32_t*>(p.status) != 0u) {
-    // a wait ran out somewhere: let loads in flight land before shared memory and TMEM are released
-    const uint64_t t0 = globaltimer_ns();
-    while (globaltimer_ns() - t0 < 200000ull) { __nanosleep(1000); }
-    __syncthreads();
-  }
+  block_settle(p.status);
   if (warp == 1) {
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, kTmemCols);

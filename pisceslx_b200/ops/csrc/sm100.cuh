@@ -162,6 +162,22 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32
   }
 }
 
+// The same answer in all threads of the block, and a barrier: threads that each read the word behind a barrier would part when
+// another block sets it between their reads, and the next barrier would not fill.
+__device__ __forceinline__ bool block_gave_up(const uint32_t* status) {
+  __syncwarp();                                    // one thread of a warp may have worked alone
+  return __syncthreads_or(gave_up(status) ? 1 : 0) != 0;
+}
+
+// The end of a block whose waits may have run out (a barrier): copies and products that are still in flight get time to land
+// before shared memory and TMEM are released.
+__device__ __forceinline__ void block_settle(const uint32_t* status) {
+  if (!block_gave_up(status)) return;
+  const uint64_t t0 = globaltimer_ns();
+  while (globaltimer_ns() - t0 < 200000ull) { __nanosleep(1000); }
+  __syncthreads();
+}
+
 // ---------------------------------------------------------------------------------------------
 // TMA (tiled bulk tensor copies).  The innermost coordinate times the element size must be a
 // multiple of 16 bytes; callers in this directory only pass multiples of the 128-byte swizzle span.

@@ -224,19 +224,20 @@ void swiglu_fwd(const Tensor& in, Tensor out, const c10::optional<Tensor>& scale
                                  scale.has_value() ? static_cast<int>(scale->numel()) : 1, cur_stream()), "swiglu_fwd");
 }
 
-// row_w holds one weight per row, or (fewer) one per row modulo its length; actw is optional
+// row_w holds one weight per row or, with a period, one per row modulo the period; actw is optional
 void swiglu_bwd_rows(const Tensor& in, const Tensor& dact, const Tensor& row_w, Tensor din, const c10::optional<Tensor>& actw,
-                     Tensor rowdot) {
+                     Tensor rowdot, int64_t period) {
   check_bf16(in, "in"); check_bf16(dact, "dact"); check_bf16(din, "din");
   if (actw.has_value()) check_bf16(*actw, "actw");
   TORCH_CHECK(in.is_contiguous() && dact.is_contiguous() && din.is_contiguous() && (!actw.has_value() || actw->is_contiguous()) &&
               row_w.is_contiguous() && rowdot.is_contiguous(), "swiglu_bwd_rows: contiguous expected");
   TORCH_CHECK(row_w.scalar_type() == at::kFloat && rowdot.scalar_type() == at::kFloat, "swiglu_bwd_rows: fp32 row vectors");
   const int F = static_cast<int>(dact.size(-1));
-  const int64_t rows = dact.numel() / F, period = row_w.numel() == rows ? 0 : row_w.numel();
+  const int64_t rows = dact.numel() / F;
   TORCH_CHECK(in.size(-1) == 2 * F && in.numel() == rows * 2 * F && din.numel() == in.numel() &&
               (!actw.has_value() || actw->numel() == dact.numel()) && rowdot.numel() == rows &&
-              (period == 0 || rows % period == 0), "swiglu_bwd_rows: shape mismatch");
+              period >= 0 && row_w.numel() == (period > 0 ? period : rows) && (period == 0 || rows % period == 0),
+              "swiglu_bwd_rows: shape mismatch");
   const c10::cuda::CUDAGuard guard(in.device());
   check_rc(yv::launch_swiglu_bwd_rows(in.data_ptr(), dact.data_ptr(), row_w.data_ptr<float>(), din.data_ptr(),
                                       actw.has_value() ? actw->data_ptr() : nullptr, rowdot.data_ptr<float>(), rows, F,

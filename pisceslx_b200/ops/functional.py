@@ -323,7 +323,7 @@ class _SwiGLUMixFn(torch.autograd.Function):
         d2 = _as2d(dout).contiguous()
         din = torch.empty_like(g2)
         dots = torch.empty(g2.shape[0], dtype=torch.float32, device=g2.device)
-        _k().swiglu_bwd_rows(g2, d2, mix, din, None, dots)
+        _k().swiglu_bwd_rows(g2, d2, mix, din, None, dots, mix.numel())
         return din.view(ctx.shape), dots.view(-1, mix.numel()).sum(0) if ctx.needs_input_grad[1] else None
 
 

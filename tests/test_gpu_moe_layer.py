@@ -106,3 +106,13 @@ def test_gate_in_fp32_is_read_as_it_is():
         got, fresh = layer.router(x)[0], copy.deepcopy(layer.router)(x)[0]
         graph.replay()
     assert torch.equal(got, fresh) and torch.equal(captured, fresh)
+
+
+@pytest.mark.parametrize("weights,period", [(0, 0), (3, 0), (12, 3), (5, 5), (3, -3), (0, 3)])
+def test_row_weights_of_another_number_are_refused(weights, period):
+    """One weight per row, or one per row modulo a period that divides the rows: the host checks it."""
+    from pisceslx_b200.ops import kernels
+    inp, dact = torch.zeros(12, 32, device=DEV).bfloat16(), torch.zeros(12, 16, device=DEV).bfloat16()
+    out = (torch.empty_like(inp), torch.empty_like(dact), torch.empty(12, device=DEV))
+    with pytest.raises(RuntimeError, match="swiglu_bwd_rows"):
+        kernels().swiglu_bwd_rows(inp, dact, torch.ones(weights, device=DEV), *out, period)

@@ -32,6 +32,34 @@ int launch(const SkinnyParams& p, int grid, int cluster, cudaStream_t stream) {
   return launch_chained(kern, dim3(static_cast<unsigned>(grid)), dim3(kSkThreads), SkinnySmem<NT>::kTotal, stream, cluster, p);
 }
 
+// Clusters of `slices` CTAs that the device holds at two CTAs per SM: fewer than the CTAs would allow, since a cluster stays
+// within one group of SMs (148 of two, 93 of three, 71 of four, 45 of six, 33 of eight).  An empty kernel of the same shape
+// is asked about, since the answer for a kernel that allocates tensor memory counts one CTA per SM.
+__global__ void __launch_bounds__(kSkThreads, 2) skinny_shape_kernel() {}
+
+int clusters_at_once(int slices) {
+  static PerDeviceInt known[9];
+  int& n = known[slices].cur();
+  if (n != 0) return n;
+  auto kern = skinny_shape_kernel;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(slices));
+  cfg.blockDim = dim3(kSkThreads);
+  cfg.dynamicSmemBytes = SkinnySmem<128>::kTotal;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = static_cast<unsigned>(slices);
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int found = 0;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SkinnySmem<128>::kTotal) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&found, kern, &cfg) != cudaSuccess || found <= 0)
+    found = 1;
+  return n = found;
+}
+
 template <int MODE>
 int dispatch(int tokens, const SkinnyParams& p, int grid, int cluster, cudaStream_t stream) {
   if (tokens <= 16) return launch<16, MODE>(p, grid, cluster, stream);
@@ -66,11 +94,12 @@ int launch_skinny(const SkinnyArgs& a, cudaStream_t stream) {
     p.scale = a.scale;
     p.scale_fp32 = a.scale_fp32;
     p.scale_softmax = a.scale_softmax;
-    // as many slices of K as keep all CTAs resident (two per SM) and leave four 64-wide steps to each
-    const int kc = (a.K + 63) / 64, room = 2 * sm_count() / p.tiles_w;
+    // as many slices of K as keep all clusters resident and leave four 64-wide steps to each; one cluster more than fits costs
+    // a second round (6144 x 4096, one token: 48 clusters of six 15.8 us, of four 12.4; 128 tokens 24.5 and 18.4)
+    const int kc = (a.K + 63) / 64;
     int slices = 1;
     for (int s : {2, 3, 4, 6, 8})
-      if (s <= room && s * 4 <= kc) slices = s;
+      if (s * 4 <= kc && p.tiles_w <= clusters_at_once(s)) slices = s;
     const int grid = p.tiles_w * slices;
     return a.swiglu ? dispatch<3>(a.M, p, grid, slices, stream) : dispatch<0>(a.M, p, grid, slices, stream);
   }

@@ -12,10 +12,11 @@
 //   grouped  Persistent CTAs over (tile of <= 128 tokens of one expert, 128 weight rows).  With SWIGLU the 128 rows are 64
 //            gate rows and their 64 up rows, and silu(gate) * up leaves the kernel; the products stay in fp32 until then.
 //
-// Bound by HBM and, for the smaller matrices, by about 5 us of start and end.  Measured in a graph, weights not in L2, one
-// token (before: the split of K by the general kernel and a second kernel that added the parts): 11264 x 4096 18.7 us,
-// 32000 x 4096 44.7 us (5.9 TB/s; before 57), 6144 x 4096 16.4, 4096 x 4096 10.8, 4096 x 5632 12.5, 64 x 4096 5.5 (before 18);
-// 64 experts of 4096 x 1408 with 64 tokens, top-6, both products and the activation 350 us (6.3 TB/s; before 435).
+// Bound by HBM and, for the smaller matrices, by some 4 us of start and end.  Measured in a graph, weights not in L2, one token
+// (before: the split of K by the general kernel and a second kernel that added the parts): 11264 x 4096 16.8 us, 32000 x 4096
+// 44.4 (5.9 TB/s; before 57), 6144 x 4096 12.4, 4096 x 4096 9.2, 4096 x 5632 11.1, 64 x 4096 4.7 (before 8); 128 tokens
+// 23.2 (28), 49.7 (50), 18.4 (18), 14.7 (16), 16.6 (17), 7.0 (8); 64 experts of 4096 x 1408 with 64 tokens, top-6, both
+// products and the activation 350 us (6.3 TB/s; before 435).
 #pragma once
 #include "chain.cuh"
 #include "sm100.cuh"
@@ -153,10 +154,9 @@ __device__ __forceinline__ uint32_t ld_cluster_u32(uint32_t addr, uint32_t rank)
   return v;
 }
 
-// Four consecutive outputs of one token; columns at or past `n` are dropped.
-__device__ __forceinline__ void skinny_store4(void* out, int fp32, long long at, int col, int n, float4 v) {
+// Four consecutive outputs of one token, as one vector if `whole`; columns at or past `n` are dropped.
+__device__ __forceinline__ void skinny_store4(void* out, int fp32, long long at, int col, int n, bool whole, float4 v) {
   float f[4] = {v.x, v.y, v.z, v.w};
-  const bool whole = col + 4 <= n && (at & 3) == 0;
   if (fp32) {
     float* o = static_cast<float*>(out) + at;
     if (whole) {
@@ -175,6 +175,75 @@ __device__ __forceinline__ void skinny_store4(void* out, int fp32, long long at,
       for (int i = 0; i < 4; ++i)
         if (col + i < n) o[i] = __float2bfloat16(f[i]);
     }
+  }
+}
+
+// Outputs of a dense tile: the sums of the SLICES CTAs of the cluster in their order.  A thread owns four neighbouring columns
+// and takes every kRows-th token, eight loads ahead of their use: the few warps have nothing else to hide a load or an address
+// behind (one token at a time with its own addresses, 128 tokens of one slice took 6500 cycles).
+// A slice whose sums did not arrive gives zeros, so that no stale memory is read further on; what other kernels reported is no
+// reason to leave the product out.
+template <int MODE, int SLICES>
+__device__ __forceinline__ void skinny_sum(const SkinnyParams& p, uint8_t* smem, int slice, int col0, float f, uint32_t failed) {
+  constexpr int kQuads = MODE == 3 ? 16 : 32;              // groups of four outputs per token
+  constexpr int kLoads = SLICES * (MODE == 3 ? 2 : 1);
+  constexpr int kAtOnce = kLoads >= 8 ? 1 : 8 / kLoads;
+  constexpr int kRows = SLICES * kSkThreads / kQuads;      // tokens that the cluster's threads cover at a time
+  const int c = (static_cast<int>(threadIdx.x) % kQuads) * 4, col = col0 + c;
+  if (col >= p.N) return;
+  const bool whole = col + 4 <= p.N && (p.ldo & 3) == 0;
+  uint32_t bad = 0u;
+#pragma unroll
+  for (int s = 0; s < SLICES; ++s) bad |= ld_cluster_u32(failed, static_cast<uint32_t>(s));
+  float4 bias = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (p.bias != nullptr) {
+    bias.x = __bfloat162float(p.bias[col]);
+    if (col + 1 < p.N) bias.y = __bfloat162float(p.bias[col + 1]);
+    if (col + 2 < p.N) bias.z = __bfloat162float(p.bias[col + 2]);
+    if (col + 3 < p.N) bias.w = __bfloat162float(p.bias[col + 3]);
+  }
+  const int tok0 = slice * (kSkThreads / kQuads) + static_cast<int>(threadIdx.x) / kQuads;
+  const float* mine = reinterpret_cast<const float*>(smem) + tok0 * kSkRows + c;
+  const uint32_t mine_addr = smem_u32(smem) + static_cast<uint32_t>(tok0 * kSkRows + c) * 4u;
+  auto load = [&](int row, int s) -> float4 {              // `row`: tokens past tok0, or half a row for the up part
+    if (SLICES == 1) return *reinterpret_cast<const float4*>(mine + row);
+    return ld_cluster_f4(mine_addr + static_cast<uint32_t>(row) * 4u, static_cast<uint32_t>(s));
+  };
+  const long long step = static_cast<long long>(kRows) * p.ldo;
+  long long at = static_cast<long long>(tok0) * p.ldo + col;
+  int row = 0;
+  for (int tok = tok0; tok < p.M; tok += kAtOnce * kRows) {
+    float4 v[kAtOnce][SLICES], up[kAtOnce][MODE == 3 ? SLICES : 1];
+#pragma unroll
+    for (int j = 0; j < kAtOnce; ++j) {
+      if (tok + j * kRows < p.M) {
+#pragma unroll
+        for (int s = 0; s < SLICES; ++s) {
+          v[j][s] = load(row + j * kRows * kSkRows, s);
+          if (MODE == 3) up[j][s] = load(row + j * kRows * kSkRows + 64, s);
+        }
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < kAtOnce; ++j) {
+      if (tok + j * kRows < p.M) {
+        float4 o = v[j][0];
+#pragma unroll
+        for (int s = 1; s < SLICES; ++s) { o.x += v[j][s].x; o.y += v[j][s].y; o.z += v[j][s].z; o.w += v[j][s].w; }
+        if (MODE == 3) {
+          float4 u = up[j][0];
+#pragma unroll
+          for (int s = 1; s < SLICES; ++s) { u.x += up[j][s].x; u.y += up[j][s].y; u.z += up[j][s].z; u.w += up[j][s].w; }
+          o = make_float4(f * swiglu1(o.x, u.x), f * swiglu1(o.y, u.y), f * swiglu1(o.z, u.z), f * swiglu1(o.w, u.w));
+        } else {
+          o.x += bias.x; o.y += bias.y; o.z += bias.z; o.w += bias.w;
+        }
+        if (bad != 0u) o = make_float4(0.f, 0.f, 0.f, 0.f);
+        skinny_store4(p.out, p.out_fp32, at, col, p.N, whole, o);
+        at += step;
+      }
+    }
+    row += kAtOnce * kRows * kSkRows;
   }
 }
 
@@ -335,16 +404,31 @@ __global__ void __launch_bounds__(kSkThreads, 2) skinny_kernel(const __grid_cons
         tc_fence_after_sync();
         const uint32_t taddr = tmem_base + static_cast<uint32_t>(acc * NT) + (static_cast<uint32_t>(quarter * 32) << 16);
         const int boxes = (cnt + 15) / 16;
-        for (int b = 0; b < boxes; ++b) {
+        if (skinny_dense(MODE)) {
+          // [token][weight row], where all slices' threads find it
+          float* st = reinterpret_cast<float*>(smem) + row;
+          for (int b = 0; b < boxes; b += 2) {
+            uint32_t v[2][16];
+            tmem_ld16(taddr + 16 * b, v[0]);
+            if (b + 1 < boxes) tmem_ld16(taddr + 16 * b + 16, v[1]);
+            tc_wait_ld();
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+              if (b + j < boxes) {
+#pragma unroll
+                for (int i = 0; i < 16; ++i) st[(16 * (b + j) + i) * kSkRows] = __uint_as_float(v[j][i]);
+              }
+          }
+        }
+        for (int b = 0; !skinny_dense(MODE) && b < boxes; ++b) {
           uint32_t v[16];
           tmem_ld16(taddr + 16 * b, v);
           tc_wait_ld();
           // staged as [token][weight row], so that consecutive threads write consecutive outputs of one token
-          float* st = skinny_dense(MODE) ? reinterpret_cast<float*>(smem) + 16 * b * kSkRows : epi;
-          if (!skinny_dense(MODE) && b > 0) asm volatile("bar.sync 1, 128;" ::: "memory");
+          float* st = epi;
+          if (b > 0) asm volatile("bar.sync 1, 128;" ::: "memory");
 #pragma unroll
           for (int i = 0; i < 16; ++i) st[i * kSkRows + row] = __uint_as_float(v[i]);
-          if (skinny_dense(MODE)) continue;
           asm volatile("bar.sync 1, 128;" ::: "memory");
           constexpr int kQuads = MODE == 2 ? 16 : 32;          // groups of four outputs per token
 #pragma unroll
@@ -356,7 +440,8 @@ __global__ void __launch_bounds__(kSkThreads, 2) skinny_kernel(const __grid_cons
               o = make_float4(swiglu1(o.x, up.x), swiglu1(o.y, up.y), swiglu1(o.z, up.z), swiglu1(o.w, up.w));
             }
             if (16 * b + tok < cnt)
-              skinny_store4(p.out, 0, (t.x_row + at + 16 * b + tok) * p.ldo + t.col + c, t.col + c, p.N, o);
+              skinny_store4(p.out, 0, (t.x_row + at + 16 * b + tok) * p.ldo + t.col + c, t.col + c, p.N,
+                            t.col + c + 4 <= p.N && (p.ldo & 3) == 0, o);
           }
         }
         tc_fence_before_sync();
@@ -369,46 +454,18 @@ __global__ void __launch_bounds__(kSkThreads, 2) skinny_kernel(const __grid_cons
   __syncwarp();                                    // the aligned barriers below need whole warps
   tc_fence_before_sync();
   if (skinny_dense(MODE)) {
-    cluster_sync_all();                            // every slice's sums are in its shared memory
-    // a slice whose sums did not arrive: zeros, so that no stale memory is read further on.  What other kernels reported is
-    // no reason to leave the product out.
-    bool bad = false;
-    for (int s = 0; s < slices; ++s) bad |= ld_cluster_u32(smem_u32(failed), static_cast<uint32_t>(s)) != 0u;
-    const uint32_t base = smem_u32(smem);
-    constexpr int kQuads = MODE == 3 ? 16 : 32;              // groups of four outputs per token
-    const int col0 = first * 4 * kQuads;
+    if (slices > 1) cluster_sync_all(); else __syncthreads();      // every slice's sums are in its shared memory
+    const int col0 = first * (MODE == 3 ? 64 : kSkRows);
     const float f = MODE == 3 ? skinny_factor(p, col0 / p.seg) : 1.f;      // a tile lies in one segment
-    for (int w = slice * kSkThreads + static_cast<int>(threadIdx.x); w < p.M * kQuads; w += slices * kSkThreads) {
-      const int tok = w / kQuads, c = (w % kQuads) * 4, col = col0 + c;
-      if (col >= p.N) continue;
-      const uint32_t at = base + static_cast<uint32_t>(tok * kSkRows + c) * 4u;
-      float4 v[8], up[8];
-#pragma unroll
-      for (int s = 0; s < 8; ++s)
-        if (s < slices) {
-          v[s] = ld_cluster_f4(at, static_cast<uint32_t>(s));
-          if (MODE == 3) up[s] = ld_cluster_f4(at + 256u, static_cast<uint32_t>(s));
-        }
-      float4 o = v[0], u = up[0];
-#pragma unroll
-      for (int s = 1; s < 8; ++s)
-        if (s < slices) {
-          o.x += v[s].x; o.y += v[s].y; o.z += v[s].z; o.w += v[s].w;
-          if (MODE == 3) { u.x += up[s].x; u.y += up[s].y; u.z += up[s].z; u.w += up[s].w; }
-        }
-      if (MODE == 3) {
-        o = make_float4(f * swiglu1(o.x, u.x), f * swiglu1(o.y, u.y), f * swiglu1(o.z, u.z), f * swiglu1(o.w, u.w));
-      }
-      if (p.bias != nullptr) {
-        o.x += __bfloat162float(p.bias[col]);
-        if (col + 1 < p.N) o.y += __bfloat162float(p.bias[col + 1]);
-        if (col + 2 < p.N) o.z += __bfloat162float(p.bias[col + 2]);
-        if (col + 3 < p.N) o.w += __bfloat162float(p.bias[col + 3]);
-      }
-      if (bad) o = make_float4(0.f, 0.f, 0.f, 0.f);
-      skinny_store4(p.out, p.out_fp32, tok * p.ldo + col, col, p.N, o);
+    switch (slices) {
+      case 1: skinny_sum<MODE, 1>(p, smem, slice, col0, f, smem_u32(failed)); break;
+      case 2: skinny_sum<MODE, 2>(p, smem, slice, col0, f, smem_u32(failed)); break;
+      case 3: skinny_sum<MODE, 3>(p, smem, slice, col0, f, smem_u32(failed)); break;
+      case 4: skinny_sum<MODE, 4>(p, smem, slice, col0, f, smem_u32(failed)); break;
+      case 6: skinny_sum<MODE, 6>(p, smem, slice, col0, f, smem_u32(failed)); break;
+      default: skinny_sum<MODE, 8>(p, smem, slice, col0, f, smem_u32(failed));
     }
-    cluster_sync_all();                            // nobody reads this CTA's shared memory any more
+    if (slices > 1) cluster_sync_all();            // nobody reads this CTA's shared memory any more
   }
   block_settle(p.status);
   if (warp == 1) {

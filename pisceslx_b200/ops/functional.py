@@ -102,6 +102,14 @@ def gemm_skinny(x2: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] 
     return out
 
 
+def _few_rows(N: int, K: int) -> bool:
+    """Whether products of up to 128 rows with these weights go to ``gemm_skinny``.  N and K decide alone, so that rows agree
+    whatever their number.  More tiles than find a place at once (two per SM) start up again for each round, and short sums
+    are over before it pays: 1, 64 and 128 rows of 154856 x 1024 58, 71 and 94 us, by the general kernel 63, 62 and 66; of
+    256 x 256 3.7, 5.8 and 7.9 against 5.0, 5.0 and 5.1; of 2048 x 512 4.3, 6.2 and 7.7 against 7.6, 7.6 and 7.8."""
+    return (N <= 2 * 148 * 128 and K >= 512) or N % 8 != 0              # the general kernel takes no odd widths
+
+
 def skinny_swiglu(x2: torch.Tensor, w: torch.Tensor, seg: int, scale: Optional[torch.Tensor] = None,
                   softmax: bool = False) -> Optional[torch.Tensor]:
     """silu(gate) * up of up to 128 rows in the kernel that streams the weights, without a gradient: ``w`` holds ``seg`` gate
@@ -136,7 +144,7 @@ class _LinearFn(torch.autograd.Function):
         ctx.save_for_backward(x2, w)
         ctx.x_shape = x.shape
         out_dtype = torch.float32 if out_fp32 else _BF16
-        y = gemm_skinny(x2, w, None, out_dtype)
+        y = gemm_skinny(x2, w, None, out_dtype) if _few_rows(*w.shape) else None
         if y is None:
             y = gemm(x2, w, out_dtype=out_dtype)
         return y.view(*x.shape[:-1], w.shape[0])

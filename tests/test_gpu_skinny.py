@@ -32,9 +32,10 @@ def test_rows_match_fp64_and_do_not_depend_on_their_neighbours(M, N, K):
 
 
 @pytest.mark.parametrize("T,E,H,F,same", [(1, 8, 256, 64, False), (17, 8, 264, 192, False), (130, 4, 128, 64, False),
-                                          (200, 16, 520, 128, True)])
+                                          (200, 16, 520, 128, True), (100, 16, 264, 128, True)])
 def test_experts_without_gradient_match_fp64(T, E, H, F, same):
-    """Few tokens, odd widths, and all tokens at the same experts: more than one pass and more than one tile each."""
+    """Few tokens, odd widths, and all tokens at the same experts: 200 fill more than one tile, 100 more than the 64 slots of a
+    pass."""
     g = torch.Generator("cuda").manual_seed(T)
     x = torch.randn(T, H, device="cuda", generator=g).bfloat16()
     w13 = (torch.randn(E, 2 * F, H, device="cuda", generator=g) * H ** -0.5).bfloat16()
@@ -99,3 +100,40 @@ def test_combine_adds_the_shared_experts(T):
     assert _distance(both.detach(), alone.double() + add.detach().double()) < 2 * 2.0 ** -8
     grad = torch.randn(T, H, device="cuda", generator=g).bfloat16()
     assert torch.equal(torch.autograd.grad(both, add, grad)[0], grad)
+
+
+@pytest.mark.parametrize("slots", [1, 16, 32, 64, 128])
+def test_passes_over_a_tile(slots):
+    """Tiles of 1 to 128 tokens in passes of 16 to 128: each pass reads the weights again, takes the next tokens and the other
+    accumulator."""
+    from pisceslx_b200.ops import kernels, status_word
+    g = torch.Generator("cuda").manual_seed(slots)
+    tokens, H, F = [17, 128, 1, 0, 65, 129, 100], 264, 192
+    E, T = len(tokens), sum(tokens)
+    idx = torch.repeat_interleave(torch.arange(E), torch.tensor(tokens))[torch.randperm(T)].cuda().int()[:, None].contiguous()
+    x = torch.randn(T, H, device="cuda", generator=g).bfloat16()
+    w13 = (torch.randn(E, 2 * F, H, device="cuda", generator=g) * H ** -0.5).bfloat16()
+    counts = torch.tensor(tokens, dtype=torch.int32, device="cuda")
+    xp, plan = moe_ops.permute_tokens(x, idx, counts, E, False, False)
+    layout = (plan.tile_expert, plan.num_m_tiles, plan.seg_offsets, counts, slots)
+    y = torch.full((xp.shape[0], 2 * F), float("nan"), device="cuda", dtype=torch.bfloat16)
+    act = torch.full((xp.shape[0], F), float("nan"), device="cuda", dtype=torch.bfloat16)
+    kernels().gemm_skinny_grouped(xp, w13, y, *layout, False, status_word(x.device))
+    kernels().gemm_skinny_grouped(xp, w13, act, *layout, True, status_word(x.device))
+    rows = plan.row_map[:, 0].long()
+    want = torch.einsum("th,tnh->tn", x.double(), w13[idx[:, 0].long()].double())
+    gate, up = want.chunk(2, -1)
+    assert _distance(y[rows], want) < 2.0 ** -8
+    assert _distance(act[rows], torch.nn.functional.silu(gate) * up) < 2.0 ** -8
+
+
+@pytest.mark.parametrize("N,K", [(6144, 4096), (4500, 4096), (9216, 3072), (37888, 256), (40000, 128)])
+def test_sizes_whose_clusters_fill_the_chip(N, K):
+    """One cluster more than fits at six, eight and four slices, the most tiles that fit, and more than fit."""
+    g = torch.Generator("cuda").manual_seed(N)
+    w = torch.randn(N, K, device="cuda", generator=g).bfloat16()
+    for M in (1, 128):
+        x = torch.randn(M, K, device="cuda", generator=g).bfloat16()
+        y = F_.linear(x, w)
+        assert _distance(y, x.double() @ w.double().t()) < LIMIT[torch.bfloat16]
+        assert torch.equal(F_.linear(x[M - 1:], w), y[M - 1:])

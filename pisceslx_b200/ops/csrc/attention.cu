@@ -261,7 +261,8 @@ int launch_kv_cache_write(const void* k, const void* v, void* k_cache, void* v_c
                           uint32_t* status, cudaStream_t stream) {
   if (tokens <= 0) return 0;
   if ((row_elems & 7) != 0) return -1;
-  return launch_chained(kv_cache_write_kernel, dim3(static_cast<unsigned>(tokens)), dim3(128), 0, stream, 0,
+  return launch_chained_if(tokens <= kChainBlocks, kv_cache_write_kernel<true>, kv_cache_write_kernel<false>,
+                           dim3(static_cast<unsigned>(tokens)), dim3(128), 0, stream,
                         reinterpret_cast<const __nv_bfloat16*>(k), reinterpret_cast<const __nv_bfloat16*>(v),
                         reinterpret_cast<__nv_bfloat16*>(k_cache), reinterpret_cast<__nv_bfloat16*>(v_cache), slot_map, row_elems,
                         k_stride, v_stride, num_slots, status);

@@ -221,12 +221,12 @@ __global__ void paged_decode_merge_kernel(const float* __restrict__ partial_o, c
 }
 
 // Append new K/V rows into the paged cache: slot = block_id * block + offset.
+template <bool CHAIN>
 __global__ void kv_cache_write_kernel(const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __restrict__ v,
                                       __nv_bfloat16* __restrict__ k_cache, __nv_bfloat16* __restrict__ v_cache,
                                       const int* __restrict__ slot_map, int row_elems, int64_t k_stride,
                                       int64_t v_stride, int64_t num_slots, uint32_t* status) {
-  chain_next();
-  chain_wait();
+  chain_start<CHAIN>();
   const int64_t t = blockIdx.x;
   const int64_t slot = slot_map[t];
   if (slot < 0) return;                       // padding token

@@ -69,7 +69,7 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 // ---------------------------------------------------------------------------------------------
 // RMSNorm forward.  One block per row; VPT 16-byte vectors per thread stay in registers.
 // ---------------------------------------------------------------------------------------------
-template <int VPT>
+template <int VPT, bool CHAIN>
 __global__ void rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ residual,
                                    const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ fscale,
                                    const __nv_bfloat16* __restrict__ fshift, int64_t film_rows,
@@ -80,8 +80,7 @@ __global__ void rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __
   const int nvec = cols >> 3;
   float v[VPT][8];
   float ss = 0.f;
-  chain_next();
-  chain_wait();
+  chain_start<CHAIN>();
 #pragma unroll
   for (int i = 0; i < VPT; ++i) {
     const int vec = threadIdx.x + i * blockDim.x;
@@ -285,20 +284,20 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ q, __nv_bfloat16* __rest
   }
 }
 
-// The same with 16-byte accesses: a thread owns eight pairs of a token and walks every eighth head with their angles in
-// registers.  `chunks` = rot_dim / 16 threads times 8 head groups per token.  Bound by memory:
+// The same with 16-byte accesses: a thread owns eight pairs of a token and walks every `groups`-th head with their angles in
+// registers.  `chunks` = rot_dim / 16 threads times `groups` per token.  Bound by memory:
 // 16384 tokens, 40 heads of 128 in 58 us (5.8 TB/s) instead of 122 with two bytes at a time.
+template <bool CHAIN>
 __global__ void __launch_bounds__(256) rope_vec_kernel(__nv_bfloat16* __restrict__ q, __nv_bfloat16* __restrict__ k,
                                                        const float* __restrict__ cos_t, const float* __restrict__ sin_t,
                                                        const int* __restrict__ positions, int64_t tokens, int hq, int hk,
-                                                       int head_dim, int chunks, int inverse, int64_t q_stride,
+                                                       int head_dim, int chunks, int groups, int inverse, int64_t q_stride,
                                                        int64_t k_stride) {
-  chain_next();
-  chain_wait();
+  chain_start<CHAIN>();
   const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-  const int64_t t = i / (chunks * 8);
+  const int64_t t = i / (chunks * groups);
   if (t >= tokens) return;
-  const int rest = static_cast<int>(i - t * chunks * 8);
+  const int rest = static_cast<int>(i - t * chunks * groups);
   const int hg = rest / chunks, p = (rest - hg * chunks) * 8, half = chunks * 8;
   const int64_t at = static_cast<int64_t>(positions[t]) * half + p;
   float c[8], s[8];
@@ -311,7 +310,7 @@ __global__ void __launch_bounds__(256) rope_vec_kernel(__nv_bfloat16* __restrict
 #pragma unroll
     for (int j = 0; j < 8; ++j) s[j] = -s[j];
   }
-  for (int h = hg; h < hq + hk; h += 8) {
+  for (int h = hg; h < hq + hk; h += groups) {
     __nv_bfloat16* base = h < hq ? q + t * q_stride + static_cast<int64_t>(h) * head_dim + p
                                  : k + t * k_stride + static_cast<int64_t>(h - hq) * head_dim + p;
     float a[8], b[8], x[8], y[8];
@@ -521,9 +520,14 @@ int launch_rmsnorm_fwd(const void* x, const void* residual, const void* w, const
   int vpt;
   const int block = norm_block(cols, &vpt);
   const unsigned grid = static_cast<unsigned>(rows);
+  // wide rows take long enough that two of them on one SM cost more than the early start gives (128 rows of 8192: 5.0 us
+  // unchained, 5.6 chained; of 4096 3.3 and 3.1; 64 rows of 16384 8.0 and 7.8)
+  const bool chain = rows <= 64 || (rows <= kChainBlocks && cols <= 4096);
 #define YV_LAUNCH(V)                                                                                          \
-  return launch_chained(rmsnorm_fwd_kernel<V>, dim3(grid), dim3(block), 0, stream, 0, YV_BF(x), YV_BF(residual), YV_BF(w),      \
-                        YV_BF(film_scale), YV_BF(film_shift), film_rows_per_group, YV_BFM(y), YV_BFM(res_out), rstd, cols, eps)
+  return launch_chained_if(chain, rmsnorm_fwd_kernel<V, true>, rmsnorm_fwd_kernel<V, false>, dim3(grid), dim3(block), 0,        \
+                           stream, YV_BF(x), YV_BF(residual),                                                             \
+                           YV_BF(w), YV_BF(film_scale), YV_BF(film_shift), film_rows_per_group, YV_BFM(y), YV_BFM(res_out), rstd, \
+                           cols, eps)
   switch (vpt) {
     case 1: YV_LAUNCH(1);
     case 2: YV_LAUNCH(2);
@@ -568,9 +572,10 @@ int launch_rope_tables(void* q, void* k, const float* cos_t, const float* sin_t,
                          reinterpret_cast<uintptr_t>(sin_t)) & 15u) == 0;
   if (rot_dim > 0 && rot_dim % 16 == 0 && head_dim % 8 == 0 && q_stride % 8 == 0 && k_stride % 8 == 0 && aligned) {
     const int chunks = rot_dim / 16;
-    return launch_chained(rope_vec_kernel, dim3(static_cast<unsigned>((tokens * chunks * 8 + 255) / 256)), dim3(256), 0, stream, 0,
-                          YV_BFM(q), YV_BFM(k), cos_t, sin_t, positions, tokens, hq, hk, head_dim, chunks, inverse, q_stride,
-                          k_stride);
+    const int64_t blocks = (tokens * chunks * 8 + 255) / 256;
+    return launch_chained_if(blocks <= 8 * kChainBlocks, rope_vec_kernel<true>, rope_vec_kernel<false>,
+                             dim3(static_cast<unsigned>(blocks)), dim3(256), 0, stream, YV_BFM(q), YV_BFM(k), cos_t, sin_t,
+                             positions, tokens, hq, hk, head_dim, chunks, 8, inverse, q_stride, k_stride);
   }
   const int total = (hq + hk) * (rot_dim >> 1);
   const int block = total >= 256 ? 256 : ((total + 31) / 32) * 32;

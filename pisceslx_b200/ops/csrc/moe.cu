@@ -230,13 +230,13 @@ __global__ void moe_plan_kernel(const int* __restrict__ counts, int* __restrict_
 }
 
 // One block per token: reserve a row in each selected expert's segment and copy the token row there.
+template <bool CHAIN>
 __global__ void moe_permute_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ idx,
                                    int* __restrict__ cursor, int* __restrict__ row_map,
                                    __nv_bfloat16* __restrict__ xp, int k, int cols) {
   __shared__ int dest[kMaxTopK];
   const int64_t t = blockIdx.x;
-  chain_next();
-  chain_wait();
+  chain_start<CHAIN>();
   if (threadIdx.x < k) {
     const int e = idx[t * k + threadIdx.x];
     const int r = atomicAdd(&cursor[e], 1);
@@ -281,14 +281,14 @@ __global__ void moe_zero_pad_kernel(__nv_bfloat16* __restrict__ xp, const int* _
 
 // grid (tokens, column parts).  The rows and weights of the token are read once, so that the k row loads go out together;
 // with few tokens the columns are spread over blocks.
+template <bool CHAIN>
 __global__ void moe_combine_kernel(const __nv_bfloat16* __restrict__ y, const int* __restrict__ row_map,
                                    const float* __restrict__ weights, const __nv_bfloat16* __restrict__ add,
                                    __nv_bfloat16* __restrict__ out, int k, int cols) {
   __shared__ int s_row[kMaxTopK];
   __shared__ float s_w[kMaxTopK];
   const int64_t t = blockIdx.x;
-  chain_next();
-  chain_wait();
+  chain_start<CHAIN>();
   if (threadIdx.x < k) {
     const float w = weights[t * k + threadIdx.x];
     s_w[threadIdx.x] = w;
@@ -547,8 +547,9 @@ int launch_moe_permute(const void* x, const int* idx, int* cursor, int* row_map,
   if ((cols & 7) != 0 || k > kMaxTopK) return -1;
   const int block = (cols >> 3) >= 256 ? 256 : 128;
   if (cursor != nullptr) {
-    return launch_chained(moe_permute_kernel, dim3(static_cast<unsigned>(tokens)), dim3(block), 0, stream, 0, YV_BF(x), idx, cursor,
-                          row_map, YV_BFM(xp), k, cols);
+    return launch_chained_if(tokens <= kChainBlocks, moe_permute_kernel<true>, moe_permute_kernel<false>,
+                             dim3(static_cast<unsigned>(tokens)), dim3(block), 0, stream, YV_BF(x), idx, cursor, row_map,
+                             YV_BFM(xp), k, cols);
   } else {
     moe_permute_mapped_kernel<<<static_cast<unsigned>(tokens), block, 0, stream>>>(YV_BF(x), row_map, YV_BFM(xp), k,
                                                                                    cols);
@@ -570,8 +571,9 @@ int launch_moe_combine(const void* y, const int* row_map, const float* weights, 
   // enough blocks for every SM when the tokens alone are too few
   const int block = (cols >> 3) >= 256 && tokens >= 148 ? 256 : 128;
   const unsigned parts = tokens >= 148 ? 1u : static_cast<unsigned>(((cols >> 3) + block - 1) / block);
-  return launch_chained(moe_combine_kernel, dim3(static_cast<unsigned>(tokens), parts), dim3(block), 0, stream, 0, YV_BF(y), row_map,
-                        weights, YV_BF(add), YV_BFM(out), k, cols);
+  return launch_chained_if(tokens <= kChainBlocks, moe_combine_kernel<true>, moe_combine_kernel<false>,
+                           dim3(static_cast<unsigned>(tokens), parts), dim3(block), 0, stream, YV_BF(y), row_map, weights, YV_BF(add), YV_BFM(out), k,
+                           cols);
 }
 
 int launch_moe_combine_bwd(const void* dout, const void* y, const int* row_map, const float* weights, void* dy,

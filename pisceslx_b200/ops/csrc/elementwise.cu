@@ -570,12 +570,24 @@ int launch_rope_tables(void* q, void* k, const float* cos_t, const float* sin_t,
   // whole vectors of pairs, and every head, row and table row on a 16-byte boundary
   const bool aligned = ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(cos_t) |
                          reinterpret_cast<uintptr_t>(sin_t)) & 15u) == 0;
-  if (rot_dim > 0 && rot_dim % 16 == 0 && head_dim % 8 == 0 && q_stride % 8 == 0 && k_stride % 8 == 0 && aligned) {
-    const int chunks = rot_dim / 16;
-    const int64_t blocks = (tokens * chunks * 8 + 255) / 256;
+  // A quarter of a head's pairs or less per thread leaves too few loads in flight: 40 heads of 128 of which 32 are rotated, 8192
+  // tokens 23.7 us by vectors and 17.3 by pairs, 1000 tokens 5.6 and 3.9; of 64, 20 heads, 13.2 and 17.5, 3.7 and 3.8.
+  if (rot_dim >= 64 && rot_dim % 16 == 0 && head_dim % 8 == 0 && q_stride % 8 == 0 && k_stride % 8 == 0 && aligned) {
+    // A thread reads its angles once for the heads that it walks, one behind the other at a load's latency: as many heads, up to
+    // an eighth of them, as still leave 2048 threads to every SM; small blocks where there is less than one for each SM.  Eight
+    // groups and blocks of 256 at any size, and now: 40 heads of 128, 1 token 3.0 and 1.8 us, 128 tokens 4.3 and 2.7, 1000 6.7
+    // and 6.1; 20 heads of 64, 128 tokens 3.5 and 2.3 (by pairs 2.4).
+    const int chunks = rot_dim / 16, heads = hq + hk;
+    const int64_t each = tokens * chunks * heads / (int64_t{148} * 2048), most = (heads + 7) / 8;
+    const int walk = static_cast<int>(each < 1 ? 1 : each < most ? each : most);
+    const int groups = (heads + walk - 1) / walk;
+    const int64_t threads = tokens * chunks * groups;
+    const int block = threads >= 148 * 256 ? 256 : 64;
+    const int64_t blocks = (threads + block - 1) / block;
+    // the blocks that start early all find a place (8192 tokens, 6 heads of 64: 5.3 us chained, 5.9 not)
     return launch_chained_if(blocks <= 8 * kChainBlocks, rope_vec_kernel<true>, rope_vec_kernel<false>,
-                             dim3(static_cast<unsigned>(blocks)), dim3(256), 0, stream, YV_BFM(q), YV_BFM(k), cos_t, sin_t,
-                             positions, tokens, hq, hk, head_dim, chunks, 8, inverse, q_stride, k_stride);
+                             dim3(static_cast<unsigned>(blocks)), dim3(block), 0, stream, YV_BFM(q), YV_BFM(k), cos_t, sin_t,
+                             positions, tokens, hq, hk, head_dim, chunks, groups, inverse, q_stride, k_stride);
   }
   const int total = (hq + hk) * (rot_dim >> 1);
   const int block = total >= 256 ? 256 : ((total + 31) / 32) * 32;

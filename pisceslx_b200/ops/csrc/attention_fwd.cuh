@@ -1,7 +1,9 @@
 // Flash attention forward for sm_100a: GQA, causal or full, packed variable-length sequences.
 //
-// One persistent CTA per SM walks (256-query block, query head, sequence) items, heavy blocks first; 384 threads:
-//   warps 0..3  softmax of tile 0, warps 4..7 of tile 1: a thread owns one query row (= TMEM lane): tcgen05.ld the 128 scores,
+// One persistent CTA per SM walks (query block, query head, sequence) items, heavy blocks first.  A block has two tiles of 128
+// queries or one; the key tiles of a lone query tile are dealt out to both halves of the CTA in turn, whose sums are added at
+// the end (the tile is "split").  384 threads:
+//   warps 0..3  softmax of tile 0, warps 4..7 of tile 1 (split: of every other key tile): a thread owns one query row (= TMEM lane): tcgen05.ld the 128 scores,
 //               online softmax with lazy rescaling of the O accumulator, pack P to bf16, tcgen05.st
 //   warp 8      TMA producer: the item's two 128-row Q tiles, then K_j / V_j tiles through rings
 //   warp 9      MMA issuer: per tile S = Q K_j^T (SS), O += P_j V_j (TS: P is read from TMEM where the softmax warps wrote it
@@ -14,6 +16,8 @@
 // Q loads, first scores and epilogue overlap the neighbouring items' work: nothing is allocated or set up per item.
 // Measured, before (one tile per CTA, 2^x on bf16 pairs) and now: 1 x 16384, 32 / 8 heads of 128, causal 2368 -> 1810 us (929 ->
 // 1215 TFLOP/s); 2 x 4096 390 -> 283 us; 4 x 5329, 16 heads of 64, not causal 1036 -> 775 us (449 -> 601 TFLOP/s).
+// A lone tile, one half of the CTA idle and now split (and one tile per CTA): 64 queries of 8192 keys, 32 / 8 heads of 128 110 ->
+// 67 us (86), 16 / 4 of 64 88 -> 56 (84); one after the other, S, softmax and P V of a tile leave nothing to overlap.
 #pragma once
 #include "attention_math.cuh"
 
@@ -28,7 +32,8 @@ struct AttnFwdParams {
   const int* cu_q;     // [B+1]
   const int* cu_k;     // [B+1]
   int hq, hk, batch;
-  int64_t items;       // ceil(max_q / 256) * hq * batch, in descending order of work
+  int two;             // 1: items of two query tiles, 0: of one
+  int64_t items;       // query blocks of the longest sequence times hq * batch, in descending order of work
   int64_t o_stride;    // elements between consecutive tokens of o
   int64_t total_q;
   int causal;
@@ -47,7 +52,7 @@ template <int D>
 struct AttnFwdSmem {
   static constexpr int kTile = kAttnBlock * D * 2;       // bytes of one Q/K/V tile
   static constexpr int kStages = D == 64 ? 3 : 2;
-  static constexpr int kTotal = kTile * (2 + 2 * kStages) + 256 + 1024;
+  static constexpr int kTotal = kTile * (2 + 2 * kStages) + kAttnBlock * 8 + 256 + 1024;
 };
 
 // Item of round r of a CTA.  Every other round runs backwards, so that no CTA gets the heaviest item of each (16 rounds of a
@@ -56,10 +61,12 @@ __device__ __forceinline__ int64_t attn_item_of(int64_t r) {
   return r * gridDim.x + ((r & 1) ? gridDim.x - 1 - blockIdx.x : blockIdx.x);
 }
 
-// One item: 256 queries of one head of one sequence, and how many key tiles each of its two query tiles sees.
+// One item: a block of queries of one head of one sequence, and how many key tiles each half of the CTA works on.
 struct AttnItem {
   int h, q0, q_begin, q_len, k_begin, k_len, shift;
-  int n[2];            // key tiles; a query tile past the sequence's end has none and writes nothing
+  bool second;         // there is a second query tile
+  bool split;          // both halves have the first query tile, and every other key tile of it
+  int n[2];            // key tiles; a query tile that sees none is written as zeros
   __device__ __forceinline__ bool load(const AttnFwdParams& p, int64_t r) {
     const int64_t w = attn_item_of(r);
     if (w >= p.items) return false;
@@ -71,9 +78,11 @@ struct AttnItem {
     q_len = p.cu_q[b + 1] - q_begin;
     k_begin = p.cu_k[b];
     k_len = p.cu_k[b + 1] - k_begin;
-    const int blk = (q_len + 2 * kAttnBlock - 1) / (2 * kAttnBlock) - 1 - rank;   // heavy (late) blocks first
+    const int log_rows = 7 + p.two;
+    const int blk = ((q_len + (1 << log_rows) - 1) >> log_rows) - 1 - rank;       // heavy (late) blocks first
     if (blk < 0) return false;
-    q0 = blk * 2 * kAttnBlock;
+    q0 = blk << log_rows;
+    second = p.two != 0 && q0 + kAttnBlock < q_len;
     // causal: query i (bottom-right aligned when k_len != q_len) sees keys <= i + (k_len - q_len)
     shift = k_len - q_len;
     const int all = (k_len + kAttnBlock - 1) / kAttnBlock;
@@ -85,11 +94,23 @@ struct AttnItem {
         const int lim = last_key / kAttnBlock + 1;
         v = last_key < 0 ? 0 : (lim < all ? lim : all);
       }
-      n[t] = q0 + t * kAttnBlock < q_len ? v : 0;
+      n[t] = t == 0 || second ? v : 0;
+    }
+    split = !second && n[0] > 1;
+    if (split) {
+      n[1] = n[0] / 2;
+      n[0] -= n[1];
     }
     return true;
   }
-  __device__ __forceinline__ int tiles() const { return n[0] > n[1] ? n[0] : n[1]; }
+  __device__ __forceinline__ int count(int t) const { return t == 0 ? n[0] : n[1]; }
+  __device__ __forceinline__ int tiles() const { return split ? n[0] + n[1] : n[0] > n[1] ? n[0] : n[1]; }
+  __device__ __forceinline__ int steps() const { return n[0] > n[1] ? n[0] : n[1]; }
+  // key tile of step j of a half, and first query of its tile
+  __device__ __forceinline__ int key_tile(int t, int j) const { return split ? 2 * j + t : j; }
+  __device__ __forceinline__ int first_query(int t) const { return q0 + (split ? 0 : t * kAttnBlock); }
+  // whether a half's products of step j are the last that read its key tile
+  __device__ __forceinline__ bool last_reader(int t, int j) const { return split || t == 1 || j >= n[1]; }
 };
 
 template <int D>
@@ -118,7 +139,10 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
   uint64_t* k_empty = k_full + kStages;
   uint64_t* v_full = k_empty + kStages;
   uint64_t* v_empty = v_full + kStages;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(v_empty + kStages);
+  uint64_t* ml_full = v_empty + kStages;   // split: the second half's maxima and sums are in ml
+  uint64_t* ml_empty = ml_full + 1;        //        they and its O have been read
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(ml_empty + 1);
+  float2* ml = reinterpret_cast<float2*>(reinterpret_cast<uint8_t*>(bars) + 256);     // [128] per query row
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -140,6 +164,8 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
       mbar_init(&v_full[s], 1);
       mbar_init(&v_empty[s], 1);
     }
+    mbar_init(ml_full, 4);
+    mbar_init(ml_empty, 4);
     fence_barrier_init();
   }
   if (warp == 9) {
@@ -157,13 +183,13 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
     if (elect_one()) {
       bool ok = true;
       uint32_t kv = 0, nq[2] = {0u, 0u};          // key tiles and Q tiles so far
-      AttnItem it;
       for (int64_t r = 0; r * gridDim.x < p.items && ok; ++r) {
+        AttnItem it;
         if (!it.load(p, r)) continue;
         const int hkv = it.h / (p.hq / p.hk);
         const int n = it.tiles();
         for (int t = 0; t < 2 && ok; ++t) {
-          if (it.n[t] == 0) continue;
+          if (it.count(t) == 0) continue;
           ok = mbar_wait(&q_empty[t], (nq[t] & 1u) ^ 1u, p.status);
           if (!ok) break;
           ++nq[t];
@@ -171,7 +197,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
 #pragma unroll
           for (int c = 0; c < kDBoxes; ++c)
             tma_load_3d(sQ + t * S::kTile + c * kBoxBytes, &p.tma_q, &q_full[t], c * 64, it.h,
-                        it.q_begin + it.q0 + t * kAttnBlock);
+                        it.q_begin + it.first_query(t));
         }
         for (int j = 0; j < n && ok; ++j, ++kv) {
           const uint32_t s = kv % kStages, ph = (kv / kStages) & 1u;
@@ -197,14 +223,13 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
     if (elect_one()) {
       bool ok = true;
       uint32_t kv = 0, nq[2] = {0u, 0u}, np[2] = {0u, 0u};   // key tiles, Q tiles and P tiles so far
-      AttnItem it;
       for (int64_t r = 0; r * gridDim.x < p.items && ok; ++r) {
+        AttnItem it;
         if (!it.load(p, r)) continue;
-        const int n = it.tiles();
-        // S_t of key tile j; the products of one thread execute in order, so it follows the P V that read the same columns
+        // S_t of step j; the products of one thread execute in order, so it follows the P V that read the same columns
         auto issue_qk = [&](int t, int j) -> bool {
-          const uint32_t s = (kv + j) % kStages;
-          if (!mbar_wait(&k_full[s], ((kv + j) / kStages) & 1u, p.status)) return false;
+          const uint32_t at = kv + it.key_tile(t, j), s = at % kStages;
+          if (!mbar_wait(&k_full[s], (at / kStages) & 1u, p.status)) return false;
           tc_fence_after_sync();
           const uint32_t aQ = smem_u32(sQ + t * S::kTile), aK = smem_u32(sK + s * S::kTile);
           const uint32_t tS = tmem_base + static_cast<uint32_t>(t * 128);
@@ -215,26 +240,26 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
                           kk != 0 ? 1u : 0u);
           }
           tc_commit(&s_full[t]);
-          if (j + 1 == it.n[t]) tc_commit(&q_empty[t]);
+          if (j + 1 == it.count(t)) tc_commit(&q_empty[t]);
           // the tile is free once the last query tile that sees it has been multiplied
-          if (t == 1 || j >= it.n[1]) tc_commit(&k_empty[s]);
+          if (it.last_reader(t, j)) tc_commit(&k_empty[s]);
           return true;
         };
         for (int t = 0; t < 2 && ok; ++t) {
-          if (it.n[t] == 0) continue;
+          if (it.count(t) == 0) continue;
           ok = mbar_wait(&q_full[t], nq[t] & 1u, p.status);
           if (!ok) break;
           ++nq[t];
           ok = issue_qk(t, 0);
         }
-        for (int j = 0; j < n && ok; ++j) {
-          const uint32_t s = (kv + j) % kStages;
+        for (int j = 0; j < it.steps() && ok; ++j) {
           for (int t = 0; t < 2 && ok; ++t) {
-            if (j >= it.n[t]) continue;
+            if (j >= it.count(t)) continue;
+            const uint32_t at = kv + it.key_tile(t, j), s = at % kStages;
             ok = mbar_wait(&p_full[t], np[t] & 1u, p.status);
             if (!ok) break;
             ++np[t];
-            ok = mbar_wait(&v_full[s], ((kv + j) / kStages) & 1u, p.status);
+            ok = mbar_wait(&v_full[s], (at / kStages) & 1u, p.status);
             if (!ok) break;
             tc_fence_after_sync();
             const uint32_t aV = smem_u32(sV + s * S::kTile);
@@ -246,12 +271,12 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
               tc_mma_f16_ts(tO, tP + kk * 8, make_smem_desc(aV + kk * 2048, kBoxBytes, 1024), kIdescPV,
                             (j | kk) != 0 ? 1u : 0u);
             }
-            if (j + 1 == it.n[t]) tc_commit(&o_full[t]);
-            if (t == 1 || j >= it.n[1]) tc_commit(&v_empty[s]);
-            if (j + 1 < it.n[t]) ok = issue_qk(t, j + 1);
+            if (j + 1 == it.count(t)) tc_commit(&o_full[t]);
+            if (it.last_reader(t, j)) tc_commit(&v_empty[s]);
+            if (j + 1 < it.count(t)) ok = issue_qk(t, j + 1);
           }
         }
-        kv += n;
+        kv += it.tiles();
       }
     }
   } else if (warp < 8) {
@@ -264,12 +289,12 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
     const uint32_t tS = tmem_base + lane_off + static_cast<uint32_t>(t * 128);
     const uint32_t tO = tmem_base + lane_off + kOCol + static_cast<uint32_t>(t * 128);
     bool ok = true;
-    uint32_t ns = 0, no = 0;                          // score tiles and finished items so far
-    AttnItem it;
+    uint32_t ns = 0, no0 = 0, no1 = 0, nx = 0;        // score tiles, finished items of either half and split items so far
     for (int64_t r = 0; r * gridDim.x < p.items && ok; ++r) {
+      AttnItem it;
       if (!it.load(p, r)) continue;
-      const int n_kv = it.n[t];
-      const int q_pos = it.q0 + t * kAttnBlock + row; // position inside the sequence
+      const int n_kv = it.count(t);
+      const int q_pos = it.first_query(t) + row;      // position inside the sequence
       const int key_limit = p.causal ? min(q_pos + it.shift, it.k_len - 1) : (it.k_len - 1);   // last visible key
       float m_used = -1.0e29f;                        // running max (log2 domain); above kMaskValue so masked scores give 0
       float l_sum = 0.f;
@@ -292,7 +317,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
         }
         // The row maximum is taken over the raw scores (the scale is positive); scaling and the subtraction of the
         // reference maximum are one fused multiply-add per pair of scores further down.
-        const int last = key_limit - j * kAttnBlock;  // last visible column of this tile
+        const int last = key_limit - it.key_tile(t, j) * kAttnBlock;  // last visible column of this tile
         if (last < kAttnBlock - 1) {
 #pragma unroll
           for (int i = 0; i < 128; ++i)
@@ -318,7 +343,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
         }
         if (__any_sync(0xFFFFFFFFu, rescale)) {
           // O holds sums relative to the old max; the products that wrote it precede the scores just read
-#pragma unroll
+#pragma unroll 1
           for (int c = 0; c < D / 32; ++c) {
             uint32_t ov[32];
             tmem_ld32(tO + c * 32, ov);
@@ -354,18 +379,52 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
         l_sum = l_sum * alpha + (rs.x + rs.y);
       }
       // ---- epilogue: O / l, LSE ----
+      const uint32_t done0 = no0 & 1u, done1 = no1 & 1u, turn = nx & 1u;
+      no0 += it.n[0] > 0 ? 1u : 0u;
+      no1 += it.n[1] > 0 ? 1u : 0u;
+      if (it.split) {
+        ++nx;
+        if (t == 1) {
+          // hand this half's maxima and sums over; its O stays where it is until it has been read
+          if (ok) {
+            ml[row] = make_float2(m_used, l_sum);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(ml_full);
+            ok = mbar_wait(ml_empty, turn, p.status);
+            ok = __all_sync(0xFFFFFFFFu, ok);
+            tc_fence_after_sync();
+          }
+          continue;
+        }
+        if (ok) {
+          // in this order: once the second half has handed over, its earlier items' products are known to have landed, so that
+          // the phase that is waited for next is this item's
+          ok = mbar_wait(ml_full, turn, p.status) && mbar_wait(&o_full[1], done1, p.status);
+          ok = __all_sync(0xFFFFFFFFu, ok);
+        }
+      }
       if (ok && n_kv > 0) {
-        ok = mbar_wait(&o_full[t], no & 1u, p.status);
+        ok = mbar_wait(&o_full[t], t == 0 ? done0 : done1, p.status);
         ok = __all_sync(0xFFFFFFFFu, ok);
-        ++no;
       }
       if (ok) {
         tc_fence_after_sync();
-        const bool valid = q_pos < it.q_len;
+        float f0 = 1.f, f1 = 0.f;                     // factors of the halves' sums
+        if (it.split) {
+          const float2 other = ml[row];
+          const float m = max_nan(m_used, other.x);
+          f0 = exp2f(m_used - m);
+          f1 = exp2f(other.x - m);
+          m_used = m;
+          l_sum = l_sum * f0 + other.y * f1;
+        }
+        const bool valid = q_pos < it.q_len && (t == 0 || it.second);
         const float inv_l = (l_sum > 0.f) ? 1.f / l_sum : 0.f;
+        f0 *= inv_l;
+        f1 *= inv_l;
         __nv_bfloat16* orow = p.o + (static_cast<int64_t>(it.q_begin + q_pos) * p.o_stride) + static_cast<int64_t>(it.h) * D;
-#pragma unroll
-        for (int c = 0; c < D / 32; ++c) {
+#pragma unroll 1
+        for (int c = 0; c < D / 32; ++c) {             // a loop, since short items run it once each: the code has to stay small
           uint32_t ov[32];
           if (n_kv > 0) {
             tmem_ld32(tO + c * 32, ov);
@@ -374,19 +433,34 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
 #pragma unroll
             for (int i = 0; i < 32; ++i) ov[i] = 0u;
           }
+          if (it.split) {
+            uint32_t o1[32];
+            tmem_ld32(tO + 128 + c * 32, o1);
+            tc_wait_ld();
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+              ov[i] = __float_as_uint(__uint_as_float(ov[i]) * f0 + __uint_as_float(o1[i]) * f1);
+          } else {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * f0);
+          }
           if (valid) {
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
               uint4 v;
-              v.x = pack_bf16(__uint_as_float(ov[8 * i + 0]) * inv_l, __uint_as_float(ov[8 * i + 1]) * inv_l);
-              v.y = pack_bf16(__uint_as_float(ov[8 * i + 2]) * inv_l, __uint_as_float(ov[8 * i + 3]) * inv_l);
-              v.z = pack_bf16(__uint_as_float(ov[8 * i + 4]) * inv_l, __uint_as_float(ov[8 * i + 5]) * inv_l);
-              v.w = pack_bf16(__uint_as_float(ov[8 * i + 6]) * inv_l, __uint_as_float(ov[8 * i + 7]) * inv_l);
+              v.x = pack_bf16(__uint_as_float(ov[8 * i + 0]), __uint_as_float(ov[8 * i + 1]));
+              v.y = pack_bf16(__uint_as_float(ov[8 * i + 2]), __uint_as_float(ov[8 * i + 3]));
+              v.z = pack_bf16(__uint_as_float(ov[8 * i + 4]), __uint_as_float(ov[8 * i + 5]));
+              v.w = pack_bf16(__uint_as_float(ov[8 * i + 6]), __uint_as_float(ov[8 * i + 7]));
               *reinterpret_cast<uint4*>(orow + c * 32 + i * 8) = v;
             }
           }
         }
         tc_fence_before_sync();                       // O is read before the next item's first P is announced
+        if (it.split) {
+          __syncwarp();
+          if (lane == 0) mbar_arrive(ml_empty);
+        }
         if (valid && p.lse != nullptr) {
           // natural-log LSE of the scaled scores
           p.lse[static_cast<int64_t>(it.h) * p.total_q + it.q_begin + q_pos] =

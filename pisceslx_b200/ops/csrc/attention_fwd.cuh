@@ -3,8 +3,8 @@
 // One persistent CTA per SM walks (query block, query head, sequence) items, heavy blocks first.  A block has two tiles of 128
 // queries or one; the key tiles of a lone query tile are dealt out to both halves of the CTA in turn, whose sums are added at
 // the end (the tile is "split").  384 threads:
-//   warps 0..3  softmax of tile 0, warps 4..7 of tile 1 (split: of every other key tile): a thread owns one query row (= TMEM lane): tcgen05.ld the 128 scores,
-//               online softmax with lazy rescaling of the O accumulator, pack P to bf16, tcgen05.st
+//   warps 0..3  softmax of tile 0, warps 4..7 of tile 1 (split: of every other key tile): a thread owns one query row (= TMEM
+//               lane): tcgen05.ld the 128 scores, online softmax with lazy rescaling of the O accumulator, pack P to bf16, tcgen05.st
 //   warp 8      TMA producer: the item's two 128-row Q tiles, then K_j / V_j tiles through rings
 //   warp 9      MMA issuer: per tile S = Q K_j^T (SS), O += P_j V_j (TS: P is read from TMEM where the softmax warps wrote it
 //               over S); the two tiles take turns, so the tensor core works on one while the other is in softmax

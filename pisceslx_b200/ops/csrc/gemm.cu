@@ -168,28 +168,28 @@ int launch_gemm(const GemmArgs& a, cudaStream_t stream) {
     if ((a.mode != kDense && !mx) || a.a_mn || a.b_mn || a.out_fp32 || a.accumulate || a.comm != 0) return -70;
     r = make_tmap_2d(&p.tma_a, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a.a, a_inner, a_outer, lda, 128, kBM);
     if (r != 0) return -20 + r;
-    r = make_tmap_2d(&p.tma_b, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a.b, b_inner, b_outer, ldb, 128,
-                     static_cast<uint32_t>(bn));
+    r = make_tmap_2d(&p.tma_b, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a.b, b_inner, b_outer, ldb, 128, 128);
     if (r != 0) return -30 + r;
   } else {
     r = make_tmap_2d(&p.tma_a, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, a.a, a_inner, a_outer, lda, 64,
                      a.a_mn ? kBK : kBM);
     if (r != 0) return -20 + r;
     r = make_tmap_2d(&p.tma_b, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, a.b, b_inner, b_outer, ldb, 64,
-                     a.b_mn ? kBK : static_cast<uint32_t>(bn));
+                     a.b_mn ? kBK : 128);
     if (r != 0) return -30 + r;
   }
   r = make_tmap_2d(&p.tma_c, a.out_fp32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16,
                    out_bytes, a.c, static_cast<uint64_t>(a.N), c_outer, ldc, 128 / out_bytes, kBM);
   if (r != 0) return -40 + r;
 
-  p.symmetric = 0; p.sym_tiles = 0; p.sym_c = nullptr;
+  p.symmetric = 0; p.sym_tiles = 0;
   if (a.symmetric) {
     if (a.mode != kBatched || a.M != a.N || a.out_fp32 || a.accumulate || a.comm != 0 || a.fp8 ||
         (a.ldc != 0 && a.ldc != a.N))
       return -81;
     p.symmetric = 1;
-    p.sym_c = reinterpret_cast<__nv_bfloat16*>(a.c);
+    r = make_tmap_2d(&p.tma_ct, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, a.c, static_cast<uint64_t>(a.N), c_outer, ldc, 64, 64);
+    if (r != 0) return -40 + r;
     const int tm = (a.M + kBM - 1) / kBM, tn = (a.N + bn - 1) / bn;
     for (int j = 0; j < tn; ++j) p.sym_tiles += (tm < (j + 1) * (bn / kBM)) ? tm : (j + 1) * (bn / kBM);
   }

@@ -68,11 +68,12 @@ struct GemmParams {
   // epi_cin laid out like C; the identity is per group in the batched mode ----
   const __nv_bfloat16* epi_cin;
   float epi_a, epi_b, epi_c;
-  // ---- symmetric output (batched mode, M == N, bf16): tiles entirely below the diagonal are skipped and filled by
-  // the mirrored stores of the computed tiles; sym_tiles = computed tiles per group, sym_c = C as a plain pointer ----
+  // ---- symmetric output (batched mode, M == N, bf16): of the 128 x 128 blocks only those on or above the diagonal are
+  // computed; the epilogue also stores each block above it transposed, through tma_ct (C in boxes of 64 x 64).  sym_tiles =
+  // computed tiles per group ----
   int symmetric;
   int sym_tiles;
-  __nv_bfloat16* sym_c;
+  CUtensorMap tma_ct;
 };
 
 constexpr int kBM = 128;
@@ -99,16 +100,22 @@ struct TileCoord {
   int a_x, a_y;      // TMA coordinates of the first A box (x = inner)
   int b_x, b_y;
   int c_x, c_y;
+  int width;         // columns of the tile that are computed: BN, or half of it (see decode_tile)
   int k_iters;
   int m_blk;         // 128-row block of A / C this tile covers
 };
 
 // Decode linear tile index -> coordinates.  Returns false when idx is past the end.
+//
+// A 256-wide tile of which only one 128-wide half is wanted (the last columns of N = 1408, or a symmetric product's block
+// below the diagonal) runs products half as wide: 64 problems of 1408 x 1408 count 33 full tiles each instead of 41.
 template <int BN, bool A_MN, bool B_MN, int COMM = 0, int FP8 = 0>
 __device__ __forceinline__ bool decode_tile(const GemmParams& p, int idx, int tiles_m, int tiles_n, TileCoord& t) {
   int m_blk, n_blk, group = 0;
+  int n_skip = 0;                                    // leading 128-column blocks of the tile that are left out
   if (p.mode == kBatched && p.symmetric) {
-    // column tile j keeps the row tiles that start above the column tile's last column: i * 128 < (j + 1) * BN
+    // column tile j keeps the row tiles that start above the column tile's last column: i * 128 < (j + 1) * BN.  The last of
+    // them lies below the diagonal in its first 128 columns
     group = idx / p.sym_tiles;
     if (group >= p.num_groups) return false;
     int r = idx - group * p.sym_tiles;
@@ -120,6 +127,7 @@ __device__ __forceinline__ bool decode_tile(const GemmParams& p, int idx, int ti
     }
     n_blk = j;
     m_blk = r;
+    n_skip = r * kBM > j * BN ? 1 : 0;
   } else if (p.mode == kGroupedK || p.mode == kBatched) {
     const int per_group = tiles_m * tiles_n;
     group = idx / per_group;
@@ -143,7 +151,7 @@ __device__ __forceinline__ bool decode_tile(const GemmParams& p, int idx, int ti
   }
   // grouped-M problems may list their 128-row tiles explicitly (receive regions of several sources)
   const int row_tile = (p.mode == kGroupedM && p.tile_rows != nullptr) ? p.tile_rows[m_blk] : m_blk;
-  const int m0 = row_tile * kBM, n0 = n_blk * BN;
+  const int m0 = row_tile * kBM, n0 = n_blk * BN + n_skip * 128;
   const int m0_a = (p.mode == kGroupedM && p.tile_rows_c_only) ? m_blk * kBM : m0;
   int k_begin = 0, k_len = p.K;
   int a_outer_off = 0, b_outer_off = 0, c_row_off = 0;
@@ -160,6 +168,7 @@ __device__ __forceinline__ bool decode_tile(const GemmParams& p, int idx, int ti
     c_row_off = group * p.c_group_stride;
   }
   constexpr int kBKe = FP8 ? 2 * kBK : kBK;          // elements of K per pipeline stage (128 bytes per row)
+  t.width = (FP8 == 0 && BN == 256 && (n_skip != 0 || p.N - n0 <= 128)) ? 128 : BN;
   t.k_iters = (k_len + kBKe - 1) / kBKe;
   if (A_MN) { t.a_x = m0_a; t.a_y = a_outer_off + k_begin; } else { t.a_x = k_begin; t.a_y = a_outer_off + m0_a; }
   if (B_MN) { t.b_x = n0; t.b_y = b_outer_off + k_begin; } else { t.b_x = k_begin; t.b_y = b_outer_off + n0; }
@@ -186,6 +195,7 @@ __global__ void __launch_bounds__(kGemmThreadsAllGather, 1) gemm_sm100_kernel(co
   constexpr int kBKe = FP8 ? 2 * kBK : kBK;
   constexpr uint32_t kIdesc = MX ? make_idesc_mxf8(kBM, BN)
                                  : (FP8 ? make_idesc_e4m3(kBM, BN) : make_idesc_bf16(kBM, BN, A_MN, B_MN));
+  constexpr uint32_t kIdescHalf = make_idesc_bf16(kBM, 128, A_MN, B_MN);    // 128 columns of a 256-wide tile
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -276,7 +286,7 @@ __global__ void __launch_bounds__(kGemmThreadsAllGather, 1) gemm_sm100_kernel(co
               bulk_load_1d(ssf + 512 * (1 + j), p.sfb + (static_cast<int64_t>(b_tile + j) * p.sf_kchunks + k) * 512, 512,
                            &full_bar[s]);
           } else {
-            mbar_expect_tx(&full_bar[s], S::kStageBytes);
+            mbar_expect_tx(&full_bar[s], S::kABytes + static_cast<uint32_t>(t.width) * (kBK * 2));
           }
           if (A_MN) {
 #pragma unroll
@@ -288,9 +298,13 @@ __global__ void __launch_bounds__(kGemmThreadsAllGather, 1) gemm_sm100_kernel(co
           if (B_MN) {
 #pragma unroll
             for (int j = 0; j < BN / 64; ++j)
-              tma_load_2d(sb + j * (kBK * 128), &p.tma_b, &full_bar[s], t.b_x + j * 64, t.b_y + k * kBK);
+              if (j * 64 < t.width)
+                tma_load_2d(sb + j * (kBK * 128), &p.tma_b, &full_bar[s], t.b_x + j * 64, t.b_y + k * kBK);
           } else {
-            tma_load_2d(sb, &p.tma_b, &full_bar[s], t.b_x + k * kBKe, t.b_y);
+#pragma unroll
+            for (int j = 0; j < BN / 128; ++j)
+              if (j * 128 < t.width)
+                tma_load_2d(sb + j * (128 * 128), &p.tma_b, &full_bar[s], t.b_x + k * kBKe, t.b_y + j * 128);
           }
         }
       }
@@ -309,6 +323,7 @@ __global__ void __launch_bounds__(kGemmThreadsAllGather, 1) gemm_sm100_kernel(co
         if (!ok) break;
         tc_fence_after_sync();
         const uint32_t tmem_d = tmem_base + static_cast<uint32_t>(acc * BN);
+        const uint32_t idesc = t.width == BN ? kIdesc : kIdescHalf;
         for (int k = 0; k < t.k_iters && ok; ++k, ++it) {
           const int s = it % kStages;
           const uint32_t ph = (it / kStages) & 1u;
@@ -337,7 +352,7 @@ __global__ void __launch_bounds__(kGemmThreadsAllGather, 1) gemm_sm100_kernel(co
             } else if (FP8) {
               tc_mma_f8_ss(tmem_d, da, db, kIdesc, (k | kk) != 0 ? 1u : 0u);
             } else {
-              tc_mma_f16_ss(tmem_d, da, db, kIdesc, (k | kk) != 0 ? 1u : 0u);
+              tc_mma_f16_ss(tmem_d, da, db, idesc, (k | kk) != 0 ? 1u : 0u);
             }
           }
           tc_commit(&empty_bar[s]);     // releases the stage once these MMAs have read it
@@ -413,13 +428,35 @@ __global__ void __launch_bounds__(kGemmThreadsAllGather, 1) gemm_sm100_kernel(co
     const int quarter = warp & 3;                      // TMEM lane quarter this warp may access
     const int row = quarter * 32 + lane;               // row of the tile owned by this thread
     const bool issuer = (threadIdx.x == 64);           // first epilogue thread issues the TMA stores
-    uint32_t tile_it = 0, chunk_it = 0;
+    uint32_t tile_it = 0, buf_it = 0;
     bool ok = true;
+    // The next staging buffer, once the store that last used it (two stores ago) has finished reading it.
+    auto next_buffer = [&]() -> uint8_t* {
+      uint8_t* buf = smem_epi + (buf_it++ & 1) * S::kEpiBytes;
+      if (issuer) tma_store_wait_read<1>();
+      asm volatile("bar.sync 1, 128;" ::: "memory");
+      return buf;
+    };
+    // this thread's row of the affine epilogue's Cin in one chunk of columns (zeros past N); fetched a chunk ahead, the first
+    // one while the products still run
+    constexpr bool kAffine = !FP8 && COMM == 0 && sizeof(OutT) == 2;
+    uint4 cin[8];
+    auto load_cin = [&](const TileCoord& t, int c) {
+      const int col0 = t.c_x + c * kColsPerChunk;
+      const bool in = c * kColsPerChunk < t.width && col0 + kColsPerChunk <= p.N;
+      const uint4* src = reinterpret_cast<const uint4*>(p.epi_cin + static_cast<int64_t>(t.c_y + row) * p.N + col0);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) cin[j] = in ? src[j] : make_uint4(0u, 0u, 0u, 0u);
+    };
     for (int idx = blockIdx.x; ok; idx += gridDim.x, ++tile_it) {
       TileCoord t;
       if (!decode_tile<BN, A_MN, B_MN, COMM, FP8>(p, idx, tiles_m, tiles_n, t)) break;
       const int acc = tile_it % kAccBufs;
       const uint32_t acc_ph = (tile_it / kAccBufs) & 1u;
+      const bool affine = kAffine && p.epi_cin != nullptr;
+      if (affine) load_cin(t, 0);
+      // row of the tile inside its matrix
+      const int lrow0 = p.c_group_stride > 0 ? t.c_y % p.c_group_stride : t.c_y;
       ok = mbar_wait(&acc_full[acc], acc_ph, p.status);
       // all 128 epilogue threads must take the same branch: barrier with an AND reduction
       {
@@ -452,11 +489,9 @@ __global__ void __launch_bounds__(kGemmThreadsAllGather, 1) gemm_sm100_kernel(co
                       (static_cast<int64_t>(p.comm_rank) * rows_per_rank + in_row0) * p.comm_row_bytes;
       }
 #pragma unroll 1
-      for (int c = 0; c < kChunks; ++c, ++chunk_it) {
-        uint8_t* buf = smem_epi + (chunk_it & 1) * S::kEpiBytes;
-        // the store that last used this buffer (two chunks ago) must have finished reading it
-        if (issuer) tma_store_wait_read<1>();
-        asm volatile("bar.sync 1, 128;" ::: "memory");
+      for (int c = 0; c < kChunks; ++c) {
+        if (c * kColsPerChunk >= t.width) break;
+        uint8_t* buf = next_buffer();
         uint32_t packed[32];
         if (sizeof(OutT) == 2) {
           uint32_t v0[32], v1[32];
@@ -469,17 +504,12 @@ __global__ void __launch_bounds__(kGemmThreadsAllGather, 1) gemm_sm100_kernel(co
             for (int i = 0; i < 32; ++i) { v0[i] = 0u; v1[i] = 0u; }
           }
           const float osc = (FP8 == 1 && p.out_scale != nullptr) ? *p.out_scale : 1.f;
-          if (!FP8 && COMM == 0 && p.epi_cin != nullptr) {
+          if (affine) {
             // out = epi_c * acc + epi_b * Cin + epi_a * I: the Newton-Schulz polynomial b A + c A^2 (+ a I) formed in
             // the epilogue of the A * A product, Cin = A in the layout of C (N a multiple of 64)
             const int col0 = t.c_x + c * kColsPerChunk;
-            const bool in = col0 + kColsPerChunk <= p.N;
-            const uint4* src = reinterpret_cast<const uint4*>(p.epi_cin + static_cast<int64_t>(t.c_y + row) * p.N + col0);
-            uint4 cin[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) cin[j] = in ? src[j] : make_uint4(0u, 0u, 0u, 0u);
             const __nv_bfloat16* cb = reinterpret_cast<const __nv_bfloat16*>(cin);
-            const int lrow = (p.c_group_stride > 0 ? t.c_y % p.c_group_stride : t.c_y) + row;
+            const int lrow = lrow0 + row;
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
               const int ca = col0 + 2 * i, cbk = col0 + 32 + 2 * i;
@@ -490,6 +520,7 @@ __global__ void __launch_bounds__(kGemmThreadsAllGather, 1) gemm_sm100_kernel(co
               packed[i] = pack_bf16(a0, a1);
               packed[16 + i] = pack_bf16(b0, b1);
             }
+            load_cin(t, c + 1);
           } else {
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
@@ -504,30 +535,6 @@ __global__ void __launch_bounds__(kGemmThreadsAllGather, 1) gemm_sm100_kernel(co
           } else {
 #pragma unroll
             for (int i = 0; i < 32; ++i) packed[i] = 0u;
-          }
-        }
-        if (sizeof(OutT) == 2 && COMM == 0 && !FP8 && p.symmetric) {
-          // mirrored elements C[col][row] = C[row][col] for the positions whose own tile was skipped.  For a fixed
-          // column the 32 lanes of a warp hold 32 consecutive rows: every store instruction writes 64 contiguous bytes.
-          const int grp_rows = p.c_group_stride;
-          const int lrow = t.c_y % grp_rows + row;                       // row inside the matrix
-          __nv_bfloat16* cbase = p.sym_c + static_cast<int64_t>(t.c_y - t.c_y % grp_rows) * p.N;
-          const int row_tile_end = (lrow / BN + 1) * BN;                 // end of the column tile that holds `lrow` as a column
-          const int col0 = t.c_x + c * kColsPerChunk;
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            // packed[i] (i < 16) holds columns 2i, 2i+1 of the chunk; packed[16 + i] holds columns 32 + 2i, 33 + 2i
-            const int cc = col0 + (i < 16 ? 2 * i : 32 + 2 * (i - 16));
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              const int gcol = cc + h;
-              // the mirror position (gcol, lrow) lies in row tile gcol / 128 and column tile lrow / BN: skipped iff
-              // that column tile ends at or before the row tile starts
-              if (gcol < p.N && row_tile_end <= (gcol / kBM) * kBM && lrow < p.N) {
-                const uint16_t bits = static_cast<uint16_t>(h == 0 ? (packed[i] & 0xffffu) : (packed[i] >> 16));
-                reinterpret_cast<uint16_t*>(cbase)[static_cast<int64_t>(gcol) * p.N + lrow] = bits;
-              }
-            }
           }
         }
         // 128-byte row, eight 16-byte pieces, XOR-swizzled with the row index (TMA SWIZZLE_128B)
@@ -559,6 +566,32 @@ __global__ void __launch_bounds__(kGemmThreadsAllGather, 1) gemm_sm100_kernel(co
             tma_store_2d(&p.tma_c, buf, t.c_x + c * kColsPerChunk, t.c_y);
           }
           tma_store_commit();
+        }
+        const int col_first = t.c_x + c * kColsPerChunk;
+        if (kAffine && p.symmetric && col_first - lrow0 >= kBM) {
+          // A block above the diagonal is also stored transposed, as two boxes of 64 rows (= columns of the chunk) by 64.  A
+          // warp's 32 rows are 32 consecutive two-byte elements of a staged row: no bank conflicts, and what leaves are whole
+          // 128-byte rows.  (Written straight to memory, two bytes a thread, the epilogue of 64 products of 1408^3 took
+          // 19 us a tile, twice as long as the products.)
+          uint8_t* tb = next_buffer() + (row >> 6) * (S::kEpiBytes / 2) + (row & 7) * 2;
+          const int piece = (row & 63) >> 3;
+#pragma unroll
+          for (int i = 0; i < 32; ++i) {
+            // packed[i] (i < 16) holds columns 2i, 2i+1 of the chunk; packed[16 + i] holds columns 32 + 2i, 33 + 2i
+            const int cc = i < 16 ? 2 * i : 32 + 2 * (i - 16);
+            *reinterpret_cast<uint16_t*>(tb + cc * 128 + ((piece ^ (cc & 7)) << 4)) = static_cast<uint16_t>(packed[i] & 0xffffu);
+            *reinterpret_cast<uint16_t*>(tb + (cc + 1) * 128 + ((piece ^ ((cc + 1) & 7)) << 4)) =
+                static_cast<uint16_t>(packed[i] >> 16);
+          }
+          fence_proxy_async_smem();
+          asm volatile("bar.sync 1, 128;" ::: "memory");
+          if (issuer) {
+            const uint8_t* boxes = smem_epi + ((buf_it - 1) & 1) * S::kEpiBytes;
+            const int y = t.c_y - lrow0 + col_first;
+            tma_store_2d(&p.tma_ct, boxes, lrow0, y);
+            tma_store_2d(&p.tma_ct, boxes + S::kEpiBytes / 2, lrow0 + 64, y);
+            tma_store_commit();
+          }
         }
       }
       // all TMEM reads of this accumulator are done: hand it back to the MMA warp

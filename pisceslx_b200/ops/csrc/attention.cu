@@ -1,6 +1,7 @@
 // Host launchers for the attention kernels: tensor-map construction, grid sizing, template dispatch.
 #include "per_device.h"
 #include "attention_bwd.cuh"
+#include "attention_bwd_fused.cuh"
 #include "attention_decode.cuh"
 #include "attention_decode_mma.cuh"
 #include "attention_decode_tma.cuh"
@@ -80,6 +81,47 @@ int launch_attn_fwd(const AttnArgs& a, cudaStream_t stream) {
   return static_cast<int>(cudaGetLastError());
 }
 
+namespace {
+// As many KV heads per launch as the caller's sums have room for.
+template <int D>
+int launch_attn_bwd_fused(const AttnBwdArgs& b, const AttnBwdParams& p, cudaStream_t stream) {
+  using S = AttnBwdFusedSmem<D>;
+  const AttnArgs& a = b.f;
+  static PerDeviceInt cfg;
+  if (!cfg.cur()) {
+    const int r = set_smem(attn_bwd_fused_kernel<D>, S::kTotal);
+    if (r != 0) return r;
+    cfg.cur() = 1;
+  }
+  if (b.dq_acc_kv_heads <= 0 || b.stats == nullptr) return -4;
+  // the tensor maps have seen to 16-byte alignment of dO
+  const unsigned grid_s = static_cast<unsigned>((a.total_q * a.hq * (D / 8) + 255) / 256);
+  const bool vec = (reinterpret_cast<uintptr_t>(a.o) & 15u) == 0 && (a.o_stride & 7) == 0;
+  (vec ? attn_stats_kernel<D, true> : attn_stats_kernel<D, false>)<<<grid_s, 256, 0, stream>>>(
+      reinterpret_cast<const __nv_bfloat16*>(a.o), reinterpret_cast<const __nv_bfloat16*>(b.dout), a.lse,
+      reinterpret_cast<uint4*>(b.stats), a.total_q, a.hq, a.o_stride, b.do_stride, 1.f / a.scale);
+  const int G = a.hq / a.hk;
+  AttnBwdFusedParams fp;
+  fp.b = p;
+  fp.dq_acc = b.dq_acc;
+  fp.stats = reinterpret_cast<const uint4*>(b.stats);
+  for (int h0 = 0; h0 < a.hk; h0 += b.dq_acc_kv_heads) {
+    const int n = a.hk - h0 < b.dq_acc_kv_heads ? a.hk - h0 : b.dq_acc_kv_heads;
+    const int r = static_cast<int>(cudaMemsetAsync(b.dq_acc, 0, static_cast<size_t>(n) * G * D * a.total_q * 4, stream));
+    if (r != 0) return r;
+    fp.hk0 = h0;
+    fp.heads = n;
+    fp.batch = a.batch;
+    fp.blocks = (a.max_k + 127) / 128;
+    const int64_t grid = static_cast<int64_t>(fp.blocks) * n * a.batch;
+    if (grid > 0) attn_bwd_fused_kernel<D><<<static_cast<unsigned>(grid), kFusedThreads, S::kTotal, stream>>>(fp);
+    attn_dq_finish_kernel<D><<<dim3(static_cast<unsigned>((a.total_q + 31) / 32), n * G), 256, 0, stream>>>(
+        reinterpret_cast<const float4*>(b.dq_acc), p.dq, a.total_q, p.dq_stride, h0 * G, p.scale);
+  }
+  return static_cast<int>(cudaGetLastError());
+}
+}  // namespace
+
 int launch_attn_bwd(const AttnBwdArgs& b, cudaStream_t stream) {
   const AttnArgs& a = b.f;
   if (a.batch <= 0 || a.total_q <= 0) return 0;
@@ -109,6 +151,10 @@ int launch_attn_bwd(const AttnBwdArgs& b, cudaStream_t stream) {
   p.scale = a.scale;
   p.scale_log2 = a.scale * kLog2eHost;
   p.status = a.status;
+
+  // The statistics enter the one-pass kernel divided by the scale.
+  if (b.dq_acc != nullptr && fabsf(a.scale) > 1e-20f)
+    return a.d == 128 ? launch_attn_bwd_fused<128>(b, p, stream) : launch_attn_bwd_fused<64>(b, p, stream);
 
   // the tensor maps have seen to 16-byte alignment of dO
   const int64_t lanes = a.total_q * a.hq * (a.d / 8);

@@ -1,4 +1,6 @@
-// Flash attention backward for sm_100a, as two tcgen05 kernels that recompute the probabilities from
+// Flash attention backward for sm_100a with one writer for every row, for callers that ask torch for deterministic algorithms (and
+// for softmax scales that are next to nothing); attention_bwd_fused.cuh is the faster form, whose sums of dq have no fixed order.
+// Two tcgen05 kernels that recompute the probabilities from
 // the saved log-sum-exp (natural log of the scaled scores) and delta = rowsum(dO * O):
 //
 //   attn_bwd_dq_kernel   one CTA per (128-query block, query head, sequence), loops over key blocks:

@@ -314,16 +314,11 @@ __global__ void __launch_bounds__(kAttnBwdThreads, 1) attn_bwd_dkv_kernel(const 
 // reads 512 contiguous bytes twice.  Bound by memory:
 // 16384 tokens of 32 heads of 128 in 48 us (5.5 TB/s) instead of 107 with one warp and 4-byte loads per head.  O that is not aligned to 16 bytes is read in pairs.
 template <int D, bool VEC>
-__global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __restrict__ o,
-                                                         const __nv_bfloat16* __restrict__ dout, float* __restrict__ delta,
-                                                         int64_t total_q, int hq, int64_t o_stride, int64_t do_stride) {
+__device__ __forceinline__ float attn_delta_row(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ dout,
+                                                int64_t t, int h, int c, bool valid, int64_t o_stride, int64_t do_stride) {
   constexpr int kLanes = D / 8;
-  const int64_t w = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) / kLanes;
-  const int c = threadIdx.x & (kLanes - 1);
-  const int64_t t = w / hq;
-  const int h = static_cast<int>(w - t * hq);
   float s = 0.f;
-  if (t < total_q) {
+  if (valid) {
     const __nv_bfloat16* orow = o + t * o_stride + static_cast<int64_t>(h) * D + c * 8;
     uint4 a;
     if (VEC) {
@@ -342,6 +337,19 @@ __global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __
   }
 #pragma unroll
   for (int off = kLanes / 2; off > 0; off >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, off);
+  return s;
+}
+
+template <int D, bool VEC>
+__global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __restrict__ o,
+                                                         const __nv_bfloat16* __restrict__ dout, float* __restrict__ delta,
+                                                         int64_t total_q, int hq, int64_t o_stride, int64_t do_stride) {
+  constexpr int kLanes = D / 8;
+  const int64_t w = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) / kLanes;
+  const int c = threadIdx.x & (kLanes - 1);
+  const int64_t t = w / hq;
+  const int h = static_cast<int>(w - t * hq);
+  const float s = attn_delta_row<D, VEC>(o, dout, t, h, c, t < total_q, o_stride, do_stride);
   if (c == 0 && t < total_q) delta[static_cast<int64_t>(h) * total_q + t] = s;
 }
 

@@ -216,6 +216,10 @@ struct AttnBwdArgs {
   void* dk = nullptr;          // bf16 [Tk, hk, d]
   void* dv = nullptr;          // bf16 [Tk, hk, d]
   float* delta = nullptr;      // fp32 [hq, Tq] scratch
+  // sums of dq, fp32 [KV heads at a time, hq / hk, d, Tq] in any order of their own; without them two kernels without atomics run
+  float* dq_acc = nullptr;
+  void* stats = nullptr;       // 16 bytes per (query head, token), with dq_acc
+  int dq_acc_kv_heads = 0;
   int64_t do_stride = 0, dq_stride = 0, dk_stride = 0, dv_stride = 0;
 };
 int launch_attn_bwd(const AttnBwdArgs& a, cudaStream_t stream);

@@ -325,6 +325,43 @@ def test_flash_attention_fwd_bwd(status, lens, hq, hk, d, causal):
     assert e1 < 6e-3 and e2 < 6e-3 and eg < 1.2e-2
 
 
+@pytest.mark.parametrize("lq,lk,hq,hk,d,causal", [
+    ([1, 127, 128, 129], [1, 127, 128, 129], 4, 2, 64, True),       # edges of the key and query blocks
+    ([1, 127, 128, 129], [1, 127, 128, 129], 4, 2, 128, True),
+    ([5, 130, 300, 255], [200, 64, 100, 257], 4, 4, 64, True),      # more queries than keys: queries without a key, and the other way
+    ([5, 130, 300, 255], [200, 64, 100, 257], 4, 1, 128, True),
+    ([385, 640], [511, 3], 8, 2, 64, False), ([385, 640], [511, 3], 8, 2, 128, False),
+    ([1900], [1900], 8, 1, 64, True), ([1900], [1900], 4, 1, 128, False),   # many blocks: every stage of the loop comes round
+    ([1000] * 70, [1000] * 70, 16, 2, 128, True)])                  # sums of dq above 512 MB: a KV head at a time
+def test_attention_backward_against_one_writer_per_row(status, lq, lk, hq, hk, d, causal):
+    """The one-pass backward against the two kernels that deterministic algorithms select, which repeat their bits, and against
+    fp32.  Both round P and dS to bf16 (2^-9 relative, about 1e-3 of a sum's norm each way)."""
+    from pisceslx_b200.ops import functional as F_, reference as ref
+    torch.manual_seed(13)
+    cu = lambda l: torch.tensor([0] + list(torch.tensor(l).cumsum(0)), dtype=torch.int32, device=DEV)
+    mk = lambda n, h: torch.randn(n, h * d, device=DEV, dtype=torch.bfloat16).requires_grad_(True)
+    cq, ck, (q, k, v) = cu(lq), cu(lk), (mk(sum(lq), hq), mk(sum(lk), hk), mk(sum(lk), hk))
+    do = torch.randn(sum(lq), hq * d, device=DEV, dtype=torch.bfloat16)
+
+    def grads(deterministic):
+        torch.use_deterministic_algorithms(deterministic)
+        try:
+            o = F_.attention(q, k, v, cq, ck, max(lq), max(lk), hq, hk, d, causal)
+            return torch.autograd.grad(o, (q, k, v), do)
+        finally:
+            torch.use_deterministic_algorithms(False)
+
+    one, two, again = grads(False), grads(True), grads(True)
+    for a, b, c in zip(one, two, again):
+        assert torch.equal(b, c) and torch.isfinite(a).all() and rel(a, b) < 3e-3
+    if sum(lq) < 5000:
+        f = [t.detach().float().requires_grad_(True) for t in (q, k, v)]
+        ro = ref.attention_varlen(f[0].view(-1, hq, d), f[1].view(-1, hk, d), f[2].view(-1, hk, d), cq.cpu(), ck.cpu(), causal,
+                                  1 / math.sqrt(d)).reshape(-1, hq * d)
+        for a, r in zip(one, torch.autograd.grad(torch.nan_to_num(ro), f, do.float())):
+            assert rel(a, torch.nan_to_num(r)) < 1.2e-2
+
+
 def test_cross_attention_unequal_lengths(status):
     from pisceslx_b200.ops import functional as F_, reference as ref
     torch.manual_seed(12)

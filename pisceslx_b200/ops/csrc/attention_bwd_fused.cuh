@@ -61,42 +61,6 @@ struct AttnBwdFusedSmem {
 // a warp, a token each, meet no bank of shared memory twice.
 __device__ __forceinline__ int dq_piece(int64_t token, int j) { return j ^ (static_cast<int>(token >> 1) & 3); }
 
-__device__ __forceinline__ void tc_mma_f16_ss_if(uint32_t lead, uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
-                                                 uint32_t accumulate) {
-  asm volatile(
-      "{\n"
-      ".reg .pred p, q;\n"
-      "setp.ne.b32 p, %4, 0;\n"
-      "setp.ne.b32 q, %5, 0;\n"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
-      "}\n" ::"r"(tmem_d),
-      "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(lead)
-      : "memory");
-}
-
-__device__ __forceinline__ void tc_mma_f16_ts_if(uint32_t lead, uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc,
-                                                 uint32_t accumulate) {
-  asm volatile(
-      "{\n"
-      ".reg .pred p, q;\n"
-      "setp.ne.b32 p, %4, 0;\n"
-      "setp.ne.b32 q, %5, 0;\n"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
-      "}\n" ::"r"(tmem_d),
-      "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(lead)
-      : "memory");
-}
-
-__device__ __forceinline__ void tc_commit_if(uint32_t lead, uint64_t* bar) {
-  asm volatile(
-      "{\n"
-      ".reg .pred q;\n"
-      "setp.ne.b32 q, %1, 0;\n"
-      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n"
-      "}\n" ::"r"(smem_u32(bar)), "r"(lead)
-      : "memory");
-}
-
 // Unswizzled K-major operand of 16 along the summed dimension: rows of 16 bytes, the groups of 8 rows `sbo` bytes apart, the second
 // 8 of the 16 `lbo` bytes behind the first.
 __device__ __forceinline__ uint64_t make_smem_desc_plain(const uint8_t* tile, uint32_t lbo, uint32_t sbo) {

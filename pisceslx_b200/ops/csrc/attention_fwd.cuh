@@ -144,7 +144,10 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(ml_empty + 1);
   float2* ml = reinterpret_cast<float2*>(reinterpret_cast<uint8_t*>(bars) + 256);     // [128] per query row
 
-  const int warp = threadIdx.x >> 5;
+  // At 128 the products are issued by a whole warp (1 x 16384, 32 / 8 heads, causal 1797 -> 1753 us; 2 x 4096 254 -> 247); at 64,
+  // where the softmax warps have no issue slots to spare, by one thread (4 x 5329, 16 heads: 675 us, by the warp 704).
+  constexpr bool kWarpIssues = D == 128;
+  const int warp = kWarpIssues ? __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0) : threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
@@ -220,7 +223,11 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
     }
   } else if (warp == 9) {
     // ------------------------------------ MMA issuer ----------------------------------------
-    if (elect_one()) {
+    const uint32_t lead = elect_one() ? 1u : 0u;
+    auto commit = [&](uint64_t* bar) {
+      if (kWarpIssues) tc_commit_if(lead, bar); else tc_commit(bar);
+    };
+    if (kWarpIssues || lead != 0u) {
       bool ok = true;
       uint32_t kv = 0, nq[2] = {0u, 0u}, np[2] = {0u, 0u};   // key tiles, Q tiles and P tiles so far
       for (int64_t r = 0; r * gridDim.x < p.items && ok; ++r) {
@@ -236,13 +243,14 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
 #pragma unroll
           for (int kk = 0; kk < D / 16; ++kk) {
             const uint32_t off = (kk / 4) * kBoxBytes + (kk % 4) * 32;
-            tc_mma_f16_ss(tS, make_smem_desc(aQ + off, 16, 1024), make_smem_desc(aK + off, 16, 1024), kIdescQK,
-                          kk != 0 ? 1u : 0u);
+            const uint64_t dq = make_smem_desc(aQ + off, 16, 1024), dk = make_smem_desc(aK + off, 16, 1024);
+            if (kWarpIssues) tc_mma_f16_ss_if(lead, tS, dq, dk, kIdescQK, kk != 0 ? 1u : 0u);
+            else tc_mma_f16_ss(tS, dq, dk, kIdescQK, kk != 0 ? 1u : 0u);
           }
-          tc_commit(&s_full[t]);
-          if (j + 1 == it.count(t)) tc_commit(&q_empty[t]);
+          commit(&s_full[t]);
+          if (j + 1 == it.count(t)) commit(&q_empty[t]);
           // the tile is free once the last query tile that sees it has been multiplied
-          if (it.last_reader(t, j)) tc_commit(&k_empty[s]);
+          if (it.last_reader(t, j)) commit(&k_empty[s]);
           return true;
         };
         for (int t = 0; t < 2 && ok; ++t) {
@@ -268,11 +276,12 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
 #pragma unroll
             for (int kk = 0; kk < kAttnBlock / 16; ++kk) {
               // 16 keys per step: 8 packed bf16x2 columns of P; 16 key rows (2048 B) of the V tile
-              tc_mma_f16_ts(tO, tP + kk * 8, make_smem_desc(aV + kk * 2048, kBoxBytes, 1024), kIdescPV,
-                            (j | kk) != 0 ? 1u : 0u);
+              const uint64_t dv = make_smem_desc(aV + kk * 2048, kBoxBytes, 1024);
+              if (kWarpIssues) tc_mma_f16_ts_if(lead, tO, tP + kk * 8, dv, kIdescPV, (j | kk) != 0 ? 1u : 0u);
+              else tc_mma_f16_ts(tO, tP + kk * 8, dv, kIdescPV, (j | kk) != 0 ? 1u : 0u);
             }
-            if (j + 1 == it.count(t)) tc_commit(&o_full[t]);
-            if (it.last_reader(t, j)) tc_commit(&v_empty[s]);
+            if (j + 1 == it.count(t)) commit(&o_full[t]);
+            if (it.last_reader(t, j)) commit(&v_empty[s]);
             if (j + 1 < it.count(t)) ok = issue_qk(t, j + 1);
           }
         }

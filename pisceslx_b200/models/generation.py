@@ -142,6 +142,12 @@ def _tp_size(model) -> int:
     return par.tp_size if par is not None else 1
 
 
+def to_device(values: List, dtype: torch.dtype, device: torch.device) -> torch.Tensor:
+    """A list as a tensor on ``device``, by way of pinned memory: a copy from pageable memory waits for all that runs there."""
+    t = torch.tensor(values, dtype=dtype)
+    return t.pin_memory().to(device, non_blocking=True) if device.type == "cuda" else t.to(device)
+
+
 def _prefill(model, ids: torch.Tensor, cache: YvPagedKVCache, seq_ids: List[int],
              want: Optional[List[int]] = None) -> Optional[torch.Tensor]:
     """Run the prompt(s), or the next portion of the prompt(s), [B, S] through the model, filling the cache; returns
@@ -163,20 +169,23 @@ def _prefill(model, ids: torch.Tensor, cache: YvPagedKVCache, seq_ids: List[int]
             raise ValueError("this model's attention does not continue a prompt from the cache")
         ctx.starts, ctx.lens = starts, [S] * B
         ctx.slots_of = lambda b, lo, hi: cache.slots(seq_ids[b], lo, hi)
-        first = torch.tensor(starts, dtype=torch.int32).to(ids.device)
+        first = to_device(starts, torch.int32, ids.device)
         ctx.positions = ctx.positions + first.repeat_interleave(S + pad)
         ctx.max_position = max(starts) + S + pad
     slots: List[int] = []
     for s in seq_ids:
         slots += cache.append_slots(s, S) + [-1] * pad
     ctx.cache = cache
-    ctx.slot_map = torch.tensor(slots, dtype=torch.int32).to(ids.device)
+    ctx.slot_map = to_device(slots, torch.int32, ids.device)
     ctx.page_source = lambda: (cache.block_table_tensor(seq_ids), cache.seq_lens_tensor(seq_ids))
     if want is not None and B != 1:
         raise ValueError("wanted places are given for one sequence at a time")
     out = model(input_ids=ids, ctx=ctx, return_logits=False, return_hidden=True)
     if want is not None:
-        return model.logits(out["hidden_states"][0, want, :]) if want else None
+        if not want:
+            return None
+        rows = out["hidden_states"][0]
+        return model.logits(rows.narrow(0, want[0], 1) if len(want) == 1 else rows[to_device(want, torch.long, rows.device)])
     return model.logits(out["hidden_states"][:, S - 1, :])
 
 

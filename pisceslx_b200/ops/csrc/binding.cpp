@@ -1,6 +1,7 @@
 // PyTorch bindings (torch.ops.yv.*) for the sm_100a kernels.  Every op checks device, dtype, layout
 // and alignment on the host, passes raw pointers plus the current stream to a launcher, and raises on
-// a non-zero launcher code.  No op allocates: outputs and scratch are passed in by the Python layer.
+// a non-zero launcher code.  The ops that wrap one kernel do not allocate, but for the attention backward's sums: outputs and scratch
+// are passed in; the differentiable ones of binding_autograd.inc make theirs.
 #include "binding_gemm.inc"
 
 namespace {
@@ -517,6 +518,24 @@ void moe_unpermute_sum(const Tensor& dxp, const Tensor& row_map, Tensor dx, int6
   check_rc(yv::launch_moe_unpermute_sum(dxp.data_ptr(), row_map.data_ptr<int>(), dx.data_ptr(), dx.numel() / cols,
                                         static_cast<int>(k), cols, cur_stream()),
            "moe_unpermute_sum");
+}
+
+void moe_row_weights(const Tensor& w, const Tensor& row_map, Tensor row_w) {
+  check_f32(w, "w"); check_i32(row_map, "row_map"); check_f32(row_w, "row_w");
+  TORCH_CHECK(w.is_contiguous() && row_map.is_contiguous() && row_w.is_contiguous() && w.numel() == row_map.numel(),
+              "moe_row_weights: one weight per assignment");
+  const c10::cuda::CUDAGuard guard(w.device());
+  check_rc(yv::launch_moe_row_weights(w.data_ptr<float>(), row_map.data_ptr<int>(), row_w.data_ptr<float>(), w.numel(), cur_stream()),
+           "moe_row_weights");
+}
+
+void moe_row_dots(const Tensor& rows, const Tensor& row_map, Tensor out) {
+  check_f32(rows, "rows"); check_i32(row_map, "row_map"); check_f32(out, "out");
+  TORCH_CHECK(rows.is_contiguous() && row_map.is_contiguous() && out.is_contiguous() && out.numel() == row_map.numel(),
+              "moe_row_dots: one value per assignment");
+  const c10::cuda::CUDAGuard guard(rows.device());
+  check_rc(yv::launch_moe_row_dots(rows.data_ptr<float>(), row_map.data_ptr<int>(), out.data_ptr<float>(), out.numel(), cur_stream()),
+           "moe_row_dots");
 }
 
 void gate_bias_update(Tensor bias, const Tensor& counts, double rate, double clampv) {

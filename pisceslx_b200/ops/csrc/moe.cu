@@ -373,6 +373,19 @@ __global__ void moe_unpermute_sum_kernel(const __nv_bfloat16* __restrict__ dxp, 
   }
 }
 
+// row_w[row_map[i]] = w[i], and out[i] = rows[row_map[i]]: the weights of the assignments to the rows of the expert order and back
+__global__ void moe_row_weights_kernel(const float* __restrict__ w, const int* __restrict__ row_map, float* __restrict__ row_w,
+                                       int64_t n) {
+  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i < n) row_w[row_map[i]] = w[i];
+}
+
+__global__ void moe_row_dots_kernel(const float* __restrict__ rows, const int* __restrict__ row_map, float* __restrict__ out,
+                                    int64_t n) {
+  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i < n) out[i] = rows[row_map[i]];
+}
+
 __global__ void gate_bias_update_kernel(float* __restrict__ bias, const int* __restrict__ counts, int E, float rate,
                                         float clampv) {
   __shared__ float total;
@@ -594,6 +607,18 @@ int launch_moe_unpermute_sum(const void* dxp, const int* row_map, void* dx, int6
   const int block = (cols >> 3) >= 256 ? 256 : 128;
   moe_unpermute_sum_kernel<<<static_cast<unsigned>(tokens), block, 0, stream>>>(YV_BF(dxp), row_map, YV_BFM(dx), k,
                                                                                 cols);
+  return static_cast<int>(cudaGetLastError());
+}
+
+int launch_moe_row_weights(const float* w, const int* row_map, float* row_w, int64_t n, cudaStream_t stream) {
+  if (n <= 0) return 0;
+  moe_row_weights_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, stream>>>(w, row_map, row_w, n);
+  return static_cast<int>(cudaGetLastError());
+}
+
+int launch_moe_row_dots(const float* rows, const int* row_map, float* out, int64_t n, cudaStream_t stream) {
+  if (n <= 0) return 0;
+  moe_row_dots_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, stream>>>(rows, row_map, out, n);
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -185,6 +185,9 @@ int launch_moe_combine_bwd(const void* dout, const void* y, const int* row_map, 
 // backward of permute: dx[t] = sum_j dxp[row_map[t,j]]
 int launch_moe_unpermute_sum(const void* dxp, const int* row_map, void* dx, int64_t tokens, int k, int cols,
                              cudaStream_t stream);
+// row_w[row_map[i]] = w[i] (zero the rest first); out[i] = rows[row_map[i]]
+int launch_moe_row_weights(const float* w, const int* row_map, float* row_w, int64_t n, cudaStream_t stream);
+int launch_moe_row_dots(const float* rows, const int* row_map, float* out, int64_t n, cudaStream_t stream);
 // aux-loss-free bias update: bias += rate * (1/E - counts/total), clamped to [-clamp, clamp]
 int launch_gate_bias_update(float* bias, const int* counts, int E, float rate, float clamp, cudaStream_t stream);
 

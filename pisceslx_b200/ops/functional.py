@@ -1,7 +1,7 @@
 """Differentiable operator API used by the models.
 
-CUDA tensors run the sm_100a kernels through ``torch.autograd.Function`` wrappers that allocate their
-outputs with the caching allocator and never synchronise with the host; CPU tensors run
+CUDA tensors run the sm_100a kernels through autograd functions (of a decoder layer in ``csrc/binding_autograd.inc``, the others
+here) that allocate their outputs with the caching allocator and never synchronise with the host; CPU tensors run
 ``ops.reference``.  Shapes follow the "tokens first" convention: activations are 2-D ``[T, features]``
 with sequences packed along ``T`` and described by ``cu_seqlens``.
 """
@@ -135,43 +135,13 @@ def skinny_parts(x2: torch.Tensor, w: torch.Tensor) -> Optional[torch.Tensor]:
     return ws[:slices * 128 * w.shape[0]].view(slices, 128, w.shape[0])
 
 
-class _LinearFn(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, w, out_fp32):
-        x2 = _as2d(x)
-        if not x2.is_contiguous() and x2.stride(1) != 1:
-            x2 = x2.contiguous()
-        ctx.save_for_backward(x2, w)
-        ctx.x_shape = x.shape
-        out_dtype = torch.float32 if out_fp32 else _BF16
-        y = gemm_skinny(x2, w, None, out_dtype) if _few_rows(*w.shape) else None
-        if y is None:
-            y = gemm(x2, w, out_dtype=out_dtype)
-        return y.view(*x.shape[:-1], w.shape[0])
-
-    @staticmethod
-    def backward(ctx, dy):
-        x2, w = ctx.saved_tensors
-        dy2 = _as2d(dy)
-        if dy2.dtype != _BF16:
-            dy2 = dy2.to(_BF16)
-        if not dy2.is_contiguous():
-            dy2 = dy2.contiguous()
-        dx = dw = None
-        if ctx.needs_input_grad[0]:
-            dx = gemm(dy2, w, b_mn=True).view(ctx.x_shape)           # [M,N] x [N,K]
-        if ctx.needs_input_grad[1]:
-            dw = gemm(dy2, x2, a_mn=True, b_mn=True)                # [N,M] x [M,K]
-        return dx, dw, None
-
-
 def linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None,
            out_fp32: bool = False) -> torch.Tensor:
     """y = x @ w.T (+ bias); w is [out, in]."""
     if x.is_cuda:
         if x.dtype != _BF16:
             x = x.to(_BF16)
-        y = _LinearFn.apply(x, w if w.dtype == _BF16 else w.to(_BF16), out_fp32)
+        y = _k().linear(x, w if w.dtype == _BF16 else w.to(_BF16), out_fp32, _few_rows(*w.shape), _st(x))
     else:
         y = torch.nn.functional.linear(x, w.to(x.dtype))
         if out_fp32:
@@ -184,7 +154,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None
 # --------------------------------------------------------------------------------------------------
 # RMSNorm (+ residual add, + FiLM epilogue)
 # --------------------------------------------------------------------------------------------------
-class _RMSNormFn(torch.autograd.Function):
+class _FiLMNormFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, residual, w, eps, film_scale, film_shift):
         shape = x.shape
@@ -197,13 +167,10 @@ class _RMSNormFn(torch.autograd.Function):
         if residual is not None:
             r2 = _as2d(residual).contiguous()
             res_out = torch.empty_like(x2)
-        film_rows = 1
-        fs = fb = None
-        if film_scale is not None:
-            fs = _as2d(film_scale).contiguous()
-            fb = _as2d(film_shift).contiguous()
-            assert rows % fs.shape[0] == 0, "FiLM groups must divide the rows"
-            film_rows = rows // fs.shape[0]
+        fs = _as2d(film_scale).contiguous()
+        fb = _as2d(film_shift).contiguous()
+        assert rows % fs.shape[0] == 0, "FiLM groups must divide the rows"
+        film_rows = rows // fs.shape[0]
         _k().rmsnorm_fwd(x2, r2, w, fs, fb, film_rows, y, res_out, rstd, eps)
         normed_in = res_out if res_out is not None else x2
         ctx.save_for_backward(normed_in, w, rstd, fs, fb)
@@ -219,15 +186,13 @@ class _RMSNormFn(torch.autograd.Function):
         xin, w, rstd, fs, fb = ctx.saved_tensors
         dy2 = _as2d(dy).contiguous()
         rows, cols = xin.shape
-        dfs = dfb = None
-        if fs is not None:
-            # y = n * (1 + s) + b  ->  dn = dy * (1 + s), ds = sum_rows dy * n, db = sum_rows dy
-            G = fs.shape[0]
-            xf = xin.float() * rstd.unsqueeze(1) * w.float()
-            dyf = dy2.float().view(G, ctx.film_rows, cols)
-            dfs = (dyf * xf.view(G, ctx.film_rows, cols)).sum(1).to(fs.dtype)
-            dfb = dyf.sum(1).to(fs.dtype)
-            dy2 = (dyf * (1.0 + fs.float()).unsqueeze(1)).view(rows, cols).to(_BF16)
+        # y = n * (1 + s) + b  ->  dn = dy * (1 + s), ds = sum_rows dy * n, db = sum_rows dy
+        G = fs.shape[0]
+        xf = xin.float() * rstd.unsqueeze(1) * w.float()
+        dyf = dy2.float().view(G, ctx.film_rows, cols)
+        dfs = (dyf * xf.view(G, ctx.film_rows, cols)).sum(1).to(fs.dtype)
+        dfb = dyf.sum(1).to(fs.dtype)
+        dy2 = (dyf * (1.0 + fs.float()).unsqueeze(1)).view(rows, cols).to(_BF16)
         dx = torch.empty_like(xin)
         dwp = torch.empty(min(rows, _NORM_BWD_BLOCKS), cols, dtype=torch.float32, device=xin.device)
         dw = torch.empty(cols, dtype=torch.float32, device=xin.device)
@@ -242,7 +207,11 @@ def rms_norm(x: torch.Tensor, w: torch.Tensor, eps: float = 1e-6, residual: Opti
     """Returns ``(y, new_residual)``: y = rmsnorm(x + residual) * w [then FiLM]; new_residual = x + residual
     (``None`` when no residual is given)."""
     if x.is_cuda:
-        return _RMSNormFn.apply(x, residual, w, eps, film_scale, film_shift)
+        if film_scale is not None:
+            return _FiLMNormFn.apply(x, residual, w, eps, film_scale, film_shift)
+        if residual is None:
+            return _k().rms_norm(x, w, eps), None
+        return _k().rms_norm_residual(x, residual, w, eps)
     s = x if residual is None else x + residual
     y = ref.rms_norm(s, w, eps)
     if film_scale is not None:
@@ -312,33 +281,10 @@ def swiglu(gate_up: torch.Tensor) -> torch.Tensor:
     return ref.swiglu(gate_up)
 
 
-class _SwiGLUMixFn(torch.autograd.Function):
-    """SwiGLU whose rows are multiplied by weights that repeat with their number: out[r] = mix[r % S] * swiglu(in[r])."""
-
-    @staticmethod
-    def forward(ctx, gate_up, mix):
-        g2 = _as2d(gate_up).contiguous()
-        out = torch.empty(g2.shape[0], g2.shape[1] // 2, dtype=_BF16, device=g2.device)
-        mix = mix.float().contiguous()
-        _k().swiglu_fwd(g2, out, mix)
-        ctx.save_for_backward(g2, mix)
-        ctx.shape = gate_up.shape
-        return out.view(*gate_up.shape[:-1], out.shape[1])
-
-    @staticmethod
-    def backward(ctx, dout):
-        g2, mix = ctx.saved_tensors
-        d2 = _as2d(dout).contiguous()
-        din = torch.empty_like(g2)
-        dots = torch.empty(g2.shape[0], dtype=torch.float32, device=g2.device)
-        _k().swiglu_bwd_rows(g2, d2, mix, din, None, dots, mix.numel())
-        return din.view(ctx.shape), dots.view(-1, mix.numel()).sum(0) if ctx.needs_input_grad[1] else None
-
-
 def swiglu_mix(gate_up: torch.Tensor, mix: torch.Tensor) -> torch.Tensor:
     """mix[r % S] * silu(x[r, :F]) * x[r, F:] for rows r of ``gate_up`` [.., 2 F] and fp32 weights ``mix`` [S]."""
     if gate_up.is_cuda and gate_up.dtype == _BF16:
-        return _SwiGLUMixFn.apply(gate_up, mix)
+        return _k().swiglu_mix(gate_up, mix)
     act = ref.swiglu(gate_up)
     return (act.reshape(-1, mix.numel(), act.shape[-1]) * mix.to(act.dtype).view(1, -1, 1)).reshape(act.shape)
 
@@ -346,55 +292,14 @@ def swiglu_mix(gate_up: torch.Tensor, mix: torch.Tensor) -> torch.Tensor:
 # --------------------------------------------------------------------------------------------------
 # RoPE + flash attention on a fused QKV buffer
 # --------------------------------------------------------------------------------------------------
-class _RopeAttentionFn(torch.autograd.Function):
-    """qkv [T, (hq+2hk)*d] -> o [T, hq*d].  RoPE is applied in place to the q and k columns of the buffer
-    (after the call the buffer holds the rotated q/k, which is what a KV cache stores)."""
-
-    @staticmethod
-    def forward(ctx, qkv, cos, sin, positions, cu_q, max_len, hq, hk, d, rot_dim, causal, scale):
-        T = qkv.shape[0]
-        q = qkv[:, : hq * d]
-        k = qkv[:, hq * d: (hq + hk) * d]
-        v = qkv[:, (hq + hk) * d:]
-        K = _k()
-        if cos is not None:
-            K.rope(q, k, cos, sin, positions, hq, hk, d, rot_dim, False)
-        o = torch.empty(T, hq * d, dtype=_BF16, device=qkv.device)
-        lse = torch.empty(hq, T, dtype=torch.float32, device=qkv.device)
-        K.attn_fwd(q, k, v, o, lse, cu_q, None, max_len, max_len, hq, hk, d, causal, scale, _st(qkv))
-        ctx.save_for_backward(qkv, o, lse, cos, sin, positions, cu_q)
-        ctx.cfg = (max_len, hq, hk, d, rot_dim, causal, scale)
-        return o
-
-    @staticmethod
-    def backward(ctx, do):
-        qkv, o, lse, cos, sin, positions, cu_q = ctx.saved_tensors
-        max_len, hq, hk, d, rot_dim, causal, scale = ctx.cfg
-        T = qkv.shape[0]
-        q = qkv[:, : hq * d]
-        k = qkv[:, hq * d: (hq + hk) * d]
-        v = qkv[:, (hq + hk) * d:]
-        dqkv = torch.empty_like(qkv)
-        dq = dqkv[:, : hq * d]
-        dk = dqkv[:, hq * d: (hq + hk) * d]
-        dv = dqkv[:, (hq + hk) * d:]
-        delta = torch.empty(hq, T, dtype=torch.float32, device=qkv.device)
-        K = _k()
-        K.attn_bwd(do.contiguous(), q, k, v, o, lse, dq, dk, dv, delta, cu_q, None, max_len, max_len, hq, hk, d,
-                   causal, scale, _st(qkv))
-        if cos is not None:
-            K.rope(dq, dk, cos, sin, positions, hq, hk, d, rot_dim, True)
-        return (dqkv,) + (None,) * 11
-
-
 def rope_attention(qkv: torch.Tensor, cos: Optional[torch.Tensor], sin: Optional[torch.Tensor],
                    positions: Optional[torch.Tensor], cu_seqlens: torch.Tensor, max_len: int, hq: int, hk: int,
                    d: int, rot_dim: int, causal: bool = True, scale: Optional[float] = None) -> torch.Tensor:
-    """Self-attention over packed sequences from a fused projection ``qkv [T, (hq+2hk)*d]``."""
+    """Self-attention over packed sequences from a fused projection ``qkv [T, (hq+2hk)*d]``.  On the GPU RoPE is applied in
+    place to the q and k columns of the buffer (after the call it holds the rotated q/k, which is what a KV cache stores)."""
     scale = 1.0 / math.sqrt(d) if scale is None else scale
     if qkv.is_cuda:
-        return _RopeAttentionFn.apply(qkv, cos, sin, positions, cu_seqlens, max_len, hq, hk, d, rot_dim, causal,
-                                      scale)
+        return _k().rope_attention(qkv, cos, sin, positions, cu_seqlens, max_len, hq, hk, d, rot_dim, causal, scale, _st(qkv))
     T = qkv.shape[0]
     q = qkv[:, : hq * d].reshape(T, hq, d)
     k = qkv[:, hq * d: (hq + hk) * d].reshape(T, hk, d)

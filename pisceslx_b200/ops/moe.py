@@ -25,30 +25,6 @@ def _k():
 # --------------------------------------------------------------------------------------------------
 # routing
 # --------------------------------------------------------------------------------------------------
-class _GateFn(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, logits, bias, k, bias_in_combine, renorm_mode):
-        T, E = logits.shape
-        lf = logits.float().contiguous()
-        w = torch.empty(T, k, dtype=torch.float32, device=logits.device)
-        idx = torch.empty(T, k, dtype=torch.int32, device=logits.device)
-        probs = torch.empty(T, E, dtype=torch.float32, device=logits.device)
-        counts = torch.zeros(E, dtype=torch.int32, device=logits.device)
-        _k().gate_topk(lf, bias, w, idx, probs, counts, bias_in_combine, renorm_mode)
-        ctx.save_for_backward(probs, idx, w)
-        ctx.renorm_mode = renorm_mode
-        ctx.in_dtype = logits.dtype
-        ctx.mark_non_differentiable(idx, counts, probs)
-        return w, idx, counts, probs
-
-    @staticmethod
-    def backward(ctx, dw, _didx, _dcounts, _dprobs):
-        probs, idx, w = ctx.saved_tensors
-        dlogits = torch.empty_like(probs)
-        _k().gate_topk_bwd(dw.float().contiguous(), probs, idx, w, dlogits, ctx.renorm_mode)
-        return dlogits.to(ctx.in_dtype), None, None, None, None
-
-
 def gate_topk(logits: torch.Tensor, bias: Optional[torch.Tensor], k: int, bias_in_combine: bool = True,
               renorm_mode: int = 0) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor]:
     """logits [T,E] -> (weights [T,k] fp32, idx [T,k], counts [E], probs [T,E]).
@@ -59,7 +35,7 @@ def gate_topk(logits: torch.Tensor, bias: Optional[torch.Tensor], k: int, bias_i
     (reference, gate.py:1221)."""
     if logits.is_cuda:
         b = bias.float().contiguous() if bias is not None else None
-        return _GateFn.apply(logits, b, k, bias_in_combine, renorm_mode)
+        return _k().route(logits, b, k, bias_in_combine, renorm_mode)
     w, idx, probs, counts = ref.gate_topk(logits, bias, k, bias_in_combine, renorm_mode)
     return w, idx, counts, probs
 
@@ -119,35 +95,20 @@ def _few_tokens(assignments: int, w13: torch.Tensor, w2: torch.Tensor) -> bool:
     return assignments <= 192 * E and F % 64 == 0 and w13.is_contiguous() and w2.is_contiguous()
 
 
-def _experts_few(xp: torch.Tensor, plan: DispatchPlan, w13: torch.Tensor, w2: torch.Tensor, st) -> torch.Tensor:
-    """Expert outputs [rows, H] of a permuted layout without a gradient; rows that hold no token are left as they are."""
-    K = _k()
-    E, H, F = w2.shape
-    # token slots per pass over a tile's weights: no expert gets a token twice from the router, and a second pass (80 % of the
-    # first one's time again at T = 1024) costs far more than empty slots (1 us)
-    tokens = plan.row_map.shape[0]
-    slots = min(tokens, 64 if tokens * plan.k <= 16 * E else 128)
-    act = torch.empty(xp.shape[0], F, dtype=_BF16, device=xp.device)
-    y2 = torch.empty(xp.shape[0], H, dtype=_BF16, device=xp.device)
-    layout = (plan.tile_expert, plan.num_m_tiles, plan.seg_offsets, plan.counts, slots)
-    K.gemm_skinny_grouped(xp, w13, act, *layout, True, st)
-    K.gemm_skinny_grouped(act, w2, y2, *layout, False, st)
-    return y2
+def _few_slots(tokens: int, k: int, E: int) -> int:
+    """Token slots per pass over a tile's weights: no expert gets a token twice from the router, and a second pass (80 % of the
+    first one's time again at T = 1024) costs far more than empty slots (1 us)."""
+    return min(tokens, 64 if tokens * k <= 16 * E else 128)
 
 
-class _MoEExpertsFn(torch.autograd.Function):
-    """Keeps only the token rows ``x`` and the up-projection output ``y1`` for backward (per micro-batch of 8192
-    tokens x top-6 at hidden 4096 / FFN 1408: 0.07 + 0.28 GB instead of 1.3 GB with the permuted rows, the activation
-    and the expert outputs).  Backward rebuilds what it needs:
-      * the permuted rows from ``x`` and the saved row map (one gather);
-      * the activation from ``y1`` inside the SwiGLU-backward kernel;
-      * the combine-weight gradient without the expert outputs: with ``dA' = dout[token] @ W2[e]`` (the UNWEIGHTED
-        activation gradient), ``d weight = <SwiGLU(y1), dA'>`` per row, and the weight is applied afterwards
-        (``dy1 = w * dSwiGLU(y1, dA')``, ``dW2 = dout^T (w * act)``).  That is also exact for assignments whose weight
-        is zero (dropped by the capacity rule)."""
+class _MxExpertsFn(torch.autograd.Function):
+    """Routed experts whose forward products run on the block-scaled fp8 tensor cores: rows quantised per 32 elements on the fly,
+    the expert weights once per optimizer step; backward stays in bf16 from the saved bf16 tensors, which are those of the
+    function in ``csrc/binding_autograd.inc``."""
 
     @staticmethod
-    def forward(ctx, x, w13, w2, weights, idx, counts, deterministic, training=True, fp8=None, add=None, few=True):
+    def forward(ctx, x, w13, w2, weights, idx, counts, deterministic, add):
+        from ..quant import fp8 as q8
         K = _k()
         st = status_word(x.device)
         T, H = x.shape
@@ -155,37 +116,21 @@ class _MoEExpertsFn(torch.autograd.Function):
         F = twoF // 2
         x = x.contiguous()
         add = None if add is None else add.contiguous()
-        mx = fp8 == "mx" and H % 128 == 0 and twoF % 128 == 0 and F % 128 == 0
-        xp, plan = permute_tokens(x, idx, counts, E, deterministic, zero_pad=training or mx)
+        xp, plan = permute_tokens(x, idx, counts, E, deterministic, zero_pad=True)
         wts = weights.float().contiguous()
-        if few and not training and not mx and _few_tokens(T * idx.shape[1], w13, w2):
-            y2 = _experts_few(xp, plan, w13, w2, st)
-            out = torch.empty(T, H, dtype=_BF16, device=x.device)
-            K.moe_combine(y2, plan.row_map, wts, add, out)
-            return out
         y1 = torch.empty(plan.max_rows, twoF, dtype=_BF16, device=x.device)
         act = torch.empty(plan.max_rows, F, dtype=_BF16, device=x.device)
         y2 = torch.empty(plan.max_rows, H, dtype=_BF16, device=x.device)
-        if mx:
-            # forward products on the block-scaled fp8 tensor cores: rows quantised per 32 elements on the fly, the
-            # expert weights once per optimizer step; backward stays in bf16 from the saved bf16 tensors
-            from ..quant import fp8 as q8
-            xq, xs = q8.quantize_mx(xp)
-            del xp
-            wq, ws = _mx_weight(w13)
-            K.gemm_mxfp8(xq, xs, wq, ws, y1, plan.tile_expert, plan.num_m_tiles, 0, st)
-            del xq, xs
-            K.swiglu_fwd(y1, act)
-            aq, as_ = q8.quantize_mx(act)
-            wq, ws = _mx_weight(w2)
-            K.gemm_mxfp8(aq, as_, wq, ws, y2, plan.tile_expert, plan.num_m_tiles, 0, st)
-            del aq, as_
-        else:
-            K.gemm_grouped_m(xp, w13, y1, plan.tile_expert, plan.num_m_tiles, False, 0, st)
-            del xp
-            K.swiglu_fwd(y1, act)
-            K.gemm_grouped_m(act, w2, y2, plan.tile_expert, plan.num_m_tiles, False, 0, st)
-        del act
+        xq, xs = q8.quantize_mx(xp)
+        del xp
+        wq, ws = _mx_weight(w13)
+        K.gemm_mxfp8(xq, xs, wq, ws, y1, plan.tile_expert, plan.num_m_tiles, 0, st)
+        del xq, xs
+        K.swiglu_fwd(y1, act)
+        aq, as_ = q8.quantize_mx(act)
+        wq, ws = _mx_weight(w2)
+        K.gemm_mxfp8(aq, as_, wq, ws, y2, plan.tile_expert, plan.num_m_tiles, 0, st)
+        del aq, as_, act
         out = torch.empty(T, H, dtype=_BF16, device=x.device)
         K.moe_combine(y2, plan.row_map, wts, add, out)
         ctx.save_for_backward(x, y1, w13, w2, wts, idx, plan.row_map, plan.seg_offsets, plan.tile_expert,
@@ -205,7 +150,7 @@ class _MoEExpertsFn(torch.autograd.Function):
         dout = dout.contiguous()
         # combine weight of every expert row (0 on pad rows)
         row_w = torch.zeros(max_rows, dtype=torch.float32, device=dev)
-        row_w.index_put_((row_map.flatten().long(),), wts.flatten())
+        K.moe_row_weights(wts, row_map, row_w)
         # unweighted output gradient in expert-row order
         dy2 = torch.empty(max_rows, H, dtype=_BF16, device=dev)
         K.moe_permute(dout, idx, None, row_map, dy2)
@@ -221,7 +166,8 @@ class _MoEExpertsFn(torch.autograd.Function):
         dw2 = torch.empty_like(w2)
         K.gemm_grouped_k(dy2, act_w, dw2, seg, False, 0, st)                          # [H, rows_e] x [rows_e, F]
         del dy2, act_w
-        dwts = rowdot[row_map.flatten().long()].view(T, k)
+        dwts = torch.empty(T, k, dtype=torch.float32, device=dev)
+        K.moe_row_dots(rowdot, row_map, dwts)
         # up projection
         dxp = torch.empty(max_rows, H, dtype=_BF16, device=dev)
         K.gemm_grouped_m(dy1, w13, dxp, tile_expert, num_tiles, True, 0, st)          # dy1 [rows,2F] x w13[e] [2F,H]
@@ -233,7 +179,7 @@ class _MoEExpertsFn(torch.autograd.Function):
         del xp, dy1
         dx = torch.empty(T, H, dtype=_BF16, device=dev)
         K.moe_unpermute_sum(dxp, row_map, dx, k)
-        return dx, dw13, dw2, dwts.to(ctx.w_dtype), None, None, None, None, None, (dout if ctx.has_add else None), None
+        return dx, dw13, dw2, dwts.to(ctx.w_dtype), None, None, None, (dout if ctx.has_add else None)
 
 
 _MX_WEIGHTS = WeakIdKeyDictionary()      # the copies of a weight live as long as the tensor that they were made of
@@ -268,9 +214,16 @@ def moe_experts(x: torch.Tensor, w13: torch.Tensor, w2: torch.Tensor, weights: t
     E = w13.shape[0]
     if counts is None:
         counts = torch.bincount(idx.flatten().long(), minlength=E).int()
-    # without autograd (inference) nothing reads what the pad rows of the expert segments produce: skip zeroing them
-    return _MoEExpertsFn.apply(x.to(_BF16), w13, w2, weights, idx.int(), counts.int(), deterministic,
-                               torch.is_grad_enabled(), fp8, None if add is None else add.to(_BF16), few)
+    x, idx, counts = x.to(_BF16), idx.int(), counts.int()
+    add = None if add is None else add.to(_BF16)
+    training = torch.is_grad_enabled()
+    F, H = w13.shape[1] // 2, x.shape[1]
+    if fp8 == "mx" and H % 128 == 0 and F % 128 == 0:
+        return _MxExpertsFn.apply(x, w13, w2, weights, idx, counts, deterministic, add)
+    # without autograd (inference) nothing reads what the pad rows of the expert segments produce: zeroing them is skipped
+    T, k = idx.shape
+    slots = _few_slots(T, k, E) if few and not training and _few_tokens(T * k, w13, w2) else 0
+    return _k().moe_experts(x, w13, w2, weights, add, idx, counts, deterministic, training, slots, status_word(x.device))
 
 
 def capacity_mask(weights: torch.Tensor, idx: torch.Tensor, probs: torch.Tensor, counts: torch.Tensor,

@@ -18,7 +18,7 @@ from typing import Any, Callable, Deque, Dict, Iterator, List, Optional
 import torch
 
 from ..models.cache import YvPagedKVCache, cache_for_model
-from ..models.generation import YvSampler, YvSamplingConfig, _decode_step, _prefill
+from ..models.generation import YvSampler, YvSamplingConfig, _decode_step, _prefill, to_device
 from ..models.tokenizer import YvTokenizer
 
 
@@ -179,7 +179,7 @@ class YvInferenceEngine:
         for lo in range(0, len(tokens), size):
             part = tokens[lo:lo + size]
             here = [w - lo for w in order if lo <= w < lo + len(part)]
-            ids = torch.tensor([part], dtype=torch.long, device=self.device)
+            ids = to_device([part], torch.long, self.device)
             parts.append(_prefill(self.model, ids, self.cache, [seq_id], want=here))
         if not want:
             return None

@@ -65,6 +65,13 @@ class YvPackedTrunk(nn.Module):
                            max_position=max_len)
 
 
+class YvTokenEmbedding(nn.Embedding):
+    """``nn.Embedding`` whose gradient comes from ``ops.functional.embedding``."""
+
+    def forward(self, input: torch.Tensor) -> torch.Tensor:
+        return F_.embedding(input, self.weight)
+
+
 class YvModel(YvPackedTrunk):
     def __init__(self, cfg: YvConfig, parallel=None):
         super().__init__()
@@ -75,7 +82,7 @@ class YvModel(YvPackedTrunk):
         self.layer_lo, self.layer_hi = pp_rank * per, min(cfg.n_layer, (pp_rank + 1) * per)
         self.is_first_stage, self.is_last_stage = pp_rank == 0, pp_rank == pp_size - 1
         if self.is_first_stage:
-            self.embed = nn.Embedding(cfg.vocab_size, cfg.hidden_size)
+            self.embed = YvTokenEmbedding(cfg.vocab_size, cfg.hidden_size)
             nn.init.normal_(self.embed.weight, std=cfg.initializer_range)
         self.layers = nn.ModuleList([YvTransformerBlock(cfg, i, parallel) for i in range(self.layer_lo, self.layer_hi)])
         if self.is_last_stage:
@@ -271,8 +278,9 @@ class YvModelForCausalLM(nn.Module):
             B, S, H = hidden.shape
             L = labels.shape[1]
             h_txt = hidden[:, S - L:, :]                      # right-align to the labels (modal prefix skipped)
-            h_in = h_txt[:, :-1, :].reshape(-1, H)
-            tgt = labels[:, 1:].reshape(-1)
+            # the last token has no target: its row stays and is ignored, so that the states need not be copied
+            h_in = h_txt.reshape(-1, H)
+            tgt = torch.nn.functional.pad(labels[:, 1:], (0, 1), value=-100).reshape(-1)
             nv = None
             if num_valid is not None:
                 nv = num_valid

@@ -19,7 +19,7 @@ CSRC = HERE / "csrc"
 OBJ = HERE / "build"
 SO = HERE / "_yv_ops.so"
 
-CUDA_SOURCES = ["gemm.cu", "skinny.cu", "elementwise.cu", "moe.cu", "loss_optim.cu", "attention.cu", "comm.cu", "noalloc.cu", "ssm.cu", "pq_film.cu",
+CUDA_SOURCES = ["gemm.cu", "skinny.cu", "elementwise.cu", "moe.cu", "loss_optim.cu", "embedding.cu", "attention.cu", "comm.cu", "noalloc.cu", "ssm.cu", "pq_film.cu",
                 "stream.cu", "latent.cu", "grouped.cu"]
 CPP_SOURCES = ["binding.cpp"]
 # Layered models can be served by a library of their own: the products and the stream, and the operators of their mixers.

@@ -185,6 +185,11 @@ int launch_moe_combine_bwd(const void* dout, const void* y, const int* row_map, 
 // backward of permute: dx[t] = sum_j dxp[row_map[t,j]]
 int launch_moe_unpermute_sum(const void* dxp, const int* row_map, void* dx, int64_t tokens, int k, int cols,
                              cudaStream_t stream);
+// dw [V, H] (bf16) = sums of the rows of dy [T, H] (bf16) by their words ids [T]; order: 2 T ints, carry: 2 ceil(T / 32) H floats of
+// scratch.  H a multiple of 8, T up to the limit: the places are found by T^2 comparisons.
+constexpr int64_t kEmbeddingGradTokens = 65536;
+int launch_embedding_grad(const void* dy, const int64_t* ids, void* dw, int* order, float* carry, int64_t T, int64_t V, int H,
+                          cudaStream_t stream);
 // row_w[row_map[i]] = w[i] (zero the rest first); out[i] = rows[row_map[i]]
 int launch_moe_row_weights(const float* w, const int* row_map, float* row_w, int64_t n, cudaStream_t stream);
 int launch_moe_row_dots(const float* rows, const int* row_map, float* out, int64_t n, cudaStream_t stream);

@@ -151,6 +151,13 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None
     return y
 
 
+def embedding(ids: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
+    """Rows of ``w`` [V, H]; on the GPU with a gradient that is summed by word without a sort."""
+    if w.is_cuda and w.dtype == _BF16 and w.requires_grad and torch.is_grad_enabled():
+        return _k().embedding(w, ids)
+    return torch.nn.functional.embedding(ids, w)
+
+
 # --------------------------------------------------------------------------------------------------
 # RMSNorm (+ residual add, + FiLM epilogue)
 # --------------------------------------------------------------------------------------------------

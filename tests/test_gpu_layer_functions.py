@@ -110,3 +110,21 @@ def test_saved_tensors_pass_the_hooks_and_transforms_stay_refused():
     import torch.autograd.forward_ad as fw
     with pytest.raises((RuntimeError, NotImplementedError)), fw.dual_level():
         F_.linear(fw.make_dual(x.detach(), torch.ones_like(x)), w.detach())
+
+
+@pytest.mark.parametrize("T,V,H", [(1, 5, 8), (32, 4000, 264), (33, 1, 2056), (95, 2, 128), (2049, 7, 64), (4100, 100000, 40)])
+def test_embedding_gradient(T, V, H):
+    """Runs of equal words within a block of 32 places, over its edges and over many blocks; chunks of 2048 comparisons."""
+    F_, _, _ = _ops()
+    r = _gen(T)
+    w = r(V, H).to(BF16).requires_grad_(True)
+    ids = torch.randint(0, V, (1, T), device="cuda", generator=torch.Generator("cuda").manual_seed(V))
+    y = F_.embedding(ids, w)
+    assert torch.equal(y, torch.nn.functional.embedding(ids, w))
+    dy = r(1, T, H).to(BF16)
+    grads = [torch.autograd.grad(F_.embedding(i, w), w, dy)[0] for i in (ids, ids, ids.int())]
+    assert all(torch.equal(grads[0], g) for g in grads[1:])
+    want = torch.zeros(V, H, device="cuda", dtype=torch.float64).index_add_(0, ids[0], dy[0].double())
+    # one rounding to bf16 of sums whose fp32 additions err far less
+    assert ((grads[0].double() - want).abs() <= want.abs() * 2.0 ** -8 + T * 2.0 ** -22).all()
+    assert (grads[0][want.abs().sum(1) == 0] == 0).all()

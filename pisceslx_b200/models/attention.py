@@ -247,20 +247,20 @@ class YvAttention(nn.Module):
         B = qkv.shape[0]
         nq, nk = self.hq * self.d, self.hk * self.d
         q, k, v = qkv[:, :nq], qkv[:, nq:nq + nk], qkv[:, nq + nk:]
-        if ctx.cos is not None:
-            if qkv.is_cuda:
-                from ..ops import kernels
-                kernels().rope(q, k, ctx.cos, ctx.sin, ctx.positions, self.hq, self.hk, self.d, self.rot_dim, False)
-            else:
+        kc, vc = ctx.cache.layer(self.layer_idx)
+        if ctx.cos is not None and qkv.is_cuda:
+            F_.rope_cache(q, k, v, ctx.cos, ctx.sin, ctx.positions, self.hq, self.hk, self.d, self.rot_dim, kc, vc, ctx.slot_map)
+        else:
+            if ctx.cos is not None:
                 from ..ops import reference as ref
                 q = ref.apply_rope(q.reshape(B, self.hq, self.d), ctx.cos, ctx.sin, ctx.positions,
                                    self.rot_dim).reshape(B, nq)
                 k = ref.apply_rope(k.reshape(B, self.hk, self.d), ctx.cos, ctx.sin, ctx.positions,
                                    self.rot_dim).reshape(B, nk)
-        kc, vc = ctx.cache.layer(self.layer_idx)
-        F_.kv_cache_write(k, v, kc, vc, ctx.slot_map)
-        o = F_.paged_decode(q.reshape(B, self.hq, self.d).contiguous(), kc, vc, ctx.block_table, ctx.seq_lens,
-                            self.scale)
+            F_.kv_cache_write(k, v, kc, vc, ctx.slot_map)
+        # on the GPU the queries are read where they lie in the projection
+        q = q.view(B, self.hq, self.d) if q.is_cuda else q.reshape(B, self.hq, self.d).contiguous()
+        o = F_.paged_decode(q, kc, vc, ctx.block_table, ctx.seq_lens, self.scale)
         return o.reshape(B, nq)
 
     # -- checkpoint key mapping ----------------------------------------------------------------------------

@@ -77,6 +77,7 @@ class YvStableMoEGate(nn.Module):
         self._calls = 0
         self.recomputing = False          # set by the activation-checkpoint wrapper during recomputation
         self.last_counts: Optional[torch.Tensor] = None
+        self.last_plan: Optional[torch.Tensor] = None      # dispatch plan of the last call, where the router made it
         self.load_predictor: Optional[nn.LSTM] = None
         if cfg.moe_use_load_predictor:
             self.load_predictor = nn.LSTM(self.num_experts, 32, batch_first=True)
@@ -103,6 +104,12 @@ class YvStableMoEGate(nn.Module):
         if adj is not None:
             logits = logits + adj.to(logits.dtype)
         bias = self.expert_bias if self.aux_loss_free else None
+        self.last_plan = None
+        if self.aux_loss_free and not (self.training or self.drop_tokens):
+            few = moe_ops.route_few(logits, bias, self.top_k, self.bias_in_combine, self.renorm_mode)
+            if few is not None:
+                weights, idx, self.last_counts, self.last_plan, zero = few
+                return weights, idx, zero
         weights, idx, counts, probs = moe_ops.gate_topk(logits, bias, self.top_k, self.bias_in_combine,
                                                         self.renorm_mode)
         if self.drop_tokens:
@@ -147,6 +154,7 @@ class YvMoEGate(YvStableMoEGate):
     def forward(self, x: torch.Tensor):
         if self.temperature == 1.0 and not (self.training and self.noise_std > 0):
             return super().forward(x)
+        self.last_plan = None
         x2 = x.reshape(-1, x.shape[-1])
         T = x2.shape[0]
         logits = F_.linear(x2, self.gate.weight, out_fp32=True) / self.temperature

@@ -119,7 +119,7 @@ class YvDeepSeekMoELayer(nn.Module):
         else:
             out = moe_ops.moe_experts(x, self.experts_w13, self.experts_w2, weights, idx, counts,
                                       self.deterministic, fp8=getattr(self.cfg, "expert_fp8", None), add=sh,
-                                      few=not self.training)
+                                      few=not self.training, plan=getattr(self.router, "last_plan", None))
         if sh is not None and self.skip_prev:
             if self._prev_shared is not None and self._prev_shared.shape == sh.shape:
                 out = out + 0.1 * self._prev_shared

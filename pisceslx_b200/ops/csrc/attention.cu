@@ -229,6 +229,13 @@ int decode_tma_dispatch(const PagedDecodeTmaParams& pp, int G, dim3 grid, int sm
 }
 }  // namespace
 
+// The tensor-core kernel: pages of 64 tokens, and a group of query heads that fits a tile of 16.
+bool paged_decode_uses_mma(const PagedDecodeArgs& a) {
+  const int G = a.hk > 0 && a.hq % a.hk == 0 ? a.hq / a.hk : 0;
+  return a.block == 64 && static_cast<int64_t>(a.num_blocks) * a.block < (1ll << 31) && !a.force_direct &&
+         (G == 1 || G == 2 || G == 4 || G == 8);
+}
+
 int launch_paged_decode(const PagedDecodeArgs& a, cudaStream_t stream) {
   if (a.batch <= 0) return 0;
   if (a.d != 64 && a.d != 128) return -1;
@@ -253,7 +260,7 @@ int launch_paged_decode(const PagedDecodeArgs& a, cudaStream_t stream) {
   // TMA-fed kernel: whole cache blocks of up to 128 tokens travel as one bulk copy each
   const int64_t slots = static_cast<int64_t>(a.num_blocks) * a.block;
   const bool use_tma = a.block >= 16 && a.block <= 128 && a.block % 16 == 0 && slots < (1ll << 31) && !a.force_direct;
-  const bool use_mma = use_tma && a.block == 64 && (G == 1 || G == 2 || G == 4 || G == 8);
+  const bool use_mma = paged_decode_uses_mma(a);
   if (use_mma) {
     // tensor-core kernel: keys are the M dimension, the query heads of the group are padded to N = 16
     PagedDecodeMmaParams pm = {};
@@ -261,8 +268,8 @@ int launch_paged_decode(const PagedDecodeArgs& a, cudaStream_t stream) {
     if (r != 0) return -40 + r;
     r = paged_decode_map(&pm.tma_v, a.v_cache, a.d, a.hk, slots);
     if (r != 0) return -50 + r;
-    pm.q = p.q; pm.q_ld = static_cast<int64_t>(a.hq) * a.d;
-    pm.o = p.o; pm.o_ld = pm.q_ld;
+    pm.q = p.q; pm.q_ld = a.q_stride != 0 ? a.q_stride : static_cast<int64_t>(a.hq) * a.d;
+    pm.o = p.o; pm.o_ld = static_cast<int64_t>(a.hq) * a.d;
     pm.partial_o = a.partial_o; pm.partial_ml = a.partial_ml;
     pm.block_table = a.block_table; pm.seq_lens = a.seq_lens;
     pm.hq = a.hq; pm.group = G; pm.chunks = 1;
@@ -311,7 +318,10 @@ int launch_kv_cache_write(const void* k, const void* v, void* k_cache, void* v_c
                           int64_t tokens, int row_elems, int64_t k_stride, int64_t v_stride, int64_t num_slots,
                           uint32_t* status, cudaStream_t stream) {
   if (tokens <= 0) return 0;
-  if ((row_elems & 7) != 0) return -1;
+  // rows are read and written 16 bytes at a time
+  const uintptr_t at = reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(k_cache) |
+                       reinterpret_cast<uintptr_t>(v_cache);
+  if ((row_elems & 7) != 0 || ((k_stride | v_stride) & 7) != 0 || (at & 15u) != 0) return -1;
   return launch_chained_if(tokens <= kChainBlocks, kv_cache_write_kernel<true>, kv_cache_write_kernel<false>,
                            dim3(static_cast<unsigned>(tokens)), dim3(128), 0, stream,
                         reinterpret_cast<const __nv_bfloat16*>(k), reinterpret_cast<const __nv_bfloat16*>(v),

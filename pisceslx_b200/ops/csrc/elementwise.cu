@@ -7,6 +7,7 @@
 #include <stdint.h>
 
 #include "chain.cuh"
+#include "sm100.cuh"
 #include "yv_ops.h"
 
 namespace yv {
@@ -287,12 +288,21 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ q, __nv_bfloat16* __rest
 // The same with 16-byte accesses: a thread owns eight pairs of a token and walks every `groups`-th head with their angles in
 // registers.  `chunks` = rot_dim / 16 threads times `groups` per token.  Bound by memory:
 // 16384 tokens, 40 heads of 128 in 58 us (5.8 TB/s) instead of 122 with two bytes at a time.
-template <bool CHAIN>
+// With CACHE the k heads go to a paged cache as well, and the hk heads of v, which are only copied.
+struct RopeCache {
+  const __nv_bfloat16* v;
+  __nv_bfloat16 *k_cache, *v_cache;
+  const int* slot_map;
+  int64_t v_stride, num_slots;
+  uint32_t* status;
+};
+
+template <bool CHAIN, bool CACHE>
 __global__ void __launch_bounds__(256) rope_vec_kernel(__nv_bfloat16* __restrict__ q, __nv_bfloat16* __restrict__ k,
                                                        const float* __restrict__ cos_t, const float* __restrict__ sin_t,
                                                        const int* __restrict__ positions, int64_t tokens, int hq, int hk,
                                                        int head_dim, int chunks, int groups, int inverse, int64_t q_stride,
-                                                       int64_t k_stride) {
+                                                       int64_t k_stride, const RopeCache cache) {
   chain_start<CHAIN>();
   const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
   const int64_t t = i / (chunks * groups);
@@ -310,7 +320,24 @@ __global__ void __launch_bounds__(256) rope_vec_kernel(__nv_bfloat16* __restrict
 #pragma unroll
     for (int j = 0; j < 8; ++j) s[j] = -s[j];
   }
-  for (int h = hg; h < hq + hk; h += groups) {
+  int64_t slot = -1;
+  if (CACHE) {
+    slot = cache.slot_map[t];
+    if (slot >= cache.num_slots) {
+      if (cache.status != nullptr && rest == 0) atomicOr(cache.status, kStatusIndexOutOfRange);
+      slot = -1;
+    }
+  }
+  for (int h = hg; h < hq + (CACHE ? 2 * hk : hk); h += groups) {
+    if (CACHE && h >= hq + hk) {
+      if (slot < 0) continue;                            // a padding token
+      const int64_t at_v = static_cast<int64_t>(h - hq - hk) * head_dim + p;
+      const __nv_bfloat16* from = cache.v + t * cache.v_stride + at_v;
+      __nv_bfloat16* to = cache.v_cache + slot * hk * head_dim + at_v;
+      *reinterpret_cast<uint4*>(to) = *reinterpret_cast<const uint4*>(from);
+      *reinterpret_cast<uint4*>(to + half) = *reinterpret_cast<const uint4*>(from + half);
+      continue;
+    }
     __nv_bfloat16* base = h < hq ? q + t * q_stride + static_cast<int64_t>(h) * head_dim + p
                                  : k + t * k_stride + static_cast<int64_t>(h - hq) * head_dim + p;
     float a[8], b[8], x[8], y[8];
@@ -323,6 +350,11 @@ __global__ void __launch_bounds__(256) rope_vec_kernel(__nv_bfloat16* __restrict
     }
     store8(base, x);
     store8(base + half, y);
+    if (CACHE && h >= hq && slot >= 0) {
+      __nv_bfloat16* to = cache.k_cache + slot * hk * head_dim + static_cast<int64_t>(h - hq) * head_dim + p;
+      store8(to, x);
+      store8(to + half, y);
+    }
   }
 }
 
@@ -562,6 +594,43 @@ int launch_colsum(const float* partial, int blocks, int cols, void* out, int out
   return static_cast<int>(cudaGetLastError());
 }
 
+namespace {
+template <bool CACHE>
+int launch_rope_vec(__nv_bfloat16* q, __nv_bfloat16* k, const float* cos_t, const float* sin_t, const int* positions,
+                    int64_t tokens, int hq, int hk, int head_dim, int rot_dim, int inverse, int64_t q_stride, int64_t k_stride,
+                    const RopeCache& cache, cudaStream_t stream) {
+  // A thread reads its angles once for the heads that it walks, one behind the other at a load's latency: as many heads, up to
+  // an eighth of them, as still leave 2048 threads to every SM; small blocks where there is less than one for each SM.  Eight
+  // groups and blocks of 256 at any size, and now: 40 heads of 128, 1 token 3.0 and 1.8 us, 128 tokens 4.3 and 2.7, 1000 6.7
+  // and 6.1; 20 heads of 64, 128 tokens 3.5 and 2.3 (by pairs 2.4).
+  const int chunks = rot_dim / 16, heads = hq + (CACHE ? 2 * hk : hk);
+  const int64_t each = tokens * chunks * heads / (int64_t{148} * 2048), most = (heads + 7) / 8;
+  const int walk = static_cast<int>(each < 1 ? 1 : each < most ? each : most);
+  const int groups = (heads + walk - 1) / walk;
+  const int64_t threads = tokens * chunks * groups;
+  const int block = threads >= 148 * 256 ? 256 : 64;
+  const int64_t blocks = (threads + block - 1) / block;
+  // the blocks that start early all find a place (8192 tokens, 6 heads of 64: 5.3 us chained, 5.9 not)
+  return launch_chained_if(blocks <= 8 * kChainBlocks, rope_vec_kernel<true, CACHE>, rope_vec_kernel<false, CACHE>,
+                           dim3(static_cast<unsigned>(blocks)), dim3(block), 0, stream, q, k, cos_t, sin_t, positions, tokens, hq, hk,
+                           head_dim, chunks, groups, inverse, q_stride, k_stride, cache);
+}
+}  // namespace
+
+int launch_rope_cache(void* q, void* k, const void* v, const float* cos_t, const float* sin_t, const int* positions, int64_t tokens,
+                      int hq, int hk, int head_dim, int64_t q_stride, int64_t k_stride, int64_t v_stride, void* k_cache,
+                      void* v_cache, const int* slot_map, int64_t num_slots, uint32_t* status, cudaStream_t stream) {
+  if (tokens <= 0) return 0;
+  const uintptr_t at = reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) |
+                       reinterpret_cast<uintptr_t>(cos_t) | reinterpret_cast<uintptr_t>(sin_t) |
+                       reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache);
+  if (head_dim < 64 || head_dim % 16 != 0 || q_stride % 8 != 0 || k_stride % 8 != 0 || v_stride % 8 != 0 || (at & 15u) != 0)
+    return kRopeCacheApart;
+  return launch_rope_vec<true>(YV_BFM(q), YV_BFM(k), cos_t, sin_t, positions, tokens, hq, hk, head_dim, head_dim, 0, q_stride,
+                               k_stride, RopeCache{YV_BF(v), YV_BFM(k_cache), YV_BFM(v_cache), slot_map, v_stride, num_slots, status},
+                               stream);
+}
+
 int launch_rope_tables(void* q, void* k, const float* cos_t, const float* sin_t, const int* positions,
                        int64_t tokens, int hq, int hk, int head_dim, int rot_dim, int inverse, int64_t q_stride,
                        int64_t k_stride, cudaStream_t stream) {
@@ -573,21 +642,8 @@ int launch_rope_tables(void* q, void* k, const float* cos_t, const float* sin_t,
   // A quarter of a head's pairs or less per thread leaves too few loads in flight: 40 heads of 128 of which 32 are rotated, 8192
   // tokens 23.7 us by vectors and 17.3 by pairs, 1000 tokens 5.6 and 3.9; of 64, 20 heads, 13.2 and 17.5, 3.7 and 3.8.
   if (rot_dim >= 64 && rot_dim % 16 == 0 && head_dim % 8 == 0 && q_stride % 8 == 0 && k_stride % 8 == 0 && aligned) {
-    // A thread reads its angles once for the heads that it walks, one behind the other at a load's latency: as many heads, up to
-    // an eighth of them, as still leave 2048 threads to every SM; small blocks where there is less than one for each SM.  Eight
-    // groups and blocks of 256 at any size, and now: 40 heads of 128, 1 token 3.0 and 1.8 us, 128 tokens 4.3 and 2.7, 1000 6.7
-    // and 6.1; 20 heads of 64, 128 tokens 3.5 and 2.3 (by pairs 2.4).
-    const int chunks = rot_dim / 16, heads = hq + hk;
-    const int64_t each = tokens * chunks * heads / (int64_t{148} * 2048), most = (heads + 7) / 8;
-    const int walk = static_cast<int>(each < 1 ? 1 : each < most ? each : most);
-    const int groups = (heads + walk - 1) / walk;
-    const int64_t threads = tokens * chunks * groups;
-    const int block = threads >= 148 * 256 ? 256 : 64;
-    const int64_t blocks = (threads + block - 1) / block;
-    // the blocks that start early all find a place (8192 tokens, 6 heads of 64: 5.3 us chained, 5.9 not)
-    return launch_chained_if(blocks <= 8 * kChainBlocks, rope_vec_kernel<true>, rope_vec_kernel<false>,
-                             dim3(static_cast<unsigned>(blocks)), dim3(block), 0, stream, YV_BFM(q), YV_BFM(k), cos_t, sin_t,
-                             positions, tokens, hq, hk, head_dim, chunks, groups, inverse, q_stride, k_stride);
+    return launch_rope_vec<false>(YV_BFM(q), YV_BFM(k), cos_t, sin_t, positions, tokens, hq, hk, head_dim, rot_dim, inverse,
+                                  q_stride, k_stride, RopeCache{}, stream);
   }
   const int total = (hq + hk) * (rot_dim >> 1);
   const int block = total >= 256 ? 256 : ((total + 31) / 32) * 32;

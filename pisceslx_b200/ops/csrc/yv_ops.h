@@ -81,6 +81,12 @@ int launch_colsum(const float* partial, int blocks, int cols, void* out, int out
 int launch_rope_tables(void* q, void* k, const float* cos_t, const float* sin_t, const int* positions,
                        int64_t tokens, int hq, int hk, int head_dim, int rot_dim, int inverse, int64_t q_stride,
                        int64_t k_stride, cudaStream_t stream);
+// The same over whole heads, and k and v appended to the paged caches at slot_map (as launch_kv_cache_write) by the same kernel;
+// returns kRopeCacheApart when the operands are not what it reads (the two launches then do it).
+constexpr int kRopeCacheApart = -100;
+int launch_rope_cache(void* q, void* k, const void* v, const float* cos_t, const float* sin_t, const int* positions, int64_t tokens,
+                      int hq, int hk, int head_dim, int64_t q_stride, int64_t k_stride, int64_t v_stride, void* k_cache,
+                      void* v_cache, const int* slot_map, int64_t num_slots, uint32_t* status, cudaStream_t stream);
 // 3-D (t, h, w) rotary embedding for video tokens: head_dim split in three sections.
 int launch_rope3d(void* q, void* k, const int* pos_thw, int64_t tokens, int hq, int hk, int head_dim, int d_t,
                   int d_h, int d_w, float theta, int inverse, cudaStream_t stream);
@@ -190,6 +196,11 @@ int launch_moe_unpermute_sum(const void* dxp, const int* row_map, void* dx, int6
 constexpr int64_t kEmbeddingGradTokens = 65536;
 int launch_embedding_grad(const void* dy, const int64_t* ids, void* dw, int* order, float* carry, int64_t T, int64_t V, int H,
                           cudaStream_t stream);
+// Router and dispatch plan of up to kPlanTokens tokens in one kernel (E <= 256); *zero = 0.
+constexpr int64_t kPlanTokens = 16;
+int launch_gate_plan(const float* logits, const float* bias, float* weights, int* idx, int* counts, int* seg_offsets,
+                     int* tile_expert, int* num_m_tiles, int* row_map, float* zero, int64_t tokens, int E, int k, int max_tiles,
+                     int bias_in_combine, int renorm_mode, cudaStream_t stream);
 // row_w[row_map[i]] = w[i] (zero the rest first); out[i] = rows[row_map[i]]
 int launch_moe_row_weights(const float* w, const int* row_map, float* row_w, int64_t n, cudaStream_t stream);
 int launch_moe_row_dots(const float* rows, const int* row_map, float* out, int64_t n, cudaStream_t stream);
@@ -233,6 +244,7 @@ struct AttnBwdArgs {
 int launch_attn_bwd(const AttnBwdArgs& a, cudaStream_t stream);
 // Paged-KV decode: one query token per sequence.
 struct PagedDecodeArgs {
+  int64_t q_stride = 0;            // elements between the rows of q, 0: hq * d (which it is unless paged_decode_uses_mma)
   const void* q = nullptr;         // bf16 [B, hq, d]
   const void* k_cache = nullptr;   // bf16 [num_blocks, block, hk, d]
   const void* v_cache = nullptr;
@@ -246,6 +258,7 @@ struct PagedDecodeArgs {
   uint32_t* status = nullptr;
   bool force_direct = false;       // true: the direct-load kernel (no TMA ring), whatever the block size
 };
+bool paged_decode_uses_mma(const PagedDecodeArgs& a);
 int launch_paged_decode(const PagedDecodeArgs& a, cudaStream_t stream);
 // k, v: [T, hk*d] rows with the given strides; caches: [num_slots, hk*d]; slot_map int32 [T] (-1 = skip)
 int launch_kv_cache_write(const void* k, const void* v, void* k_cache, void* v_cache, const int* slot_map,

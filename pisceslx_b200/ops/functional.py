@@ -372,11 +372,17 @@ def paged_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, 
         return ref.paged_decode(q, k_cache, v_cache, block_table, seq_lens, scale)
     if splits <= 0:
         splits = paged_splits(B * k_cache.shape[2], block_table.shape[1], 2 if d <= 64 else 1)
-    o = torch.empty_like(q)
+    o = torch.empty(B, hq, d, dtype=q.dtype, device=q.device)
     po = torch.empty(B, hq, splits, d, dtype=torch.float32, device=q.device)
     pml = torch.empty(B, hq, splits, 2, dtype=torch.float32, device=q.device)
-    _k().paged_decode(q.contiguous(), k_cache, v_cache, block_table, seq_lens, o, po, pml, splits, scale, _st(q))
+    _k().paged_decode(q, k_cache, v_cache, block_table, seq_lens, o, po, pml, splits, scale, _st(q))
     return o
+
+
+def rope_cache(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, positions: torch.Tensor,
+               hq: int, hk: int, d: int, rot_dim: int, k_cache: torch.Tensor, v_cache: torch.Tensor, slot_map: torch.Tensor) -> None:
+    """On the GPU: rotate q and k [T, h*d] in place and append k and v to the paged caches as ``kv_cache_write`` does."""
+    _k().rope_cache(q, k, v, cos, sin, positions, hq, hk, d, rot_dim, k_cache, v_cache, slot_map, _st(q))
 
 
 def kv_cache_write(k: torch.Tensor, v: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,

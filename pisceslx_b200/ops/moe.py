@@ -40,6 +40,18 @@ def gate_topk(logits: torch.Tensor, bias: Optional[torch.Tensor], k: int, bias_i
     return w, idx, counts, probs
 
 
+_PLAN_TOKENS = 16        # kPlanTokens of csrc/yv_ops.h
+
+
+def route_few(logits: torch.Tensor, bias: Optional[torch.Tensor], k: int, bias_in_combine: bool = True, renorm_mode: int = 0):
+    """``gate_topk`` of a few tokens without a gradient, and the experts' dispatch plan, in one kernel: (weights, idx, counts,
+    plan, a zero on the device), or None where that does not apply."""
+    if not logits.is_cuda or torch.is_grad_enabled() or not 1 <= logits.shape[0] <= _PLAN_TOKENS or logits.shape[1] > 256 or \
+            logits.dtype != torch.float32 or not logits.is_contiguous() or not 1 <= k <= 16:
+        return None
+    return _k().route_few(logits, None if bias is None else bias.float().contiguous(), k, bias_in_combine, renorm_mode)
+
+
 # --------------------------------------------------------------------------------------------------
 # dispatch plan
 # --------------------------------------------------------------------------------------------------
@@ -200,14 +212,16 @@ def _mx_weight(w: torch.Tensor):
 
 def moe_experts(x: torch.Tensor, w13: torch.Tensor, w2: torch.Tensor, weights: torch.Tensor, idx: torch.Tensor,
                 counts: Optional[torch.Tensor] = None, deterministic: bool = False,
-                fp8: Optional[str] = None, add: Optional[torch.Tensor] = None, few: bool = True) -> torch.Tensor:
+                fp8: Optional[str] = None, add: Optional[torch.Tensor] = None, few: bool = True,
+                plan: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Routed experts: out[t] = sum_j weights[t,j] * SwiGLU_FFN_{idx[t,j]}(x[t]).
 
     x [T,H]; w13 [E, 2F, H] (gate rows then up rows); w2 [E, H, F]; weights/idx [T,k]; counts [E] int32
     (the histogram the gate kernel produced; recomputed when omitted).  ``fp8="mx"`` runs the two forward products
     with e4m3 operands and one power-of-two scale per 32 elements (CUDA; H, F multiples of 128).  ``add`` [T,H], the shared
     experts' output, is added before the result is rounded.  ``few`` lets a pass without a gradient take the kernel for few
-    tokens, which rounds in other places; off, it equals a pass with a gradient bit for bit."""
+    tokens, which rounds in other places; off, it equals a pass with a gradient bit for bit.  ``plan``: what ``route_few`` returned with
+    these ``idx``."""
     if not x.is_cuda:
         out = ref.moe_experts(x, w13, w2, weights, idx)
         return out if add is None else out + add
@@ -223,7 +237,8 @@ def moe_experts(x: torch.Tensor, w13: torch.Tensor, w2: torch.Tensor, weights: t
     # without autograd (inference) nothing reads what the pad rows of the expert segments produce: zeroing them is skipped
     T, k = idx.shape
     slots = _few_slots(T, k, E) if few and not training and _few_tokens(T * k, w13, w2) else 0
-    return _k().moe_experts(x, w13, w2, weights, add, idx, counts, deterministic, training, slots, status_word(x.device))
+    return _k().moe_experts(x, w13, w2, weights, add, idx, counts, None if deterministic else plan, deterministic, training, slots,
+                            status_word(x.device))
 
 
 def capacity_mask(weights: torch.Tensor, idx: torch.Tensor, probs: torch.Tensor, counts: torch.Tensor,

@@ -20,7 +20,7 @@ import torch.nn as nn
 
 from ..config import YvConfig
 from ..ops import functional as F_
-from ..ops.loss import linear_cross_entropy
+from ..ops.loss import linear_cross_entropy, rows_at_once
 from .attention import AttnContext
 from .blocks import YvTransformerBlock
 from .norms import YvRMSNorm, YvRotaryEmbedding
@@ -284,7 +284,7 @@ class YvModelForCausalLM(nn.Module):
             nv = None
             if num_valid is not None:
                 nv = num_valid
-            lm_loss = linear_cross_entropy(h_in, self.head_weight, tgt, -100, nv)
+            lm_loss = linear_cross_entropy(h_in, self.head_weight, tgt, -100, nv, rows_at_once(h_in.shape[0], *self.head_weight.shape))
             loss = lm_loss
             res["lm_loss"] = lm_loss
             if self.num_mtp > 0:

@@ -128,3 +128,19 @@ def test_embedding_gradient(T, V, H):
     # one rounding to bf16 of sums whose fp32 additions err far less
     assert ((grads[0].double() - want).abs() <= want.abs() * 2.0 ** -8 + T * 2.0 ** -22).all()
     assert (grads[0][want.abs().sum(1) == 0] == 0).all()
+
+
+@pytest.mark.parametrize("T,V,H", [(300, 1000, 128), (513, 5000, 256)])
+def test_loss_in_one_chunk_and_in_several(T, V, H):
+    """The same sums in another order: the weight gradient is rounded to bf16 once either way, the rest row by row."""
+    from pisceslx_b200.ops.loss import linear_cross_entropy
+    r = _gen(T)
+    h, w = r(T, H).to(BF16).requires_grad_(True), (r(V, H) * H ** -0.5).to(BF16).requires_grad_(True)
+    labels = torch.randint(0, V, (T,), device="cuda", generator=torch.Generator("cuda").manual_seed(V))
+    labels[::7] = -100
+    out = []
+    for chunk in (128, T):
+        loss = linear_cross_entropy(h, w, labels, -100, None, chunk)
+        out.append((loss, *torch.autograd.grad(loss, (h, w))))
+    for a, b in zip(*out):
+        assert rel(a, b) < 2.0 ** -8

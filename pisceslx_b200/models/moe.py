@@ -56,6 +56,11 @@ def capacity_mask(weights: torch.Tensor, idx: torch.Tensor, probs: torch.Tensor,
     return torch.where(tot > 0, w / tot.clamp_min(1e-20), torch.zeros_like(w))
 
 
+def plan_version(idx: torch.Tensor) -> int:
+    """Version of expert numbers that a plan was made for; inference tensors have none."""
+    return 0 if idx.is_inference() else idx._version
+
+
 class YvStableMoEGate(nn.Module):
     def __init__(self, cfg: YvConfig, num_experts: Optional[int] = None, top_k: Optional[int] = None):
         super().__init__()
@@ -77,7 +82,8 @@ class YvStableMoEGate(nn.Module):
         self._calls = 0
         self.recomputing = False          # set by the activation-checkpoint wrapper during recomputation
         self.last_counts: Optional[torch.Tensor] = None
-        self.last_plan: Optional[torch.Tensor] = None      # dispatch plan of the last call, where the router made it
+        # expert numbers of the last call, their version, and the dispatch plan for them, where the router made it
+        self.last_plan: Optional[Tuple[torch.Tensor, int, torch.Tensor]] = None
         self.load_predictor: Optional[nn.LSTM] = None
         if cfg.moe_use_load_predictor:
             self.load_predictor = nn.LSTM(self.num_experts, 32, batch_first=True)
@@ -108,7 +114,8 @@ class YvStableMoEGate(nn.Module):
         if self.aux_loss_free and not (self.training or self.drop_tokens):
             few = moe_ops.route_few(logits, bias, self.top_k, self.bias_in_combine, self.renorm_mode)
             if few is not None:
-                weights, idx, self.last_counts, self.last_plan, zero = few
+                weights, idx, self.last_counts, plan, zero = few
+                self.last_plan = (idx, plan_version(idx), plan)
                 return weights, idx, zero
         weights, idx, counts, probs = moe_ops.gate_topk(logits, bias, self.top_k, self.bias_in_combine,
                                                         self.renorm_mode)

@@ -19,7 +19,7 @@ import torch.nn as nn
 from ..config import YvConfig
 from ..ops import functional as F_
 from ..ops import moe as moe_ops
-from .moe import YvMoEGate, YvStableMoEGate
+from .moe import YvMoEGate, YvStableMoEGate, plan_version
 
 
 class YvDeepSeekMoELayer(nn.Module):
@@ -108,6 +108,9 @@ class YvDeepSeekMoELayer(nn.Module):
         x = x.reshape(-1, shape[-1])
         weights, idx, aux = self.router(x)
         counts = self.router.last_counts
+        # the router's plan is for the very numbers that it returned
+        made = getattr(self.router, "last_plan", None)
+        plan = made[2] if made is not None and made[0] is idx and made[1] == plan_version(idx) else None
         sh = self._shared(x) if self.num_shared else None
         if self.ep_size > 1:
             from ..parallel import ep
@@ -119,7 +122,7 @@ class YvDeepSeekMoELayer(nn.Module):
         else:
             out = moe_ops.moe_experts(x, self.experts_w13, self.experts_w2, weights, idx, counts,
                                       self.deterministic, fp8=getattr(self.cfg, "expert_fp8", None), add=sh,
-                                      few=not self.training, plan=getattr(self.router, "last_plan", None))
+                                      few=not self.training, plan=plan)
         if sh is not None and self.skip_prev:
             if self._prev_shared is not None and self._prev_shared.shape == sh.shape:
                 out = out + 0.1 * self._prev_shared

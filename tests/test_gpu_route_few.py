@@ -122,3 +122,33 @@ def test_decode_reads_queries_inside_a_projection(hq, hk, d, page, extra):
             F_.paged_decode(q, kc, vc, table, lens)
         return
     assert torch.equal(F_.paged_decode(q, kc, vc, table, lens), F_.paged_decode(q.contiguous(), kc, vc, table, lens))
+
+
+def test_a_plan_is_for_the_numbers_that_the_router_returned():
+    """A router whose numbers are exchanged, or written to, after it has planned: the layer plans for itself."""
+    from pisceslx_b200 import YvConfig
+    from pisceslx_b200.models.moe_layer import YvDeepSeekMoELayer
+    torch.manual_seed(0)
+    cfg = YvConfig.tiny_text_moe()
+    layer = YvDeepSeekMoELayer(cfg, 0).to("cuda", BF16).eval()
+    x = torch.randn(9, cfg.hidden_size, device="cuda").to(BF16)
+    route = layer.router.forward
+    with torch.inference_mode():
+        served = layer(x)[0].clone()
+    with torch.no_grad():
+        plain = layer(x)[0]
+        assert layer.router.last_plan is not None and torch.equal(served, plain)
+
+        def exchanged(y):
+            w, idx, aux = route(y)
+            return w.flip(1), idx.flip(1), aux
+
+        def written(y):
+            w, idx, aux = route(y)
+            idx.copy_(idx.flip(1))
+            return w.flip(1), idx, aux
+
+        for forward in (exchanged, written):
+            layer.router.forward = forward
+            got = layer(x)[0]                              # the same sums in another order
+            assert float((got.float() - plain.float()).norm() / plain.float().norm()) < 1e-2

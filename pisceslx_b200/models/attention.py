@@ -93,6 +93,7 @@ class YvAttention(nn.Module):
         self.hq, self.hk, self.d = cfg.n_head // tp_size, cfg.n_kv_head // tp_size, cfg.head_dim
         self.rot_dim = cfg.partial_rope_dim if cfg.use_partial_rope else cfg.head_dim
         self.scale = 1.0 / math.sqrt(self.d)
+        self.deterministic = bool(cfg.extra.get("moe_deterministic", False))     # a step's bits repeat
         H = cfg.hidden_size
         std = cfg.initializer_range
         self.use_mla = bool(getattr(cfg, "use_mla", False))
@@ -205,7 +206,7 @@ class YvAttention(nn.Module):
         if ctx.cp_group is not None:
             return self._attend_context_parallel(qkv, ctx)
         o = F_.rope_attention(qkv, ctx.cos, ctx.sin, ctx.positions, ctx.cu_seqlens, ctx.max_len, self.hq, self.hk,
-                              self.d, self.rot_dim, ctx.causal, self.scale)
+                              self.d, self.rot_dim, ctx.causal, self.scale, self.deterministic)
         if ctx.cache is not None and ctx.slot_map is not None:
             kc, vc = ctx.cache.layer(self.layer_idx)
             k_rot, v_new = qkv[:, nq:nq + nk], qkv[:, nq + nk:]
@@ -237,10 +238,11 @@ class YvAttention(nn.Module):
                 # blocks of K / V travel round the ranks in both passes: no rank ever holds the whole sequence's keys
                 outs.append(cp.ring_attention_train(q[sl].contiguous(), k[sl].contiguous(), v[sl].contiguous(),
                                                     ctx.cp_group, self.hq, self.hk, self.d, causal=ctx.causal,
-                                                    scale=self.scale))
+                                                    scale=self.scale, deterministic=self.deterministic))
                 continue
             outs.append(cp.allgather_attention(q[sl].contiguous(), k[sl].contiguous(), v[sl].contiguous(), ctx.cp_group,
-                                               self.hq, self.hk, self.d, causal=ctx.causal, scale=self.scale))
+                                               self.hq, self.hk, self.d, causal=ctx.causal, scale=self.scale,
+                                               deterministic=self.deterministic))
         return torch.cat(outs, 0).to(qkv.dtype)
 
     def _decode(self, qkv: torch.Tensor, ctx: AttnContext) -> torch.Tensor:

@@ -23,7 +23,7 @@ import torch.nn.functional as F
 from ...config import YvConfig
 from ...ops import functional as F_
 from ..norms import YvLayerNorm
-from .vision import YvViTBlock, YvVideoEncoder, YvVisionEncoder
+from .vision import YvViTBlock, YvVideoEncoder, YvVisionEncoder, repeats
 
 
 def mel_filterbank(n_mels: int, n_fft: int, sr: int) -> torch.Tensor:
@@ -54,7 +54,7 @@ class YvAudioEncoder(nn.Module):
         self.register_buffer("window", torch.hann_window(self.n_fft), persistent=False)
         self.conv1 = nn.Conv1d(self.n_mels, dim, 3, padding=1)
         self.conv2 = nn.Conv1d(dim, dim, 3, stride=2, padding=1)
-        self.blocks = nn.ModuleList([YvViTBlock(dim, heads) for _ in range(depth)])
+        self.blocks = nn.ModuleList([YvViTBlock(dim, heads, deterministic=repeats(cfg)) for _ in range(depth)])
         self.norm = YvLayerNorm(dim)
         self.proj = nn.Parameter(torch.empty(cfg.hidden_size, dim).normal_(std=0.02))
         self.max_tokens = cfg.audio_tokens
@@ -88,8 +88,9 @@ class YvAudioEncoder(nn.Module):
 
 
 class YvCrossModalAttention(nn.Module):
-    def __init__(self, hidden: int, heads: int, dropout: float = 0.0):
+    def __init__(self, hidden: int, heads: int, dropout: float = 0.0, deterministic: bool = False):
         super().__init__()
+        self.deterministic = deterministic
         self.hidden, self.heads, self.hd = hidden, heads, hidden // heads
         self.norm_q, self.norm_kv = YvLayerNorm(hidden), YvLayerNorm(hidden)
         self.q_proj = nn.Parameter(torch.empty(hidden, hidden).normal_(std=0.02))
@@ -105,7 +106,8 @@ class YvCrossModalAttention(nn.Module):
         dev = query.device
         cq = torch.arange(0, (B + 1) * Sq, Sq, dtype=torch.int32, device=dev)
         ck = torch.arange(0, (B + 1) * Sk, Sk, dtype=torch.int32, device=dev)
-        o = F_.attention(q, kv[:, :H], kv[:, H:], cq, ck, Sq, Sk, self.heads, self.heads, self.hd, causal=False)
+        o = F_.attention(q, kv[:, :H], kv[:, H:], cq, ck, Sq, Sk, self.heads, self.heads, self.hd, causal=False,
+                         deterministic=self.deterministic)
         return F_.linear(o, self.o_proj).view(B, Sq, H)
 
 
@@ -117,9 +119,9 @@ class YvDynamicModalFusion(nn.Module):
         heads = heads or max(1, H // 128 if H % 128 == 0 else H // 64)
         self.n_out = cfg.native_fusion_output_tokens
         self.modal_embed = nn.Parameter(torch.zeros(4, H).normal_(std=0.02))       # image, video, audio, other
-        self.blocks = nn.ModuleList([YvViTBlock(H, heads) for _ in range(cfg.native_fusion_num_layers)])
+        self.blocks = nn.ModuleList([YvViTBlock(H, heads, deterministic=repeats(cfg)) for _ in range(cfg.native_fusion_num_layers)])
         self.queries = nn.Parameter(torch.zeros(self.n_out, H).normal_(std=0.02))
-        self.readout = YvCrossModalAttention(H, heads)
+        self.readout = YvCrossModalAttention(H, heads, deterministic=repeats(cfg))
         self.norm = YvLayerNorm(H)
 
     def forward(self, modal_tokens: Dict[str, torch.Tensor]) -> torch.Tensor:

@@ -62,9 +62,16 @@ class YvPatchEmbed(nn.Module):
         return self.weight[:, : self.k].reshape(self.dim, self.in_ch, self.patch, self.patch)
 
 
+def repeats(cfg: YvConfig) -> bool:
+    """Whether the bits of a training step are to repeat."""
+    return bool(cfg.extra.get("moe_deterministic", False))
+
+
 class YvViTBlock(nn.Module):
-    def __init__(self, dim: int, heads: int, mlp_ratio: float = 4.0, rope3d: Optional[YvSpatioTemporalRoPE3D] = None):
+    def __init__(self, dim: int, heads: int, mlp_ratio: float = 4.0, rope3d: Optional[YvSpatioTemporalRoPE3D] = None,
+                 deterministic: bool = False):
         super().__init__()
+        self.deterministic = deterministic
         self.dim, self.heads, self.hd = dim, heads, dim // heads
         self.norm1, self.norm2 = YvLayerNorm(dim), YvLayerNorm(dim)
         self.qkv = nn.Parameter(torch.empty(3 * dim, dim).normal_(std=0.02))
@@ -90,7 +97,8 @@ class YvViTBlock(nn.Module):
             q, k = q.reshape(T, d), k.reshape(T, d)
         else:
             q, k = qkv[:, :d], qkv[:, d:2 * d]
-        o = F_.attention(q, k, qkv[:, 2 * d:], cu, cu, max_len, max_len, self.heads, self.heads, self.hd, causal=False)
+        o = F_.attention(q, k, qkv[:, 2 * d:], cu, cu, max_len, max_len, self.heads, self.heads, self.hd, causal=False,
+                         deterministic=self.deterministic)
         x = x + F_.linear(o, self.proj, self.proj_bias)
         h = F.gelu(F_.linear(self.norm2(x), self.fc1, self.fc1_bias))
         return x + F_.linear(h, self.fc2, self.fc2_bias)
@@ -109,7 +117,7 @@ class YvVisionEncoder(nn.Module):
         self.base_grid = base_grid
         self.pos_embed = nn.Parameter(torch.zeros(1, self.dim, base_grid, base_grid).normal_(std=0.02))
         self.cls_token = nn.Parameter(torch.zeros(1, self.dim).normal_(std=0.02))
-        self.blocks = nn.ModuleList([YvViTBlock(self.dim, self.heads) for _ in range(self.depth)])
+        self.blocks = nn.ModuleList([YvViTBlock(self.dim, self.heads, deterministic=repeats(cfg)) for _ in range(self.depth)])
         self.norm = YvLayerNorm(self.dim)
         self.proj = nn.Parameter(torch.empty(cfg.hidden_size, self.dim).normal_(std=0.02))
 
@@ -167,7 +175,7 @@ class YvVideoEncoder(nn.Module):
         self.patch = cfg.image_patch
         self.patch_embed = YvPatchEmbed(self.patch, 3, self.dim)
         rope = YvSpatioTemporalRoPE3D(self.dim // self.heads)
-        self.blocks = nn.ModuleList([YvViTBlock(self.dim, self.heads, rope3d=rope) for _ in range(depth)])
+        self.blocks = nn.ModuleList([YvViTBlock(self.dim, self.heads, rope3d=rope, deterministic=repeats(cfg)) for _ in range(depth)])
         self.norm = YvLayerNorm(self.dim)
         self.proj = nn.Parameter(torch.empty(cfg.hidden_size, self.dim).normal_(std=0.02))
         self.out_tokens = out_tokens or cfg.video_tokens

@@ -301,12 +301,15 @@ def swiglu_mix(gate_up: torch.Tensor, mix: torch.Tensor) -> torch.Tensor:
 # --------------------------------------------------------------------------------------------------
 def rope_attention(qkv: torch.Tensor, cos: Optional[torch.Tensor], sin: Optional[torch.Tensor],
                    positions: Optional[torch.Tensor], cu_seqlens: torch.Tensor, max_len: int, hq: int, hk: int,
-                   d: int, rot_dim: int, causal: bool = True, scale: Optional[float] = None) -> torch.Tensor:
+                   d: int, rot_dim: int, causal: bool = True, scale: Optional[float] = None,
+                   deterministic: bool = False) -> torch.Tensor:
     """Self-attention over packed sequences from a fused projection ``qkv [T, (hq+2hk)*d]``.  On the GPU RoPE is applied in
-    place to the q and k columns of the buffer (after the call it holds the rotated q/k, which is what a KV cache stores)."""
+    place to the q and k columns of the buffer (after the call it holds the rotated q/k, which is what a KV cache stores).
+    ``deterministic``: gradients whose bits repeat (see ``attention``)."""
     scale = 1.0 / math.sqrt(d) if scale is None else scale
     if qkv.is_cuda:
-        return _k().rope_attention(qkv, cos, sin, positions, cu_seqlens, max_len, hq, hk, d, rot_dim, causal, scale, _st(qkv))
+        return _k().rope_attention(qkv, cos, sin, positions, cu_seqlens, max_len, hq, hk, d, rot_dim, causal, scale, _st(qkv),
+                                   deterministic)
     T = qkv.shape[0]
     q = qkv[:, : hq * d].reshape(T, hq, d)
     k = qkv[:, hq * d: (hq + hk) * d].reshape(T, hk, d)
@@ -321,34 +324,37 @@ class _AttentionFn(torch.autograd.Function):
     """Separate q [Tq, hq*d], k/v [Tk, hk*d] (cross attention, no RoPE)."""
 
     @staticmethod
-    def forward(ctx, q, k, v, cu_q, cu_k, max_q, max_k, hq, hk, d, causal, scale):
+    def forward(ctx, q, k, v, cu_q, cu_k, max_q, max_k, hq, hk, d, causal, scale, deterministic):
         q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
         o = torch.empty_like(q)
         lse = torch.empty(hq, q.shape[0], dtype=torch.float32, device=q.device)
         _k().attn_fwd(q, k, v, o, lse, cu_q, cu_k, max_q, max_k, hq, hk, d, causal, scale, _st(q))
         ctx.save_for_backward(q, k, v, o, lse, cu_q, cu_k)
-        ctx.cfg = (max_q, max_k, hq, hk, d, causal, scale)
+        ctx.cfg = (max_q, max_k, hq, hk, d, causal, scale, deterministic)
         return o
 
     @staticmethod
     def backward(ctx, do):
         q, k, v, o, lse, cu_q, cu_k = ctx.saved_tensors
-        max_q, max_k, hq, hk, d, causal, scale = ctx.cfg
+        max_q, max_k, hq, hk, d, causal, scale, deterministic = ctx.cfg
         dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
         delta = torch.empty(hq, q.shape[0], dtype=torch.float32, device=q.device)
         _k().attn_bwd(do.contiguous(), q, k, v, o, lse, dq, dk, dv, delta, cu_q, cu_k, max_q, max_k, hq, hk, d, causal,
-                      scale, _st(q))
-        return (dq, dk, dv) + (None,) * 9
+                      scale, _st(q), deterministic)
+        return (dq, dk, dv) + (None,) * 10
 
 
 def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cu_q: torch.Tensor,
               cu_k: Optional[torch.Tensor], max_q: int, max_k: int, hq: int, hk: int, d: int,
-              causal: bool = False, scale: Optional[float] = None) -> torch.Tensor:
-    """Packed attention with separate query / key sequences: q [Tq, hq*d], k/v [Tk, hk*d] -> [Tq, hq*d]."""
+              causal: bool = False, scale: Optional[float] = None, deterministic: bool = False) -> torch.Tensor:
+    """Packed attention with separate query / key sequences: q [Tq, hq*d], k/v [Tk, hk*d] -> [Tq, hq*d].
+
+    On the GPU the gradient of q is summed in no fixed order, so that its last bits may differ from call to call, unless
+    ``deterministic`` is set or ``torch.use_deterministic_algorithms`` is on."""
     scale = 1.0 / math.sqrt(d) if scale is None else scale
     if q.is_cuda:
         return _AttentionFn.apply(q.to(_BF16), k.to(_BF16), v.to(_BF16), cu_q, cu_k, max_q, max_k, hq, hk, d,
-                                  causal, scale)
+                                  causal, scale, deterministic)
     o = ref.attention_varlen(q.reshape(-1, hq, d), k.reshape(-1, hk, d), v.reshape(-1, hk, d), cu_q, cu_k, causal,
                              scale)
     return o.reshape(-1, hq * d)

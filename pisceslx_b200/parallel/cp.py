@@ -145,7 +145,7 @@ def _merge_into(o_acc: torch.Tensor, lse_acc: torch.Tensor, o_b: torch.Tensor, l
     return merge_partials(o_acc, lse_acc, o_b, lse_b)
 
 
-def _block_backward(do, q, k, v, o, lse, hq, hk, d, causal, scale):
+def _block_backward(do, q, k, v, o, lse, hq, hk, d, causal, scale, deterministic=False):
     """Gradients of ONE key/value block given the GLOBAL output and log-sum-exp of the local queries:
     p = exp(s - lse), dv = p^T do, ds = p * (do v^T - rowsum(do * o)), dq = ds k, dk = ds^T q."""
     L, Lk = q.shape[0], k.shape[0]
@@ -155,7 +155,8 @@ def _block_backward(do, q, k, v, o, lse, hq, hk, d, causal, scale):
         delta = torch.empty(hq, L, dtype=torch.float32, device=q.device)
         cq = torch.tensor([0, L], dtype=torch.int32, device=q.device)
         ck = torch.tensor([0, Lk], dtype=torch.int32, device=q.device)
-        K.attn_bwd(do, q, k, v, o, lse, dq, dk, dv, delta, cq, ck, L, Lk, hq, hk, d, causal, scale, status_word(q.device))
+        K.attn_bwd(do, q, k, v, o, lse, dq, dk, dv, delta, cq, ck, L, Lk, hq, hk, d, causal, scale, status_word(q.device),
+                   deterministic)
         return dq.float(), dk.float(), dv.float()
     g = hq // hk
     qq = q.float().view(L, hq, d).transpose(0, 1)
@@ -185,7 +186,7 @@ class _RingAttention(torch.autograd.Function):
     hand (recomputing p from the saved global log-sum-exp), and after W hops each accumulator is back at its owner."""
 
     @staticmethod
-    def forward(ctx, q, k, v, group, hq, hk, d, causal, scale):
+    def forward(ctx, q, k, v, group, hq, hk, d, causal, scale, deterministic):
         W, r = dist.get_world_size(group), dist.get_rank(group)
         L = q.shape[0]
         q, cur_k, cur_v = q.contiguous(), k.contiguous(), v.contiguous()
@@ -205,13 +206,13 @@ class _RingAttention(torch.autograd.Function):
                 cur_k, cur_v = nxt[0]
         o = o_acc.reshape(L, hq * d).to(q.dtype)
         ctx.save_for_backward(q, k.contiguous(), v.contiguous(), o, lse_acc.t().contiguous())       # lse as [hq, L]
-        ctx.cfg = (group, hq, hk, d, causal, scale)
+        ctx.cfg = (group, hq, hk, d, causal, scale, deterministic)
         return o
 
     @staticmethod
     def backward(ctx, do):
         q, k, v, o, lse = ctx.saved_tensors
-        group, hq, hk, d, causal, scale = ctx.cfg
+        group, hq, hk, d, causal, scale, deterministic = ctx.cfg
         W, r = dist.get_world_size(group), dist.get_rank(group)
         do = do.contiguous().to(q.dtype)
         dq = torch.zeros(q.shape, dtype=torch.float32, device=q.device)
@@ -220,7 +221,8 @@ class _RingAttention(torch.autograd.Function):
         for step in range(W):
             src = (r - step) % W
             if not causal or src <= r:
-                dq_b, dk_b, dv_b = _block_backward(do, q, cur[0], cur[1], o, lse, hq, hk, d, causal and src == r, scale)
+                dq_b, dk_b, dv_b = _block_backward(do, q, cur[0], cur[1], o, lse, hq, hk, d, causal and src == r, scale,
+                                                     deterministic)
                 dq += dq_b
                 cur[2] = cur[2] + dk_b
                 cur[3] = cur[3] + dv_b
@@ -230,14 +232,15 @@ class _RingAttention(torch.autograd.Function):
             for rq in reqs:
                 rq.wait()
             cur = recv if step + 1 < W else [None, None] + recv
-        return dq.to(q.dtype), cur[2].to(k.dtype), cur[3].to(v.dtype), None, None, None, None, None, None
+        return dq.to(q.dtype), cur[2].to(k.dtype), cur[3].to(v.dtype), None, None, None, None, None, None, None
 
 
 def ring_attention_train(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, group: Any, hq: int, hk: int, d: int,
-                         causal: bool = True, scale: Optional[float] = None) -> torch.Tensor:
-    """Differentiable ring attention: q [L, hq*d], k/v [L, hk*d] are this rank's contiguous chunk of one sequence."""
+                         causal: bool = True, scale: Optional[float] = None, deterministic: bool = False) -> torch.Tensor:
+    """Differentiable ring attention: q [L, hq*d], k/v [L, hk*d] are this rank's contiguous chunk of one sequence.
+    ``deterministic`` as in ``ops.functional.attention``."""
     scale = 1.0 / math.sqrt(d) if scale is None else scale
-    return _RingAttention.apply(q, k, v, group, hq, hk, d, causal, scale)
+    return _RingAttention.apply(q, k, v, group, hq, hk, d, causal, scale, deterministic)
 
 
 class _AllGatherKV(torch.autograd.Function):
@@ -265,7 +268,8 @@ class _AllGatherKV(torch.autograd.Function):
 
 
 def allgather_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, group: Any, hq: int, hk: int, d: int,
-                        causal: bool = True, scale: Optional[float] = None, zigzag: bool = False) -> torch.Tensor:
+                        causal: bool = True, scale: Optional[float] = None, zigzag: bool = False,
+                        deterministic: bool = False) -> torch.Tensor:
     """Differentiable context-parallel attention for one sequence.  Contiguous layout: rank r holds chunk r.
     Zig-zag layout: rank r holds chunks (r, 2W-1-r) stacked, each of length L/2."""
     W, r = dist.get_world_size(group), dist.get_rank(group)
@@ -275,7 +279,8 @@ def allgather_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, group
     def attend(qc: torch.Tensor, kc: torch.Tensor, vc: torch.Tensor, is_causal: bool) -> torch.Tensor:
         cq = torch.tensor([0, qc.shape[0]], dtype=torch.int32, device=q.device)
         ck = torch.tensor([0, kc.shape[0]], dtype=torch.int32, device=q.device)
-        return F_.attention(qc, kc, vc, cq, ck, qc.shape[0], kc.shape[0], hq, hk, d, causal=is_causal, scale=scale)
+        return F_.attention(qc, kc, vc, cq, ck, qc.shape[0], kc.shape[0], hq, hk, d, causal=is_causal, scale=scale,
+                            deterministic=deterministic)
 
     if not zigzag:
         horizon = (r + 1) * L if causal else W * L

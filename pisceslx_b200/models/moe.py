@@ -56,11 +56,6 @@ def capacity_mask(weights: torch.Tensor, idx: torch.Tensor, probs: torch.Tensor,
     return torch.where(tot > 0, w / tot.clamp_min(1e-20), torch.zeros_like(w))
 
 
-def plan_version(idx: torch.Tensor) -> int:
-    """Version of expert numbers that a plan was made for; inference tensors have none."""
-    return 0 if idx.is_inference() else idx._version
-
-
 class YvStableMoEGate(nn.Module):
     def __init__(self, cfg: YvConfig, num_experts: Optional[int] = None, top_k: Optional[int] = None):
         super().__init__()
@@ -111,11 +106,12 @@ class YvStableMoEGate(nn.Module):
             logits = logits + adj.to(logits.dtype)
         bias = self.expert_bias if self.aux_loss_free else None
         self.last_plan = None
-        if self.aux_loss_free and not (self.training or self.drop_tokens):
+        # inference tensors have no version: a write to the numbers would go unseen
+        if self.aux_loss_free and not (self.training or self.drop_tokens or torch.is_inference_mode_enabled()):
             few = moe_ops.route_few(logits, bias, self.top_k, self.bias_in_combine, self.renorm_mode)
             if few is not None:
                 weights, idx, self.last_counts, plan, zero = few
-                self.last_plan = (idx, plan_version(idx), plan)
+                self.last_plan = (idx, idx._version, plan)
                 return weights, idx, zero
         weights, idx, counts, probs = moe_ops.gate_topk(logits, bias, self.top_k, self.bias_in_combine,
                                                         self.renorm_mode)

@@ -19,7 +19,7 @@ import torch.nn as nn
 from ..config import YvConfig
 from ..ops import functional as F_
 from ..ops import moe as moe_ops
-from .moe import YvMoEGate, YvStableMoEGate, plan_version
+from .moe import YvMoEGate, YvStableMoEGate
 
 
 class YvDeepSeekMoELayer(nn.Module):
@@ -108,9 +108,9 @@ class YvDeepSeekMoELayer(nn.Module):
         x = x.reshape(-1, shape[-1])
         weights, idx, aux = self.router(x)
         counts = self.router.last_counts
-        # the router's plan is for the very numbers that it returned
+        # the router's plan is for the very numbers that it returned, as they were then
         made = getattr(self.router, "last_plan", None)
-        plan = made[2] if made is not None and made[0] is idx and made[1] == plan_version(idx) else None
+        plan = made[2] if made is not None and made[0] is idx and made[1] == idx._version else None
         sh = self._shared(x) if self.num_shared else None
         if self.ep_size > 1:
             from ..parallel import ep

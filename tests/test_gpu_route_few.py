@@ -152,3 +152,27 @@ def test_a_plan_is_for_the_numbers_that_the_router_returned():
             layer.router.forward = forward
             got = layer(x)[0]                              # the same sums in another order
             assert float((got.float() - plain.float()).norm() / plain.float().norm()) < 1e-2
+
+
+@pytest.mark.parametrize("mode", [torch.no_grad, torch.inference_mode])
+@pytest.mark.parametrize("tokens", [1, 9, 16])
+def test_no_plan_outlives_a_write_to_its_numbers(mode, tokens):
+    """Numbers written to in place between the router and the experts, where tensors have versions and where they have none."""
+    from pisceslx_b200 import YvConfig
+    from pisceslx_b200.models.moe_layer import YvDeepSeekMoELayer
+    torch.manual_seed(0)
+    cfg = YvConfig.tiny_text_moe()
+    layer = YvDeepSeekMoELayer(cfg, 0).to("cuda", BF16).eval()
+    x = torch.randn(tokens, cfg.hidden_size, device="cuda").to(BF16)
+    route = layer.router.forward
+
+    def written(y):
+        w, idx, aux = route(y)
+        idx.copy_(idx.flip(1))
+        return w.flip(1), idx, aux
+
+    with mode():
+        plain = layer(x)[0]
+        layer.router.forward = written
+        got = layer(x)[0]                                  # the same sums in another order
+    assert float((got.float() - plain.float()).norm() / plain.float().norm()) < 1e-2

@@ -100,7 +100,7 @@ __device__ __forceinline__ void gate_select(const float* __restrict__ logits, co
   }
   float psum = 0.f, pmax = 0.f;
   for (int j = 0; j < k; ++j) {
-    float best = -FLT_MAX;
+    float best = -INFINITY;
     int best_e = 0x7FFFFFFF;
 #pragma unroll
     for (int i = 0; i < kMaxExpertsPerLane; ++i) {
@@ -113,12 +113,17 @@ __device__ __forceinline__ void gate_select(const float* __restrict__ logits, co
       const int oe = __shfl_xor_sync(0xFFFFFFFFu, best_e, o);
       if (ob > best || (ob == best && oe < best_e)) { best = ob; best_e = oe; }
     }
-    if (best_e >= E) best_e = j;                       // nothing compares above the lowest value: NaN or -inf throughout
+    if (best_e >= E) {                                 // what is left is NaN or -inf
+      best_e = 0;                                      // the lowest expert not taken yet: j of them are, and j < k <= E
+      for (int r = 0; r < j;) {
+        if (isel[r] == best_e) { ++best_e; r = 0; } else { ++r; }
+      }
+    }
     // owner lane publishes the probability and retires the expert
     float pv = 0.f;
 #pragma unroll
     for (int i = 0; i < kMaxExpertsPerLane; ++i) {
-      if (lane + 32 * i == best_e) { pv = p[i]; sel[i] = -FLT_MAX; }
+      if (lane + 32 * i == best_e) { pv = p[i]; sel[i] = -INFINITY; }
     }
     pv = __shfl_sync(0xFFFFFFFFu, pv, best_e & 31);
     isel[j] = best_e;

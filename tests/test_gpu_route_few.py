@@ -176,3 +176,24 @@ def test_no_plan_outlives_a_write_to_its_numbers(mode, tokens):
         layer.router.forward = written
         got = layer(x)[0]                                  # the same sums in another order
     assert float((got.float() - plain.float()).norm() / plain.float().norm()) < 1e-2
+
+
+@pytest.mark.parametrize("low", [float("-inf"), float("nan"), torch.finfo(torch.float32).min])
+@pytest.mark.parametrize("E,k,alone", [(8, 3, [[1, 2], [2, 1], [7], [0], [3, 4, 5], []]), (70, 16, [[69, 33, 1, 0], [32], [2, 1], []]), (2, 2, [[1], []])])
+@pytest.mark.parametrize("few", [True, False])
+def test_no_expert_is_taken_twice(low, E, k, alone, few):
+    """Fewer experts with a logit than are taken: the others come lowest first, without a weight."""
+    from pisceslx_b200.ops import moe as M_
+    logits = torch.full((len(alone), E), low)
+    for t, experts in enumerate(alone):
+        for j, e in enumerate(experts):
+            logits[t, e] = 2.0 - j
+    with torch.no_grad():
+        w, idx, counts = (M_.route_few if few else M_.gate_topk)(logits.cuda(), None, k)[:3]
+    want = [experts[:k] + [e for e in range(E) if e not in experts][:max(k - len(experts), 0)] for experts in alone]
+    assert idx.tolist() == want and counts.tolist() == torch.bincount(torch.tensor(want).flatten(), minlength=E).tolist()
+    for t, experts in enumerate(alone):
+        if experts and low == low:                          # NaN leaves no weights
+            shares = torch.softmax(torch.tensor([2.0 - j for j in range(len(experts))]), 0)
+            torch.testing.assert_close(w[t].cpu()[:len(experts)], shares / shares.sum(), rtol=1e-5, atol=0)
+            assert not w[t, len(experts):].any()

@@ -132,7 +132,8 @@ __global__ void __launch_bounds__(256) embed_join_kernel(const int* __restrict__
 
 int launch_embedding_grad(const void* dy, const int64_t* ids, void* dw, int* order, float* carry, int64_t T, int64_t V, int H,
                           cudaStream_t stream) {
-  if ((H & 7) != 0 || T > kEmbeddingGradTokens || V <= 0 || V >= 0x7FFFFFFF) return -1;
+  const uintptr_t at = reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(dw) | reinterpret_cast<uintptr_t>(carry);
+  if ((H & 7) != 0 || (at & 15u) != 0 || T > kEmbeddingGradTokens || V <= 0 || V >= 0x7FFFFFFF) return -1;
   const int r = static_cast<int>(cudaMemsetAsync(dw, 0, static_cast<size_t>(V) * H * 2, stream));
   if (r != 0 || T <= 0) return r;
   const int n = static_cast<int>(T), blocks = (n + kPlaces - 1) / kPlaces, across = (H / 8 + 255) / 256;

@@ -144,3 +144,17 @@ def test_loss_in_one_chunk_and_in_several(T, V, H):
         out.append((loss, *torch.autograd.grad(loss, (h, w))))
     for a, b in zip(*out):
         assert rel(a, b) < 2.0 ** -8
+
+
+@pytest.mark.parametrize("off", [1, 4, 8])
+def test_embedding_gradient_off_16_bytes(off):
+    """A gradient that is contiguous but begins between 16-byte boundaries (or, at 8, on one)."""
+    F_, _, _ = _ops()
+    r = _gen(off)
+    T, V, H = 70, 50, 64
+    w = r(V, H).to(BF16).requires_grad_(True)
+    ids = torch.randint(0, V, (T,), device="cuda", generator=torch.Generator("cuda").manual_seed(V))
+    dy = r(T * H + off).to(BF16)[off:].view(T, H)
+    got, = torch.autograd.grad(F_.embedding(ids, w), w, dy)
+    want = torch.zeros(V, H, device="cuda", dtype=torch.float64).index_add_(0, ids, dy.double())
+    assert ((got.double() - want).abs() <= want.abs() * 2.0 ** -8 + T * 2.0 ** -22).all()

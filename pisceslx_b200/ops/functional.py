@@ -11,6 +11,7 @@ import math
 from typing import Optional, Tuple
 
 import torch
+from torch.autograd import forward_ad
 
 from . import kernels, reference as ref, status_word
 
@@ -152,8 +153,10 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None
 
 
 def embedding(ids: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
-    """Rows of ``w`` [V, H]; on the GPU with a gradient that is summed by word without a sort."""
-    if w.is_cuda and w.dtype == _BF16 and w.requires_grad and torch.is_grad_enabled():
+    """Rows of ``w`` [V, H]; on the GPU with a gradient that is summed by word without a sort.  Function transforms, forward mode
+    and tracing see torch's own operator."""
+    if w.is_cuda and w.dtype == _BF16 and w.requires_grad and torch.is_grad_enabled() and \
+            not (torch._C._are_functorch_transforms_active() or torch.compiler.is_compiling() or forward_ad._current_level >= 0):
         return _k().embedding(w, ids)
     return torch.nn.functional.embedding(ids, w)
 

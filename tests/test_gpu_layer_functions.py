@@ -158,3 +158,28 @@ def test_embedding_gradient_off_16_bytes(off):
     got, = torch.autograd.grad(F_.embedding(ids, w), w, dy)
     want = torch.zeros(V, H, device="cuda", dtype=torch.float64).index_add_(0, ids, dy.double())
     assert ((got.double() - want).abs() <= want.abs() * 2.0 ** -8 + T * 2.0 ** -22).all()
+
+
+def test_embedding_under_transforms_and_twice():
+    """What torch's embedding does, the model's does too: function transforms, forward mode, a gradient of a gradient."""
+    import torch.autograd.forward_ad as fw
+    from pisceslx_b200.models.model import YvTokenEmbedding
+    r = _gen(3)
+    ids = torch.tensor([1, 2, 2, 7], device="cuda")
+    layer = YvTokenEmbedding(8, 64, device="cuda", dtype=BF16)
+    plain = torch.nn.Embedding(8, 64, device="cuda", dtype=BF16)
+    plain.load_state_dict(layer.state_dict())
+    tangent, seed = r(8, 64).to(BF16), r(4, 64).to(BF16)
+
+    def results(m):
+        w = m.weight
+        call = lambda t: torch.func.functional_call(m, {"weight": t}, (ids,))
+        with fw.dual_level():
+            forward = fw.unpack_dual(call(fw.make_dual(w, tangent))).tangent
+        first, = torch.autograd.grad((m(ids).float() ** 3).sum(), w, create_graph=True)
+        second, = torch.autograd.grad((first.float() * tangent.float()).sum(), w)
+        return [torch.func.grad(lambda t: (call(t).float() * seed.float()).sum())(w), forward, first, second,
+                torch.func.vmap(call)(torch.stack([w, 2 * w])), torch.func.jvp(call, (w,), (tangent,))[1]]
+
+    for a, b in zip(results(layer), results(plain)):
+        assert torch.equal(a, b)

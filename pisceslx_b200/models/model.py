@@ -66,9 +66,11 @@ class YvPackedTrunk(nn.Module):
 
 
 class YvTokenEmbedding(nn.Embedding):
-    """``nn.Embedding`` whose gradient comes from ``ops.functional.embedding``."""
+    """``nn.Embedding`` whose gradient comes from ``ops.functional.embedding``, unless one of torch's options is set on it."""
 
     def forward(self, input: torch.Tensor) -> torch.Tensor:
+        if self.padding_idx is not None or self.max_norm is not None or self.scale_grad_by_freq or self.sparse:
+            return super().forward(input)
         return F_.embedding(input, self.weight)
 
 

@@ -82,8 +82,7 @@ def bench_attn(a: argparse.Namespace, bwd: bool) -> Dict[str, Any]:
     do = torch.randn_like(o)
     dqkv = torch.empty_like(qkv)
     dq, dk, dv = dqkv[:, : hq * d], dqkv[:, hq * d:(hq + hk) * d], dqkv[:, (hq + hk) * d:]
-    delta = torch.empty(hq, T, device="cuda")
-    ms = timeit(lambda: K.attn_bwd(do, q, k, v, o, lse, dq, dk, dv, delta, cu, None, S, S, hq, hk, d, True, sc, st), a.iters)
+    ms = timeit(lambda: K.attn_bwd(do, q, k, v, o, lse, dq, dk, dv, None, cu, None, S, S, hq, hk, d, True, sc, st), a.iters)
     tf = 2.5 * flops / ms / 1e9
     return {"kernel": "attn_bwd", "shape": [B, S, hq, hk, d], "ms": ms, "tflops_5gemm": tf,
             "frac_of_peak": tf / peaks()["bf16_tflops"]}

@@ -127,7 +127,7 @@ int launch_attn_bwd(const AttnBwdArgs& b, cudaStream_t stream) {
   if (a.batch <= 0 || a.total_q <= 0) return 0;
   if (a.d != 64 && a.d != 128) return -1;
   if (a.hk <= 0 || a.hq % a.hk != 0) return -2;
-  if (b.delta == nullptr || a.lse == nullptr) return -3;
+  if ((b.delta == nullptr && b.dq_acc == nullptr) || a.lse == nullptr) return -3;
   AttnBwdParams p;
   int r = make_head_map(&p.tma_q, a.q, a.d, a.hq, a.total_q, a.q_stride);
   if (r != 0) return -10 + r;
@@ -152,8 +152,7 @@ int launch_attn_bwd(const AttnBwdArgs& b, cudaStream_t stream) {
   p.scale_log2 = a.scale * kLog2eHost;
   p.status = a.status;
 
-  // The statistics enter the one-pass kernel divided by the scale.
-  if (b.dq_acc != nullptr && fabsf(a.scale) > 1e-20f)
+  if (b.dq_acc != nullptr)
     return a.d == 128 ? launch_attn_bwd_fused<128>(b, p, stream) : launch_attn_bwd_fused<64>(b, p, stream);
 
   // the tensor maps have seen to 16-byte alignment of dO

@@ -234,8 +234,8 @@ struct AttnBwdArgs {
   void* dq = nullptr;          // bf16 [Tq, hq, d]
   void* dk = nullptr;          // bf16 [Tk, hk, d]
   void* dv = nullptr;          // bf16 [Tk, hk, d]
-  float* delta = nullptr;      // fp32 [hq, Tq] scratch
-  // sums of dq, fp32 [KV heads at a time, hq / hk, d, Tq] in any order of their own; without them two kernels without atomics run
+  float* delta = nullptr;      // fp32 [hq, Tq] scratch of the two kernels
+  // sums of dq, fp32 [KV heads at a time, hq / hk, d, Tq] in any order of their own, for scales that may be divided by; without them two kernels without atomics run
   float* dq_acc = nullptr;
   void* stats = nullptr;       // 16 bytes per (query head, token), with dq_acc
   int dq_acc_kv_heads = 0;

@@ -341,8 +341,7 @@ class _AttentionFn(torch.autograd.Function):
         q, k, v, o, lse, cu_q, cu_k = ctx.saved_tensors
         max_q, max_k, hq, hk, d, causal, scale, deterministic = ctx.cfg
         dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-        delta = torch.empty(hq, q.shape[0], dtype=torch.float32, device=q.device)
-        _k().attn_bwd(do.contiguous(), q, k, v, o, lse, dq, dk, dv, delta, cu_q, cu_k, max_q, max_k, hq, hk, d, causal,
+        _k().attn_bwd(do.contiguous(), q, k, v, o, lse, dq, dk, dv, None, cu_q, cu_k, max_q, max_k, hq, hk, d, causal,
                       scale, _st(q), deterministic)
         return (dq, dk, dv) + (None,) * 10
 

@@ -152,10 +152,9 @@ def _block_backward(do, q, k, v, o, lse, hq, hk, d, causal, scale, deterministic
     if q.is_cuda:
         K = kernels()
         dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-        delta = torch.empty(hq, L, dtype=torch.float32, device=q.device)
         cq = torch.tensor([0, L], dtype=torch.int32, device=q.device)
         ck = torch.tensor([0, Lk], dtype=torch.int32, device=q.device)
-        K.attn_bwd(do, q, k, v, o, lse, dq, dk, dv, delta, cq, ck, L, Lk, hq, hk, d, causal, scale, status_word(q.device),
+        K.attn_bwd(do, q, k, v, o, lse, dq, dk, dv, None, cq, ck, L, Lk, hq, hk, d, causal, scale, status_word(q.device),
                    deterministic)
         return dq.float(), dk.float(), dv.float()
     g = hq // hk

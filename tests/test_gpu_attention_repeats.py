@@ -76,3 +76,36 @@ def test_option_of_the_models():
         want = _reference(grads)
         for _ in range(3):
             _same(grads(), want)
+
+
+def test_scratch_of_the_backward_is_bounded():
+    """Sums of one KV head above the bound (300 000 tokens of 8 query heads of 64: 614 MB): the two kernels."""
+    from pisceslx_b200.ops import functional as F_
+    T, hq, hk, d, S = 300000, 8, 1, 64, 1000
+    g = torch.Generator("cuda").manual_seed(1)
+    q, k, v, do = (torch.randn(T, h * d, device="cuda", generator=g).to(BF16).requires_grad_(True) for h in (hq, hk, hk, hq))
+    cu = torch.arange(0, T + 1, S, dtype=torch.int32, device="cuda")
+    o = F_.attention(q, k, v, cu, None, S, S, hq, hk, d, True)
+    torch.cuda.reset_peak_memory_stats()
+    held = torch.cuda.memory_allocated()
+    grads = torch.autograd.grad(o, (q, k, v), do, retain_graph=True)
+    scratch = torch.cuda.max_memory_allocated() - held - 2 * sum(t.numel() for t in grads)
+    assert scratch <= 4 * T * hq + 2 ** 20
+    _same(grads, _reference(lambda: torch.autograd.grad(o, (q, k, v), do)))
+
+
+@pytest.mark.parametrize("scale", [1e-21, 1e-25])
+def test_softmax_scales_next_to_nothing(scale):
+    """Probabilities that are all but even, and scores that cannot be divided by their scale: P = 1 / keys, dq = dk = 0 but for
+    scale times finite sums."""
+    from pisceslx_b200.ops import functional as F_
+    S, h, d = 300, 2, 64
+    g = torch.Generator("cuda").manual_seed(2)
+    q, k, v, do = (torch.randn(S, h * d, device="cuda", generator=g).to(BF16).requires_grad_(True) for _ in range(4))
+    cu = torch.tensor([0, S], dtype=torch.int32, device="cuda")
+    o = F_.attention(q, k, v, cu, None, S, S, h, h, d, False, scale)
+    dq, dk, dv = torch.autograd.grad(o, (q, k, v), do)
+    rel = lambda a, b: float((a.double() - b).norm() / b.norm())
+    # P is rounded to bf16 (2^-9), outputs and gradients once more
+    assert rel(o, v.double().mean(0).expand(S, -1)) < 2.0 ** -7 and rel(dv, do.double().mean(0).expand(S, -1)) < 2.0 ** -7
+    assert float(dq.abs().max()) <= scale * 1e3 and float(dk.abs().max()) <= scale * 1e3

@@ -286,7 +286,9 @@ class YvModelForCausalLM(nn.Module):
             nv = None
             if num_valid is not None:
                 nv = num_valid
-            lm_loss = linear_cross_entropy(h_in, self.head_weight, tgt, -100, nv, rows_at_once(h_in.shape[0], *self.head_weight.shape))
+            w = self.head_weight
+            rows = rows_at_once(h_in.shape[0], *w.shape, weight_grad=w.requires_grad and torch.is_grad_enabled())
+            lm_loss = linear_cross_entropy(h_in, w, tgt, -100, nv, rows)
             loss = lm_loss
             res["lm_loss"] = lm_loss
             if self.num_mtp > 0:

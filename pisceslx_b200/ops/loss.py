@@ -1,6 +1,7 @@
 """Fused LM-head + cross-entropy: logits are produced chunk by chunk ([chunk, V] fp32), turned into
-per-token losses and logit gradients by one kernel, and immediately contracted into dH and dW, so the
-[T, V] logits tensor never exists (the reference materialises it, model/core/model.py:2440,2505).
+per-token losses and logit gradients by one kernel, and immediately contracted into dH and dW, so that
+logits of many rows never exist at once (the reference materialises [T, V], model/core/model.py:2440,2505);
+``rows_at_once`` says how many rows a chunk holds.
 """
 from __future__ import annotations
 
@@ -56,7 +57,7 @@ class _LinearCEFn(torch.autograd.Function):
         need_dw = ctx.needs_input_grad[1]
         loss_rows = torch.empty(T, dtype=torch.float32, device=dev)
         dh = torch.empty_like(h) if need_dh else None
-        n_chunks = (T + chunk - 1) // chunk
+        n_chunks = -(-T // max(chunk, 1))
         dw32 = None
         dw = None
         if need_dw:
@@ -98,13 +99,17 @@ class _LinearCEFn(torch.autograd.Function):
         return dh, dw, None, None, None, None
 
 
-def rows_at_once(T: int, V: int, H: int, chunk: int = 2048) -> int:
-    """Rows of logits to hold at a time: all of them where they, in fp32 and with their gradient in bf16, take no more than the
-    chunks and the fp32 sum of the weight gradient that several chunks need, or than 2 GB.  One chunk saves that sum's zeros, its
-    reads and writes by every chunk and its conversion: head and loss of 2331 rows of 1024, 154856 words, 3035 us in two chunks
-    and 2566 in one; of 8192 rows of 4096, 32000 words, 6207 in four and 5231."""
+_ONE_CHUNK = 2 << 30     # bytes: 1.2 % of the card's memory
+
+
+def rows_at_once(T: int, V: int, H: int, chunk: int = 2048, weight_grad: bool = True) -> int:
+    """Rows of logits to hold at a time.  One chunk saves the fp32 sum of the weight gradient that several add to: its zeros, its
+    reads and writes by every chunk and its conversion.  Head and loss of 2331 rows of 1024, 154856 words, 3035 us in two chunks
+    and 2566 in one; of 8192 rows of 4096, 32000 words, 6207 in four and 5231.  So all rows are held where the weight gradient is
+    wanted and they, in fp32 and with their gradient in bf16, take no more than several chunks and that sum (the first of these
+    two: 2.2 GB for 2.5), or at most 2 GB (the second: 1.57 GB, where four chunks and the sum take 0.92)."""
     one = 6 * T * V
-    return T if T <= chunk or one <= max(6 * chunk * V + 4 * V * H, 2 << 30) else chunk
+    return T if T <= chunk or weight_grad and one <= max(6 * chunk * V + 4 * V * H, _ONE_CHUNK) else chunk
 
 
 def linear_cross_entropy(h: torch.Tensor, w: torch.Tensor, labels: torch.Tensor, ignore_index: int = -100,

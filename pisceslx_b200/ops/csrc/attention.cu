@@ -317,7 +317,8 @@ int launch_kv_cache_write(const void* k, const void* v, void* k_cache, void* v_c
                           int64_t tokens, int row_elems, int64_t k_stride, int64_t v_stride, int64_t num_slots,
                           uint32_t* status, cudaStream_t stream) {
   if (tokens <= 0) return 0;
-  // rows are read and written 16 bytes at a time
+  // rows are read and written 16 bytes at a time; a single row has no pitch
+  if (tokens == 1) k_stride = v_stride = 0;
   const uintptr_t at = reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(k_cache) |
                        reinterpret_cast<uintptr_t>(v_cache);
   if ((row_elems & 7) != 0 || ((k_stride | v_stride) & 7) != 0 || (at & 15u) != 0) return -1;

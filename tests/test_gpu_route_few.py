@@ -197,3 +197,22 @@ def test_no_expert_is_taken_twice(low, E, k, alone, few):
             shares = torch.softmax(torch.tensor([2.0 - j for j in range(len(experts))]), 0)
             torch.testing.assert_close(w[t].cpu()[:len(experts)], shares / shares.sum(), rtol=1e-5, atol=0)
             assert not w[t, len(experts):].any()
+
+
+@pytest.mark.parametrize("pitch", [132, 129])
+def test_a_single_cache_row_has_no_pitch(pitch):
+    """One token's row out of a buffer whose rows are no whole number of 16-byte pieces, with a rotation and without."""
+    from pisceslx_b200.ops import functional as F_
+    from pisceslx_b200.ops.reference import rope_tables
+    k, v = (torch.randn(1, pitch, device="cuda", generator=_gen(i)).to(BF16)[:, :128] for i in range(2))
+    assert k.stride(0) == pitch
+    slot, pos = torch.tensor([70], device="cuda", dtype=torch.int32), torch.tensor([0], device="cuda", dtype=torch.int32)
+    cos, sin = rope_tables(8, 64, 1e4, device="cuda")
+    for rotate in (False, True):
+        kc, vc = (torch.zeros(2, 64, 2, 64, device="cuda", dtype=BF16) for _ in range(2))
+        if rotate:                                          # by nothing at place 0
+            F_.rope_cache(k.clone(), k, v, cos, sin, pos, 2, 2, 64, 64, kc, vc, slot)
+        else:
+            F_.kv_cache_write(k, v, kc, vc, slot)
+        for cache, row in ((kc, k), (vc, v)):
+            assert torch.equal(cache[1, 6].flatten(), row[0]) and int((cache != 0).sum()) == int((row != 0).sum())

@@ -144,7 +144,7 @@ def _tp_size(model) -> int:
 
 def to_device(values: List, dtype: torch.dtype, device: torch.device) -> torch.Tensor:
     """A list as a tensor on ``device``, by way of pinned memory: a copy from pageable memory waits for all that runs there."""
-    t = torch.tensor(values, dtype=dtype)
+    t = torch.tensor(values, dtype=dtype, device="cpu")          # whatever the default device is
     return t.pin_memory().to(device, non_blocking=True) if device.type == "cuda" else t.to(device)
 
 

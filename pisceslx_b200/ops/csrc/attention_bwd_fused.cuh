@@ -249,7 +249,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) attn_bwd_fused_kernel(const 
     if (warp == 1 && n_it > 0) {
       // The whole warp runs this and one thread issues: descriptors stay in uniform registers.
       const uint32_t lead = elect_one() ? 1u : 0u;
-      bool ok = mbar_wait(kv_full, 0, p.status);
+      bool ok = mbar_wait_warp(kv_full, 0, p.status);
       // Descriptors of the tiles, made anew from these at each product (kept for every step of every product they would not fit
       // into the registers).  K-major: a step of 16 along d; MN-major: of 16 rows.
       auto k_major = [](const uint8_t* tile) { return (make_smem_desc(smem_u32(tile), 16, 1024)); };
@@ -263,7 +263,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) attn_bwd_fused_kernel(const 
       };
       auto issue_s = [&](int it) -> bool {
         const int s = it % kStagesQ;
-        if (!mbar_wait(&q_full[s], (it / kStagesQ) & 1u, p.status)) return false;
+        if (!mbar_wait_warp(&q_full[s], (it / kStagesQ) & 1u, p.status)) return false;
         tc_fence_after_sync();
         const uint64_t dk = k_major(sK), dq = k_major(sQ + s * S::kTile);
 #pragma unroll
@@ -275,7 +275,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) attn_bwd_fused_kernel(const 
       };
       auto issue_dp = [&](int it) -> bool {
         const int s = it % kStagesDO;
-        if (!mbar_wait(&do_full[s], (it / kStagesDO) & 1u, p.status)) return false;
+        if (!mbar_wait_warp(&do_full[s], (it / kStagesDO) & 1u, p.status)) return false;
         tc_fence_after_sync();
         const uint64_t dv = k_major(sV), ddo = k_major(sDO + s * S::kTile);
 #pragma unroll
@@ -288,8 +288,8 @@ __global__ void __launch_bounds__(kFusedThreads, 1) attn_bwd_fused_kernel(const 
       // dV of block `it`; the block's dO has arrived or is waited for
       auto issue_dv = [&](int it) -> bool {
         const int s = it % kStagesDO;
-        if (!kRoom && !mbar_wait(p_full, it & 1u, p.status)) return false;
-        if (!mbar_wait(&do_full[s], (it / kStagesDO) & 1u, p.status)) return false;
+        if (!kRoom && !mbar_wait_warp(p_full, it & 1u, p.status)) return false;
+        if (!mbar_wait_warp(&do_full[s], (it / kStagesDO) & 1u, p.status)) return false;
         tc_fence_after_sync();
         const uint64_t ddo = mn_major(sDO + s * S::kTile);
 #pragma unroll
@@ -310,10 +310,10 @@ __global__ void __launch_bounds__(kFusedThreads, 1) attn_bwd_fused_kernel(const 
       for (int it = 0; it < n_it && ok; ++it) {
         const bool more = it + 1 < n_it;
         if (kRoom && more) {
-          ok = mbar_wait(s_read, it & 1u, p.status) && issue_s(it + 1);
+          ok = mbar_wait_warp(s_read, it & 1u, p.status) && issue_s(it + 1);
           if (!ok) break;
         }
-        ok = mbar_wait(ds_full, it & 1u, p.status);
+        ok = mbar_wait_warp(ds_full, it & 1u, p.status);
         if (!ok) break;
         tc_fence_after_sync();
         if (kRoom) {                                     // P^T and dS^T arrive together
@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) attn_bwd_fused_kernel(const 
         if (!more) tc_commit_if(lead, acc_done);
         if (kRoom) {
           if (more) ok = issue_dp(it + 1);               // over dS^T, which dK has read
-          if (ok && it > 0) ok = mbar_wait(dq_read, (it - 1) & 1u, p.status);
+          if (ok && it > 0) ok = mbar_wait_warp(dq_read, (it - 1) & 1u, p.status);
           if (!ok) break;
           tc_fence_after_sync();
         }
@@ -341,7 +341,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) attn_bwd_fused_kernel(const 
         tc_commit_if(lead, dq_full);
         if (!more) break;
         if (!kRoom) {
-          ok = mbar_wait(dq_read, it & 1u, p.status);    // dQ leaves the columns of dP^T
+          ok = mbar_wait_warp(dq_read, it & 1u, p.status);    // dQ leaves the columns of dP^T
           if (ok) ok = issue_dp(it + 1);
           if (ok) ok = issue_dv(it + 1);
           if (!ok) break;

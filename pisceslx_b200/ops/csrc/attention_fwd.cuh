@@ -227,6 +227,9 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
     auto commit = [&](uint64_t* bar) {
       if (kWarpIssues) tc_commit_if(lead, bar); else tc_commit(bar);
     };
+    auto wait = [&](uint64_t* bar, uint32_t parity) {
+      return kWarpIssues ? mbar_wait_warp(bar, parity, p.status) : mbar_wait(bar, parity, p.status);
+    };
     if (kWarpIssues || lead != 0u) {
       bool ok = true;
       uint32_t kv = 0, nq[2] = {0u, 0u}, np[2] = {0u, 0u};   // key tiles, Q tiles and P tiles so far
@@ -236,7 +239,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
         // S_t of step j; the products of one thread execute in order, so it follows the P V that read the same columns
         auto issue_qk = [&](int t, int j) -> bool {
           const uint32_t at = kv + it.key_tile(t, j), s = at % kStages;
-          if (!mbar_wait(&k_full[s], (at / kStages) & 1u, p.status)) return false;
+          if (!wait(&k_full[s], (at / kStages) & 1u)) return false;
           tc_fence_after_sync();
           const uint32_t aQ = smem_u32(sQ + t * S::kTile), aK = smem_u32(sK + s * S::kTile);
           const uint32_t tS = tmem_base + static_cast<uint32_t>(t * 128);
@@ -255,7 +258,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
         };
         for (int t = 0; t < 2 && ok; ++t) {
           if (it.count(t) == 0) continue;
-          ok = mbar_wait(&q_full[t], nq[t] & 1u, p.status);
+          ok = wait(&q_full[t], nq[t] & 1u);
           if (!ok) break;
           ++nq[t];
           ok = issue_qk(t, 0);
@@ -264,10 +267,10 @@ __global__ void __launch_bounds__(kAttnThreads, 1) attn_fwd_kernel(const __grid_
           for (int t = 0; t < 2 && ok; ++t) {
             if (j >= it.count(t)) continue;
             const uint32_t at = kv + it.key_tile(t, j), s = at % kStages;
-            ok = mbar_wait(&p_full[t], np[t] & 1u, p.status);
+            ok = wait(&p_full[t], np[t] & 1u);
             if (!ok) break;
             ++np[t];
-            ok = mbar_wait(&v_full[s], (at / kStages) & 1u, p.status);
+            ok = wait(&v_full[s], (at / kStages) & 1u);
             if (!ok) break;
             tc_fence_after_sync();
             const uint32_t aV = smem_u32(sV + s * S::kTile);

@@ -24,12 +24,13 @@ from typing import Dict, Tuple
 import torch
 
 PHASES = (
-    ("attention", ("attn_fwd", "attn_bwd", "attn_delta", "rope")),
+    ("attention", ("attn_fwd", "attn_bwd", "attn_delta", "attn_stats", "attn_dq_finish", "rope")),
     ("newton_schulz", ("gemm_batched", "frob_", "ns_poly", "muon_apply", "dequant_q8")),
     ("momentum_fold/adamw", ("momentum", "adamw", "zero_reduce_fold", "sumsq")),
     ("expert_parallel comm", ("ep_dispatch", "ep_combine", "ep_unpermute", "flag_barrier", "peer_copy", "nccl")),
-    ("moe routing/permute", ("gate_topk", "moe_", "swiglu", "histogram")),
+    ("moe routing/permute", ("gate_topk", "gate_plan", "moe_", "swiglu", "histogram")),
     ("loss", ("ce_kernel", "ce_")),
+    ("embedding", ("embed_",)),
     ("norm/elementwise", ("rmsnorm", "film", "elementwise", "vectorized", "copy", "Memcpy", "Memset", "fill", "cat")),
     ("gemm", ("gemm",)),
 )

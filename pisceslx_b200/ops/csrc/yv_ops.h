@@ -55,8 +55,8 @@ struct GemmArgs {
   const void* epi_cin = nullptr;
   float epi_a = 0.f, epi_b = 0.f, epi_c = 1.f;
   // Symmetric result (batched mode, M == N, bf16 C, the caller guarantees C = C^T, e.g. X X^T or a polynomial of a
-  // symmetric matrix): only the tiles that touch the diagonal or lie above it are computed; their epilogue also writes
-  // the mirrored elements of the tiles that were skipped.
+  // symmetric matrix): of the 128 x 128 blocks only those on the diagonal or above it are computed; those above it are stored
+  // a second time, transposed.
   bool symmetric = false;
 };
 // Returns 0 on success, a negative code when an argument is rejected, a positive cudaError_t otherwise.

@@ -183,3 +183,20 @@ def test_embedding_under_transforms_and_twice():
 
     for a, b in zip(results(layer), results(plain)):
         assert torch.equal(a, b)
+
+
+def test_router_and_experts_refuse_other_ranks():
+    """Tokens of several sequences that have not been flattened: sizes taken from the wrong dimensions would reach the kernels."""
+    _, M_, _ = _ops()
+    r = _gen(4)
+    w13, w2, x = r(4, 256, 128).to(BF16), r(4, 128, 128).to(BF16), r(2, 3, 128).to(BF16)
+    for logits in (r(2, 3, 4), r(4)):
+        for grad in (True, False):
+            with torch.set_grad_enabled(grad), pytest.raises((ValueError, IndexError)):
+                M_.gate_topk(logits, None, 2)
+    w, idx, counts, _ = M_.gate_topk(r(6, 4), None, 2)
+    for bad in ((x, w13, w2, w, idx), (x.view(6, 128), w13[None], w2, w, idx), (x.view(6, 128), w13, w2[0], w, idx),
+                (x.view(6, 128), w13, w2, w, idx.view(2, 3, 2)), (x, w13, w2, w, idx.view(2, 6))):
+        for grad in (True, False):
+            with torch.set_grad_enabled(grad), pytest.raises((ValueError, IndexError)):
+                M_.moe_experts(*bad, counts)

@@ -216,3 +216,20 @@ def test_a_single_cache_row_has_no_pitch(pitch):
             F_.kv_cache_write(k, v, kc, vc, slot)
         for cache, row in ((kc, k), (vc, v)):
             assert torch.equal(cache[1, 6].flatten(), row[0]) and int((cache != 0).sum()) == int((row != 0).sum())
+
+
+def test_a_slot_map_longer_than_the_tokens():
+    """Slots of a whole bucket with fewer tokens: the first of them count, as for kv_cache_write; fewer slots than tokens are refused."""
+    from pisceslx_b200.ops import functional as F_
+    from pisceslx_b200.ops.reference import rope_tables
+    q, k, v = (torch.randn(3, 256, device="cuda", generator=_gen(i)).to(BF16) for i in range(3))
+    cos, sin = rope_tables(8, 128, 1e4, device="cuda")
+    pos, slots = torch.arange(3, device="cuda", dtype=torch.int32), torch.tensor([5, 70, 6, 90, -1], device="cuda", dtype=torch.int32)
+    out = []
+    for n in (3, 5):
+        kc, vc = (torch.zeros(2, 64, 2, 128, device="cuda", dtype=BF16) for _ in range(2))
+        F_.rope_cache(q.clone(), k.clone(), v, cos, sin, pos, 2, 2, 128, 128, kc, vc, slots[:n])
+        out.append((kc, vc))
+    assert all(torch.equal(a, b) for a, b in zip(*out))
+    with pytest.raises(RuntimeError):
+        F_.rope_cache(q.clone(), k.clone(), v, cos, sin, pos, 2, 2, 128, 128, *out[0], slots[:2])

@@ -1,5 +1,6 @@
-// Flash attention backward for sm_100a with one writer for every row, for callers that ask torch for deterministic algorithms (and
-// for softmax scales that are next to nothing); attention_bwd_fused.cuh is the faster form, whose sums of dq have no fixed order.
+// Flash attention backward for sm_100a with one writer for every row, for gradients whose bits repeat, for softmax scales that are next
+// to nothing and for calls whose sums of dq would outgrow the scratch; attention_bwd_fused.cuh is the faster form, whose sums have no
+// fixed order.
 // Two tcgen05 kernels that recompute the probabilities from
 // the saved log-sum-exp (natural log of the scaled scores) and delta = rowsum(dO * O):
 //

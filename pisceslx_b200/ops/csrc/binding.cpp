@@ -1,6 +1,6 @@
 // PyTorch bindings (torch.ops.yv.*) for the sm_100a kernels.  Every op checks device, dtype, layout
 // and alignment on the host, passes raw pointers plus the current stream to a launcher, and raises on
-// a non-zero launcher code.  The ops that wrap one kernel do not allocate, but for the attention backward's sums: outputs and scratch
+// a non-zero launcher code.  The ops that wrap one kernel do not allocate, but for the attention backward's scratch: outputs and scratch
 // are passed in; the differentiable ones of binding_autograd.inc make theirs.
 #include "binding_gemm.inc"
 

@@ -36,12 +36,22 @@ class YvSwiGLU(nn.Module):
         return F_.linear(F_.swiglu(F_.linear(x, self.w13)), self.w2)
 
 
+def repeat_attention(module: nn.Module, cfg: Any) -> None:
+    """Attention gradients whose bits repeat in all layers of ``module`` that have the choice, where ``moe_deterministic`` is set."""
+    extra = getattr(cfg, "extra", None)
+    if isinstance(extra, dict) and extra.get("moe_deterministic", False):
+        for m in module.modules():
+            if hasattr(m, "deterministic"):
+                m.deterministic = True
+
+
 class YvFlashAttention(nn.Module):
     """Dense self-attention over [B, S, H] through the flash kernels (packed layout inside)."""
 
     def __init__(self, hidden: int, n_head: int, n_kv_head: Optional[int] = None, causal: bool = True):
         super().__init__()
         self.hq, self.hk, self.d, self.causal = n_head, n_kv_head or n_head, hidden // n_head, causal
+        self.deterministic = False                          # see repeat_attention
         self.qkv = nn.Parameter(torch.empty((self.hq + 2 * self.hk) * self.d, hidden).normal_(std=0.02))
         self.o = nn.Parameter(torch.empty(hidden, self.hq * self.d).normal_(std=0.02))
 
@@ -50,7 +60,8 @@ class YvFlashAttention(nn.Module):
         qkv = F_.linear(x.reshape(B * S, H), self.qkv)
         nq, nk = self.hq * self.d, self.hk * self.d
         cu = torch.arange(0, (B + 1) * S, S, dtype=torch.int32, device=x.device)
-        o = F_.attention(qkv[:, :nq], qkv[:, nq:nq + nk], qkv[:, nq + nk:], cu, cu, S, S, self.hq, self.hk, self.d, self.causal)
+        o = F_.attention(qkv[:, :nq], qkv[:, nq:nq + nk], qkv[:, nq + nk:], cu, cu, S, S, self.hq, self.hk, self.d, self.causal,
+                         deterministic=self.deterministic)
         return F_.linear(o, self.o).view(B, S, H)
 
 
@@ -60,6 +71,7 @@ class YvCrossAttention(nn.Module):
     def __init__(self, hidden: int, context_dim: int, n_head: int):
         super().__init__()
         self.h, self.d = n_head, hidden // n_head
+        self.deterministic = False
         self.q = nn.Parameter(torch.empty(hidden, hidden).normal_(std=0.02))
         self.kv = nn.Parameter(torch.empty(2 * hidden, context_dim).normal_(std=0.02))
         self.o = nn.Parameter(torch.empty(hidden, hidden).normal_(std=0.02))
@@ -71,7 +83,8 @@ class YvCrossAttention(nn.Module):
         kv = F_.linear(context.reshape(B * T, -1).to(x.dtype), self.kv)
         cu_q = torch.arange(0, (B + 1) * S, S, dtype=torch.int32, device=x.device)
         cu_k = torch.arange(0, (B + 1) * T, T, dtype=torch.int32, device=x.device)
-        o = F_.attention(q, kv[:, :H], kv[:, H:], cu_q, cu_k, S, T, self.h, self.h, self.d, False)
+        o = F_.attention(q, kv[:, :H], kv[:, H:], cu_q, cu_k, S, T, self.h, self.h, self.d, False,
+                         deterministic=self.deterministic)
         return F_.linear(o, self.o).view(B, S, H)
 
 

@@ -32,7 +32,7 @@ import torch.nn.functional as F
 
 from ..ops import functional as F_
 from ..ops.loss import linear_cross_entropy
-from .compat import YvSwiGLU
+from .compat import YvSwiGLU, repeat_attention
 from .norms import YvRMSNorm
 
 IGNORE_INDEX = -100
@@ -60,6 +60,7 @@ class _HeadAttention(nn.Module):
     def __init__(self, hidden: int, heads: int, std: float = 0.02):
         super().__init__()
         self.h, self.d = heads, hidden // heads
+        self.deterministic = False                          # see compat.repeat_attention
         self.qkv = nn.Parameter(torch.empty(3 * hidden, hidden).normal_(std=std))
         self.o = nn.Parameter(torch.empty(hidden, hidden).normal_(std=std))
 
@@ -67,7 +68,8 @@ class _HeadAttention(nn.Module):
         B, S, H = x.shape
         qkv = F_.linear(x.reshape(B * S, H), self.qkv.to(x.dtype))
         cu = torch.arange(0, (B + 1) * S, S, dtype=torch.int32, device=x.device)
-        o = F_.attention(qkv[:, :H], qkv[:, H:2 * H], qkv[:, 2 * H:], cu, cu, S, S, self.h, self.h, self.d, causal)
+        o = F_.attention(qkv[:, :H], qkv[:, H:2 * H], qkv[:, 2 * H:], cu, cu, S, S, self.h, self.h, self.d, causal,
+                         deterministic=self.deterministic)
         return o.view(B, S, self.h, self.d).to(x.dtype)
 
     def project(self, heads_out: torch.Tensor) -> torch.Tensor:
@@ -143,6 +145,7 @@ class YvMultiPathReasoningEngine(nn.Module):
             "start_hypothesis": None, "start_evidence": None, "start_conclusion": None,
             "hypothesis_split": None, "hypothesis_merge": None}
         self.last_depth: Optional[torch.Tensor] = None        # layers applied per position in the last call [B, S]
+        repeat_attention(self, cfg)
 
     # ---- reasoning tokens -----------------------------------------------------------------------------------------------
     def initialize_reasoning_tokens(self, tokenizer: Any = None) -> None:
@@ -683,6 +686,7 @@ class YvLatentCoTReasoner(nn.Module):
         self.complexity_length_tokens = float(_x(cfg, "reasoning_complexity_length_tokens", 512))
         self.long_sequence_layer_cap = len(self.reasoning_layers)
         self.last_depth: Optional[torch.Tensor] = None
+        repeat_attention(self, cfg)
 
     # the per-position depth machinery is the engine's
     abstraction_layers = property(lambda self: self.reasoning_layers)

@@ -22,7 +22,7 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
-from .compat import YvCrossAttention
+from .compat import YvCrossAttention, repeat_attention
 from .reasoning_engine import _x
 
 
@@ -64,6 +64,7 @@ class YvMultiModalReasoningEnhancer(nn.Module):
         self.evidence_aggregator = nn.Sequential(nn.Linear(3 * H, 2 * H), nn.SiLU(), nn.Linear(2 * H, H), nn.LayerNorm(H))
         self.confidence_estimator = nn.Sequential(nn.Linear(H, max(H // 2, 1)), nn.SiLU(), nn.Linear(max(H // 2, 1), 1),
                                                   nn.Sigmoid())
+        repeat_attention(self, cfg)
 
     def _modal(self, name: str, text: torch.Tensor, feats: torch.Tensor, linear: bool) -> torch.Tensor:
         if linear:
